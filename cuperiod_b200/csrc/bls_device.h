@@ -10,29 +10,33 @@
 
 namespace blsb200 {
 
-// Accumulation modes.  Every sum is an exact integer built from native 32-bit
-// shared atomics: a point's quantised value v (|v| <= 2^bits, bits =
-// min(27, 41 - ceil(log2 n)) for a curve of n points, at least 24) is added as
-// its unsigned low 13 bits to one word and its signed high part to another, so a
-// bin's sum is (signed) B * 2^13 + A with no carry lost for up to 2^17 points.
-//  UNIFORM: every point has the same inverse variance w: r_q (the quantised
-//           centred flux * weight) and a count per bin (three atomics).
-//  GENERAL: per-point weights spanning more than 2^8: the two sums (centred
-//           flux*weight and weight, both scaled by powers of two) stay FP64, like
-//           the reference's, with FP64 shared atomics.
-//  WIDE:    per-point weights within a factor 2^8 of each other: centred
-//           flux*weight and weight each quantised to 38-bit fixed point
-//           (|v| < 2^37 after a power-of-two scale) and added as three 32-bit
-//           parts (13, 13 and a signed 12-bit high part): six native atomics,
-//           exact integer sums for up to 2^17 points.
-enum : int { MODE_UNIFORM = 0, MODE_GENERAL = 1, MODE_WIDE = 2 };
-constexpr int kModes = 3;
-constexpr int kWideBits = 13;       // WIDE: bits of the low and middle parts
+// Accumulation modes.  Every sum but GENERAL's is an exact integer built from native
+// 32-bit shared reductions, one word per plane of the histogram (bls_kernels.cu states
+// why no carry is lost).  With one weight for every point a point's quantised centred
+// flux*weight v (|v| <= 2^bits, bits = min(27, 41 - ceil(log2 n)) for a curve of n
+// points, at least 24) and a count:
+//  PAIR:    two words; the host bounds the points of one bin by kPairMax;
+//  UNIFORM: three words, any number of points in a bin.
+// With per-point weights the centred flux*weight and the weight:
+//  WIDE:    weights within a factor 2^8 of each other, both quantised to 38-bit fixed
+//           point (|v| < 2^37 after a power-of-two scale), four words, at most kWideMax
+//           points in a bin;
+//  EXACT:   any weights, both as fixed point of magnitudes summing below 2^60 (finer
+//           than an FP64 prefix of their sum), six words, any number of points;
+//  GENERAL: FP64 sums by a compare-and-swap loop, for more than kMaxExactPoints points,
+//           sums outside 1e+-150, or histograms too wide for EXACT.
+enum : int { MODE_UNIFORM = 0, MODE_GENERAL = 1, MODE_WIDE = 2, MODE_PAIR = 3, MODE_EXACT = 4 };
+constexpr int kModes = 5;
+constexpr int kPairBits = 12;       // PAIR: bits of the count
+constexpr int kPairMax = 4000;      // PAIR: 4000 x (2^7 + 1) < 2^19, 4000 x 2^20 < 2^32
+constexpr int kWideBits = 19;       // WIDE: shift of the high word
+constexpr int kWideMax = 8191;      // WIDE: 8191 x (2^18 + 1) < 2^31, 8191 x 2^19 < 2^32
+constexpr int kExactBits = 15;      // EXACT: shift between words; 2^17 x 2^15 <= 2^32
 
 constexpr int kFields = 7;          // power, depth, depth_err, depth_snr, duration, t0, loglike
 constexpr int kMaxDur = 32;         // deduplicated box widths per segment
 constexpr int kMaxTile = 16;        // periods per work item
-constexpr int kHalfBits = 13;       // bits per atomic half-word
+constexpr int kHalfBits = 13;       // UNIFORM: bits of the low word
 constexpr int kCountShift = 18;     // packed prefix: R * 2^18 + count
 constexpr int kMaxExactPoints = (1 << 17) - 1;  // UNIFORM / WIDE: 32-bit prefix words
                                                 // stay exact; longer curves take GENERAL
@@ -48,10 +52,10 @@ constexpr int kChunkThreads = 256;
 constexpr int kChunkPts = 8;
 constexpr int kChunk = kChunkThreads * kChunkPts;
 
-// The box sweep reads the FP32 screen records of starts up to 2 x kChunkThreads
-// + 31 past the last admissible start; that many records after a period's last
-// bin hold a sentinel that fails every screen, so the sweep needs no bounds test.
-constexpr int kScreenPad = 2 * kChunkThreads + 32;
+// The box sweep reads the FP32 screen records of up to 31 starts past the last
+// admissible one; that many records after a period's last bin hold a sentinel that
+// fails every screen, so the sweep needs no bounds test.
+constexpr int kScreenPad = 32;
 
 struct SegmentDesc {
     int64_t period_off;     // first period of this segment in the grid arrays
@@ -62,7 +66,7 @@ struct SegmentDesc {
     int32_t n_dur;
     int32_t oversample;
     int32_t frac_bits;      // fast fold: fraction bits of the scaled phase
-    uint32_t margin_u;      // fast fold: bin-edge margin, units of 2^-frac_bits bins
+    uint32_t margin_u;      // fast fold: edge margin (FoldConst), units of 2^-frac_bits bins
     uint32_t margin_phi;    // fast fold: cycle-edge margin, units of 2^-32 cycles
     int32_t fast_fold;      // 1: the fast fold's error bound holds for the batch
     int32_t hist_len;       // bins held per period: max n_bins + 1 over the segment
@@ -73,7 +77,7 @@ struct CurveDesc {
     int64_t out_off;        // this curve's spectrum in each output field starts at
                             // out_off + (its grid's first period in the period arrays)
     int32_t n_points;
-    int32_t mode;           // MODE_UNIFORM / MODE_GENERAL
+    int32_t mode;           // MODE_*
     int32_t exact_all;      // 1: every admissible box is evaluated in FP64
     int32_t skip;           // 1: nothing admissible (e.g. zero total weight)
     double t_min;           // time origin removed from tau (added back to t0)
@@ -82,22 +86,25 @@ struct CurveDesc {
     double ivar_floor;      // admissibility floor of either side of a box
     double ybar;            // sum_y / sum_ivar
     double w_uniform;       // UNIFORM: the common ivar
-    double i_total;         // GENERAL: sum of the scaled weights
+    double i_total;         // per-point weights: sum of the stored weights
     int32_t e_r;            // r (reference units) = stored r * 2^-e_r
-    int32_t e_i;            // GENERAL: ivar (reference units) = stored weight * 2^-e_i
+    int32_t e_i;            // per-point weights: ivar (reference units) = stored * 2^-e_i
     // UNIFORM: a point's stored value is round(y*ivar * 2^e_r) - round(ybar*ivar
     // * 2^e_r): centred by a whole number of quanta, so each point's rounding is
     // its own (centring by ybar itself gave every point the same rounding error,
     // which grew with the box instead of its square root).
     double center;          // the per-point centring, reference units
     double center_frac;     // ybar*ivar*2^e_r minus that whole number (|.| <= 1/2)
-    // WIDE: the exact sums of every point's quantised centred flux*weight and
+    // WIDE / EXACT: the exact sums of every point's quantised centred flux*weight and
     // weight.  A box's outside sums are these minus its inside sums, so a box
     // holding every point has exactly zero weight outside and fails the floor
     // test as the reference's does (sum_ivar minus a quantised inside sum would
     // leave the quantisation residual, far above the floor).
     long long rq_total;
     long long iq_total;
+    float w_small;          // per-point weights: a box whose FP32 screen weight is not above
+                            // this is empty (-1: FP32 does not resolve the smallest weight)
+    float gap;              // mean time between points
 };
 
 struct WorkItem {
@@ -134,10 +141,10 @@ struct BatchArgs {
     WorkGroup group0;           // groups[0], read from the launch parameters
     int32_t n_groups;
     const double* tau;          // per point: t - t_min (FP64)
-    const uint32_t* pay_r;      // per point: r_q as low 13 bits | signed high part << 16
+    const int32_t* pay_r;       // one weight: the quantised centred flux*weight per point
     const double* r64;          // GENERAL: (y*ivar - ybar*ivar) * 2^e_r per point;
-                                // WIDE: the same rounded to an int64 (bit pattern)
-    const double* iv64;         // GENERAL: ivar * 2^e_i per point; WIDE: int64 likewise
+                                // WIDE / EXACT: the same rounded to an int64 (bit pattern)
+    const double* iv64;         // GENERAL: ivar * 2^e_i per point; WIDE / EXACT: int64
     const double* period;       // per grid period
     const double* freq;         // RN(1/P)
     const uint32_t* scale;      // round(P/bin * 2^frac_bits)
@@ -192,7 +199,7 @@ struct JointSegment {
     int32_t oversample;
     int32_t hist_len;       // max n_bins + 1 over the segment
     int32_t frac_bits;      // fast fold (fold_fast): fraction bits of the scaled phase
-    uint32_t margin_u;      // fast fold: bin-edge margin, units of 2^-frac_bits bins
+    uint32_t margin_u;      // fast fold: edge margin (FoldConst), units of 2^-frac_bits bins
     uint32_t margin_phi;    // fast fold: cycle-edge margin, units of 2^-32 cycles
     int32_t fast_fold;      // 1: the fast fold's error bound holds for the star
 };

@@ -170,7 +170,10 @@ FoldParams fold_params(int64_t width, double bin, double tau_max, double f_max, 
     const double e_ref = 2.0 * std::ldexp(1.0, ex - 52) / bin + (double)width * std::ldexp(1.0, -52);
     const double scale = std::ldexp(1.0, fp.fb);
     const double e_u = e_phi * s_max * scale + 2.0;          // + S rounding and the floor
-    const double mu = std::ceil(e_u + e_ref * scale) + 2.0;
+    // FoldConst adds mphi to the phase (at most mphi to the position, S < 2^32) and
+    // tests this one margin: it covers the bin-edge error on either side of that
+    // shift, and the 2 mphi that phases next to a cycle edge land in
+    const double mu = std::max(std::ceil(e_u + e_ref * scale) + mphi, 2.0 * mphi) + 4.0;
     if (!(mphi < 1e6) || !(mu * 4.0 < scale)) return fp;
     fp.mu = (uint32_t)mu;
     fp.mphi = (uint32_t)mphi;
@@ -229,9 +232,9 @@ struct BlsEngine {
     std::vector<int64_t> spec_off;      // host: per-curve spectrum offsets (n_curves + 1)
     const int64_t* d_spec_off = nullptr;    // device: per-curve spectrum offsets (n_curves + 1)
     const int64_t* d_grid_base = nullptr;   // device: per-curve first period of its grid
-    int n_items_mode[kModes] = {0, 0, 0};
-    int ctas_mode[kModes] = {0, 0, 0};
-    size_t smem_mode[kModes] = {0, 0, 0};
+    int n_items_mode[kModes] = {};
+    int ctas_mode[kModes] = {};
+    size_t smem_mode[kModes] = {};
     BatchArgs args[kModes]{};
     BlsBatchInfo info{};
 
@@ -273,14 +276,6 @@ cudaStream_t pick(BlsEngine* e, void* s) {
     return s ? static_cast<cudaStream_t>(s) : e->stream;
 }
 
-// One quantised value (|v| <= 2^27) as the kernel adds it: the unsigned low 13
-// bits in the low half-word, the signed high part in the high half-word.
-inline uint32_t split_word(long long v) {
-    const uint32_t lo = (uint32_t)(v & ((1 << kHalfBits) - 1));
-    const int32_t hi = (int32_t)(v >> kHalfBits);              // arithmetic shift
-    return lo | ((uint32_t)(uint16_t)(int16_t)hi << 16);
-}
-
 // Memory slot of the point with time index j in a curve of n points: every full
 // chunk of kChunk points is stored lane-interleaved (see kChunk in bls_device.h),
 // the tail in time order.
@@ -304,15 +299,47 @@ double median_of(const double* y, int64_t n, std::vector<double>& scratch) {
     return med;
 }
 
+// What a curve's encoding depends on of the grid it is searched over: each segment's
+// phase bin and shortest period, and whether the EXACT histograms of its widest period
+// fit shared memory.
+struct GridBins {
+    std::vector<std::pair<double, double>> seg;     // {bin, shortest period}
+    bool exact_fits = false;
+};
+
+// Whether no phase bin of any trial period of the grid can hold more than `limit` of the
+// curve's points: a bin of one cycle spans `bin` in time, so it holds at most the most
+// points in any window of that length (from the smallest time gap, else by sliding the
+// window), and the curve crosses at most span / P + 2 cycles.  tau in time order;
+// an unordered curve only passes by its length.
+bool bins_hold_at_most(int64_t limit, const double* tau, int64_t n, bool ordered, double span,
+                       double min_gap, const GridBins& gb) {
+    if (n <= limit) return true;
+    if (!ordered) return false;
+    for (const auto& sg : gb.seg) {
+        // the reference's bins have edges exact to a few ulps of the time
+        const double win = sg.first * (1.0 + 1e-6) + span * 1e-14;
+        const double cycles = std::floor(span / sg.second) + 2.0;
+        if (!(cycles * 1.0 <= (double)limit)) return false;
+        if (min_gap > 0.0 && cycles * (std::floor(win / min_gap) + 1.0) <= (double)limit) continue;
+        const int64_t most = (int64_t)((double)limit / cycles);     // points per window
+        for (int64_t j = most; j < n; ++j)
+            if (tau[j] - tau[j - most] <= win) return false;
+    }
+    return true;
+}
+
 // Pack one curve: the reference's host inputs, then the fixed-point words.
-void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* pay_r,
-                double* r64, double* iv64, CurveHost& ch, std::vector<double>& scratch) {
+void pack_curve(const BlsCurves* cv, int c, int64_t off, const GridBins& gb, double* tau,
+                int32_t* pay_r, double* r64, double* iv64, CurveHost& ch,
+                std::vector<double>& scratch) {
     const int64_t b = cv->offsets[c], e = cv->offsets[c + 1];
     const int64_t n = e - b;
     CurveDesc& d = ch.d;
     std::memset(&d, 0, sizeof(d));
     d.point_off = off;
     d.n_points = (int32_t)n;
+    d.w_small = -1.0f;
     if (n < 1) {
         ch.status = BLS_E_INVALID;
         ch.err = "light curve " + std::to_string(c) + " has no points";
@@ -340,15 +367,18 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
     }
     const double med = median_of(y, n, scratch);
     // yw, ivar (reference units); sums with numpy's pairwise order
-    scratch.resize(3 * (size_t)n);
+    scratch.resize(4 * (size_t)n);
     double* yw = scratch.data();
     double* iv = yw + n;
     double* r = iv + n;
-    double tau_max = 0.0;
+    double* ts = r + n;                     // time offsets in input order
+    double tau_max = 0.0, min_gap = INFINITY;
     bool uniform = true;
     for (int64_t j = 0; j < n; ++j) {
         const double tj = t[j] - t_min;
         tau[point_slot(j, n)] = tj;
+        ts[j] = tj;
+        if (j > 0) min_gap = std::min(min_gap, tj - ts[j - 1]);
         tau_max = std::max(tau_max, tj);
         iv[j] = dy ? 1.0 / (dy[j] * dy[j]) : 1.0;
         yw[j] = (y[j] - med) * iv[j];
@@ -369,10 +399,17 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
         max_r = std::max(max_r, std::fabs(r[j]));
         max_i = std::max(max_i, iv[j]);
     }
-    // r_q = r * 2^e_r with |r_q| <= 2^bits: bits = min(27, 41 - ceil(log2 n)), so
-    // the signed high part (r_q >> 13, 16 bits in the payload word) fits and the
-    // high-part word's prefix sums, doubled at most by the wrap pad, stay below
-    // 2^31 (n * 2^(bits - 12) <= 2^29); at least 24 bits up to 2^17 points
+    auto holds = [&](int64_t limit) {
+        return bins_hold_at_most(limit, ts, n, min_gap >= 0.0, tau_max, min_gap, gb);
+    };
+    const double eps = DBL_EPSILON;
+    double floor_v = 4.0 * (double)n * eps * sum_ivar;            // _ivar_floor, 75-94
+    if (!(floor_v > 0.0)) floor_v = DBL_MIN;
+    d.exact_all = !(sum_abs >= 1e-150 && sum_abs <= 1e150 && sum_ivar >= 1e-150 &&
+                    sum_ivar <= 1e150);
+    // r_q = r * 2^e_r with |r_q| <= 2^bits: bits = min(27, 41 - ceil(log2 n)), so a
+    // prefix sum, doubled at most by the wrap pad, stays below 2^43 and packs with its
+    // count in 64 bits; at least 24 bits up to 2^17 points
     int m = 0;
     while (m < 62 && ((int64_t)1 << m) < n) ++m;
     const int bits = std::min(27, 41 - m);
@@ -392,10 +429,7 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
         cq = std::llrint(cw);
         c_frac = cw - (double)cq;
         for (int64_t j = 0; j < n; ++j)
-            pay_r[point_slot(j, n)] = split_word(std::llrint(std::ldexp(yw[j], e_r)) - cq);
-    } else {
-        for (int64_t j = 0; j < n; ++j)
-            pay_r[point_slot(j, n)] = split_word(std::llrint(std::ldexp(r[j], e_r)));
+            pay_r[point_slot(j, n)] = (int32_t)(std::llrint(std::ldexp(yw[j], e_r)) - cq);
     }
     int e_i = 0;
     double i_total = 0.0;
@@ -404,13 +438,29 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
     // (the smallest weight keeps >= 2^28 steps, a relative 2^-29)
     double min_i = max_i;
     for (int64_t j = 0; j < n && !uniform; ++j) min_i = std::min(min_i, iv[j]);
-    const bool wide = exact_ok && !uniform && min_i > 0.0 && std::isfinite(max_i) &&
-                      max_i <= 256.0 * min_i && max_r > 0.0 && std::isfinite(max_r);
-    if (wide) {
-        int kr = 0, ki = 0;
-        std::frexp(max_r, &kr);            // max_r < 2^kr
-        std::frexp(max_i, &ki);
-        const int e_rw = 37 - kr, e_iw = 37 - ki;       // |v| < 2^37
+    const bool finite = exact_ok && !uniform && min_i > 0.0 && std::isfinite(max_i) &&
+                        std::isfinite(max_r);
+    bool wide = finite && max_i <= 256.0 * min_i && max_r > 0.0;
+    // more points in a bin than WIDE's words hold, or any spread of weights: fixed point
+    // of the sums' range
+    const bool exact = finite && gb.exact_fits && !d.exact_all && !(wide && holds(kWideMax));
+    if (exact) wide = false;
+    wide = wide && holds(kWideMax);
+    if (wide || exact) {
+        int kr = 0, ki = 0, e_rw, e_iw;
+        if (wide) {
+            std::frexp(max_r, &kr);        // max_r < 2^kr
+            std::frexp(max_i, &ki);
+            e_rw = 37 - kr;                // |v| < 2^37
+            e_iw = 37 - ki;
+        } else {
+            double sum_r = 0.0;
+            for (int64_t j = 0; j < n; ++j) sum_r += std::fabs(r[j]);
+            std::frexp(sum_r * (1.0 + 1e-10), &kr);         // every prefix below 2^60
+            std::frexp(sum_ivar * (1.0 + 1e-10), &ki);
+            e_rw = sum_r > 0.0 ? 60 - kr : 0;
+            e_iw = 60 - ki;
+        }
         int64_t total = 0, rtotal = 0;
         for (int64_t j = 0; j < n; ++j) {
             const int64_t m = point_slot(j, n);
@@ -426,6 +476,12 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
         i_total = (double)total;
         rq_total = rtotal;
         iq_total = total;
+        // half the smallest weight in the FP32 screen's units, when the FP32 error of a
+        // box's weight (half an ulp per prefix: 2^-24 of the total) is at most half that
+        const int shift = screen_shift(wide ? MODE_WIDE : MODE_EXACT);
+        const double small = std::ldexp(min_i, e_i - shift);
+        if (!d.exact_all && small > std::ldexp(i_total, -shift - 22))
+            d.w_small = (float)(0.5 * small);
     } else if (!uniform) {
         // per-point weights: FP64 values scaled by powers of two (exact)
         if (max_i > 0.0 && std::isfinite(max_i)) {
@@ -439,13 +495,12 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, double* tau, uint32_t* 
             i_total += iv64[m];
         }
     }
-    const double eps = DBL_EPSILON;
-    double floor_v = 4.0 * (double)n * eps * sum_ivar;            // _ivar_floor, 75-94
-    if (!(floor_v > 0.0)) floor_v = DBL_MIN;
-    d.mode = uniform ? MODE_UNIFORM : (wide ? MODE_WIDE : MODE_GENERAL);
-    d.exact_all = !(sum_abs >= 1e-150 && sum_abs <= 1e150 && sum_ivar >= 1e-150 &&
-                    sum_ivar <= 1e150);
+    d.mode = uniform ? (holds(kPairMax) ? MODE_PAIR : MODE_UNIFORM)
+             : wide  ? MODE_WIDE
+             : exact ? MODE_EXACT
+                     : MODE_GENERAL;
     d.skip = !(sum_ivar > 0.0 && std::isfinite(sum_ivar));
+    d.gap = (float)(tau_max / (double)n);
     d.t_min = t_min;
     d.sum_y = sum_y;
     d.sum_ivar = sum_ivar;
@@ -485,15 +540,15 @@ void parallel_for(int n, F&& fn) {
 }
 
 // Dynamic shared memory per CTA: one weight per curve runs three CTAs per SM
-// (the kernel is built for 80 registers), per-point weights (FP64 or wide
-// fixed point) two.
-constexpr size_t kDefaultSmem[kModes] = {72 * 1024, 108 * 1024, 108 * 1024};
+// (the kernel is built for 80 registers), per-point weights two.
+constexpr size_t kDefaultSmem[kModes] = {70 * 1024, 108 * 1024, 108 * 1024, 70 * 1024,
+                                         108 * 1024};
 
-size_t screen_bytes(int /*mode*/, int hl) { return ((size_t)hl + kScreenPad) * 8; }
+size_t screen_bytes(int hl) { return ((size_t)hl + kScreenPad) * 8; }
 size_t period_bytes(int mode, int hl) { return period_hist_bytes(mode, hl); }
 
 int tile_cap(int mode, int hl, size_t smem, int max_tile) {
-    const size_t scr = screen_bytes(mode, hl) + 16;
+    const size_t scr = screen_bytes(hl) + 16;
     if (smem <= scr) return 0;
     int cap = (int)((smem - scr) / period_bytes(mode, hl));
     cap = std::min(cap, kMaxTile);
@@ -555,50 +610,17 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     const int64_t n_pts = cv->offsets[nc] - cv->offsets[0];
     if (cv->offsets[0] != 0 || n_pts < 0) return fail(BLS_E_INVALID, "offsets[0] must be 0");
 
-    // ---- curves ---------------------------------------------------------------
+    // ---- segments (reference binning), grids in parallel ------------------------------
     int rc;
-    if ((rc = e->h_tau.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
-    if ((rc = e->h_pay_r.ensure(sizeof(uint32_t) * std::max<int64_t>(n_pts, 1)))) return rc;
-    if ((rc = e->h_r64.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
-    if ((rc = e->h_iv64.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
-    std::vector<CurveHost> curves(nc);
-    int hw = std::max(1, (int)std::thread::hardware_concurrency());
-    std::vector<std::vector<double>> scratch(hw);
-    double* htau = e->h_tau.as<double>();
-    uint32_t* hpr = e->h_pay_r.as<uint32_t>();
-    double* hr64 = e->h_r64.as<double>();
-    double* hiv64 = e->h_iv64.as<double>();
-    parallel_for(nc, [&](int c, int w) {
-        const int64_t off = cv->offsets[c];
-        try {                       // a worker thread: nothing may escape it
-            pack_curve(cv, c, off, htau + off, hpr + off, hr64 + off, hiv64 + off, curves[c],
-                       scratch[w]);
-        } catch (const std::bad_alloc&) {
-            curves[c].status = BLS_E_NOMEM;
-            curves[c].err = "host allocation failed while packing a light curve";
-        }
-        curves[c].d.out_off = spec_off[c] - pbase[gid[c]];
-    });
-    int n_uniform = 0;
-    int n_mode[kModes] = {0, 0, 0};
-    std::vector<double> tau_max(n_grids, 0.0);                  // per grid, over its curves
-    std::vector<std::array<int, kModes>> grid_mode(n_grids, std::array<int, kModes>{0, 0, 0});
-    for (int c = 0; c < nc; ++c) {
-        if (curves[c].status) return fail(curves[c].status, "%s", curves[c].err.c_str());
-        if (e->tune.exact_sweep) curves[c].d.exact_all = 1;
-        tau_max[gid[c]] = std::max(tau_max[gid[c]], curves[c].tau_max);
-        n_uniform += curves[c].d.mode == MODE_UNIFORM;
-        n_mode[curves[c].d.mode]++;
-        grid_mode[gid[c]][curves[c].d.mode]++;
-    }
-
-    // ---- segments and period constants (reference binning), grids in parallel ---
     std::vector<SegmentHost> segs(ns);
     std::vector<double> per(P_total);
     std::vector<PeriodConst> pc(P_total);
     std::vector<double> grid_boxes(n_grids, 0.0), grid_trials(n_grids, 0.0);
     std::vector<int> grid_err(n_grids, BLS_OK);
     std::vector<std::string> grid_msg(n_grids);
+    std::vector<GridBins> grid_bins(n_grids);
+    // the opt-in limit covers the kernel's static shared state too
+    const size_t exact_limit = e->smem_optin + 1024 - search_static_smem(MODE_EXACT);
     parallel_for(n_grids, [&](int k, int /*w*/) {
       try {                         // a worker thread: nothing may escape it
         const BlsGrid& g = grids[k];
@@ -607,6 +629,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             grid_msg[k] = std::move(msg);
         };
         char buf[256];
+        int widest = 2;
         for (int sl = 0; sl < g.n_segments; ++sl) {
             const int s = sbase[k] + sl;
             const int64_t q0 = g.seg_offsets[sl], q1 = g.seg_offsets[sl + 1];   // this grid's
@@ -630,7 +653,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
                 std::snprintf(buf, sizeof buf, "segment %d has no durations", s);
                 return bad(BLS_E_INVALID, buf);
             }
-            double dmin = INFINITY, pmax = 0.0, fmax = 0.0;
+            double dmin = INFINITY, pmax = 0.0, pmin = INFINITY;
             for (int64_t i = d0; i < d1; ++i) {
                 const double d = g.durations[i];
                 if (!(std::isfinite(d) && d > 0.0)) {
@@ -648,6 +671,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
                     return bad(BLS_E_INVALID, buf);
                 }
                 pmax = std::max(pmax, P);
+                pmin = std::min(pmin, P);
                 per[pbase[k] + i] = P;
             }
             const double bin = dmin / (double)o;                              // _search_spec
@@ -671,34 +695,93 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             }
             const int64_t width = (int64_t)wmax;
             int64_t hl = 2;
-            double smax = 0.0;
             for (int64_t i = p0; i < p1; ++i) {
-                const double P = per[i];
-                const int64_t nb = period_bins(P, bin, o, width);
-                hl = std::max(hl, nb + 1);
-                fmax = std::max(fmax, 1.0 / P);
-                smax = std::max(smax, P / bin);
+                pc[i].nb = (int32_t)period_bins(per[i], bin, o, width);
+                hl = std::max<int64_t>(hl, pc[i].nb + 1);
             }
             sd.width = (int32_t)width;
             sd.bin_duration = bin;
             sd.n_dur = (int32_t)sh.dur.size();
             sd.hist_len = (int32_t)hl;
-            FoldParams fp = fold_params(width, bin, tau_max[k], fmax, smax);
+            grid_bins[k].seg.emplace_back(bin, pmin);
+            widest = std::max<int>(widest, sd.hist_len);
+        }
+        const size_t need = screen_bytes(widest) + 16 + period_hist_bytes(MODE_EXACT, widest);
+        grid_bins[k].exact_fits = need <= exact_limit;
+      } catch (const std::bad_alloc&) {
+        grid_err[k] = BLS_E_NOMEM;
+        grid_msg[k] = "host allocation failed while preparing a grid";
+      }
+    });
+
+    // ---- curves ---------------------------------------------------------------
+    if ((rc = e->h_tau.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
+    if ((rc = e->h_pay_r.ensure(sizeof(uint32_t) * std::max<int64_t>(n_pts, 1)))) return rc;
+    if ((rc = e->h_r64.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
+    if ((rc = e->h_iv64.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
+    std::vector<CurveHost> curves(nc);
+    int hw = std::max(1, (int)std::thread::hardware_concurrency());
+    std::vector<std::vector<double>> scratch(hw);
+    double* htau = e->h_tau.as<double>();
+    int32_t* hpr = e->h_pay_r.as<int32_t>();
+    double* hr64 = e->h_r64.as<double>();
+    double* hiv64 = e->h_iv64.as<double>();
+    parallel_for(nc, [&](int c, int w) {
+        const int64_t off = cv->offsets[c];
+        try {                       // a worker thread: nothing may escape it
+            pack_curve(cv, c, off, grid_bins[gid[c]], htau + off, hpr + off, hr64 + off, hiv64 + off, curves[c],
+                       scratch[w]);
+        } catch (const std::bad_alloc&) {
+            curves[c].status = BLS_E_NOMEM;
+            curves[c].err = "host allocation failed while packing a light curve";
+        }
+        curves[c].d.out_off = spec_off[c] - pbase[gid[c]];
+    });
+    int n_uniform = 0;
+    int n_mode[kModes] = {};
+    std::vector<double> tau_max(n_grids, 0.0);                  // per grid, over its curves
+    std::vector<std::array<int, kModes>> grid_mode(n_grids, std::array<int, kModes>{});
+    for (int c = 0; c < nc; ++c) {
+        if (curves[c].status) return fail(curves[c].status, "%s", curves[c].err.c_str());
+        if (e->tune.exact_sweep) {
+            curves[c].d.exact_all = 1;
+            curves[c].d.w_small = -1.0f;
+        }
+        tau_max[gid[c]] = std::max(tau_max[gid[c]], curves[c].tau_max);
+        n_uniform += curves[c].d.mode == MODE_UNIFORM || curves[c].d.mode == MODE_PAIR;
+        n_mode[curves[c].d.mode]++;
+        grid_mode[gid[c]][curves[c].d.mode]++;
+    }
+
+    // ---- fold constants, which depend on the curves' time spans --------------------
+    parallel_for(n_grids, [&](int k, int /*w*/) {
+        if (grid_err[k]) return;
+        for (int sl = 0; sl < grids[k].n_segments; ++sl) {
+            const int s = sbase[k] + sl;
+            SegmentHost& sh = segs[s];
+            SegmentDesc& sd = sh.d;
+            if (sh.empty_periods) continue;
+            const int64_t p0 = sd.period_off, p1 = p0 + sd.n_periods;
+            const double bin = sd.bin_duration;
+            double fmax = 0.0, smax = 0.0;
+            for (int64_t i = p0; i < p1; ++i) {
+                fmax = std::max(fmax, 1.0 / per[i]);
+                smax = std::max(smax, per[i] / bin);
+            }
+            FoldParams fp = fold_params(sd.width, bin, tau_max[k], fmax, smax);
             const double scale = std::ldexp(1.0, fp.fb);
             for (int64_t i = p0; i < p1 && fp.fast; ++i) {
                 const double P = per[i];
                 const double sc = std::nearbyint((P / bin) * scale);
-                const int64_t nb = period_bins(P, bin, o, width);
                 if (!(sc >= 1.0 && sc < 4294967296.0)) { fp.fast = false; break; }
                 const uint32_t S = (uint32_t)sc;
                 // the fast fold's largest bin, ((S - 1) >> fb) + 1, must stay inside n_bins
-                if ((int64_t)((S - 1u) >> fp.fb) + 1 > nb) { fp.fast = false; break; }
+                if ((int64_t)((S - 1u) >> fp.fb) + 1 > pc[i].nb) { fp.fast = false; break; }
             }
             double boxes = 0.0;
             for (int64_t i = p0; i < p1; ++i) {
                 const double P = per[i];
                 pc[i].f = 1.0 / P;
-                pc[i].nb = (int32_t)period_bins(P, bin, o, width);
                 pc[i].S = fp.fast ? (uint32_t)std::nearbyint((P / bin) * scale) : 0u;
                 for (int32_t kk : sh.dur)
                     if (kk < pc[i].nb) boxes += (double)(pc[i].nb - kk + 1);
@@ -710,10 +793,6 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             grid_boxes[k] += boxes;                  // per curve of this grid
             grid_trials[k] += (double)sd.n_periods * sh.dur.size();
         }
-      } catch (const std::bad_alloc&) {
-        grid_err[k] = BLS_E_NOMEM;
-        grid_msg[k] = "host allocation failed while preparing a grid";
-      }
     });
     for (int k = 0; k < n_grids; ++k)
         if (grid_err[k]) return fail(grid_err[k], "%s", grid_msg[k].c_str());
@@ -734,13 +813,14 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         for (int s = sbase[k]; s < sbase[k + 1]; ++s) seg_grid[s] = k;
 
     // ---- shared memory, tiles, work groups (costliest first) -------------------
-    bool modes[kModes] = {n_mode[0] > 0, n_mode[1] > 0, n_mode[2] > 0};
+    bool modes[kModes];
+    for (int m = 0; m < kModes; ++m) modes[m] = n_mode[m] > 0;
     size_t smem_mode[kModes];
     for (int m = 0; m < kModes; ++m) {
         size_t sm = e->tune.smem_per_cta > 0 ? (size_t)e->tune.smem_per_cta : kDefaultSmem[m];
         for (int s = 0; s < ns && modes[m]; ++s) {
             if (segs[s].empty_periods || grid_mode[seg_grid[s]][m] == 0) continue;
-            const size_t need = screen_bytes(m, segs[s].d.hist_len) + 16 +
+            const size_t need = screen_bytes(segs[s].d.hist_len) + 16 +
                                 period_bytes(m, segs[s].d.hist_len);
             if (need > sm) sm = need;
         }
@@ -760,7 +840,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     // (so the last work items of a launch are the cheapest)
     std::vector<WorkGroup> plan_groups[kModes];
     std::vector<int32_t> plan_tiles[kModes], plan_cap[kModes], plan_order[kModes];
-    int64_t n_items_mode[kModes] = {0, 0, 0};
+    int64_t n_items_mode[kModes] = {};
     std::vector<std::vector<int32_t>> members(n_grids);
     for (int m = 0; m < kModes; ++m) {
         plan_cap[m].assign(std::max(ns, 1), 1);
@@ -831,7 +911,8 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     }
 
     // ---- stage metadata and upload ---------------------------------------------
-    const int64_t n_items = n_items_mode[0] + n_items_mode[1] + n_items_mode[2];
+    int64_t n_items = 0;
+    for (int m = 0; m < kModes; ++m) n_items += n_items_mode[m];
     const size_t grid_bytes = (size_t)P_total * (8 + 8 + 4 + 4) + dur_all.size() * 4 + 64;
     // descriptors, per-curve spectrum offsets and grid bases (int64), then per
     // mode: groups, order, seg_tiles and seg_cap (int32 words)
@@ -947,7 +1028,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         a.seg_cap = dplan + plan_off[m][3];
         a.n_items = e->n_items_mode[m];
         a.tau = e->d_tau.as<double>();
-        a.pay_r = e->d_pay_r.as<uint32_t>();
+        a.pay_r = e->d_pay_r.as<int32_t>();
         a.r64 = e->d_r64.as<double>();
         a.iv64 = e->d_iv64.as<double>();
         a.period = dper;
@@ -987,7 +1068,9 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     in.trials = trials;
     in.h2d_bytes = h2d;
     in.ctas = ctas_total;
-    in.smem_per_cta = (int32_t)(modes[0] ? smem_mode[0] : modes[2] ? smem_mode[2] : smem_mode[1]);
+in.smem_per_cta = 0;
+    for (int m : {MODE_PAIR, MODE_UNIFORM, MODE_WIDE, MODE_EXACT, MODE_GENERAL})
+        if (in.smem_per_cta == 0 && modes[m]) in.smem_per_cta = (int32_t)smem_mode[m];
     in.uniform_curves = n_uniform;
     in.fast_fold_segments = fast_segments;
     in.spectrum = spec_total;

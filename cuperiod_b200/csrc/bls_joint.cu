@@ -299,13 +299,11 @@ __global__ void __launch_bounds__(kJThreads, 1) joint_kernel(JointArgs a) {
         const bool fast = seg.fast_fold != 0;
         const double f = a.freq[p];
         const uint32_t S = a.scale[p];
-        const int fb = seg.frac_bits;
-        const uint32_t fmask = (1u << fb) - 1u, mu = seg.margin_u, mphi = seg.margin_phi;
-        const uint32_t fr_span = (1u << fb) - 2u * mu, phi_span = 0u - 2u * mphi;
+        const FoldConst fc(seg.frac_bits, seg.margin_u, seg.margin_phi, fast);
         for (int j = tid; j < a.n_points; j += kJThreads) {
             const int k = a.band_of[j];
             const double x = a.tau[j];
-            int ind = fast ? fold_fast(x, f, S, fb, fmask, mu, fr_span, mphi, phi_span) : -1;
+            int ind = fold_fast(x, f, S, fc);
             if (ind < 0) ind = fold_exact(x, P, bin, seg.width);
             if (ind > nb) {
                 atomicOr(a.error_flag, JERR_BIN);

@@ -6,28 +6,24 @@
 //      period of the tile.  The phase bin is the reference's
 //      w = x - P*floor(x/P); ind = int(w/bin) + 1   (cuPeriod
 //      src/cuperiod/methods/_bls_core.py:369-376 / 536-538), computed by a fast
-//      FP64 path -- q = x * RN(1/P) rounded onto a 2^-32 grid, then one 32-bit
-//      multiply-high by P/bin -- whose result is used only when it is provably
-//      the reference's (the scaled phase is further than the combined rounding
-//      error from a cycle or bin edge); otherwise the reference's own IEEE chain
-//      runs.  With one weight for every point the bin sums are exact integers
-//      built with native 32-bit shared atomics only (64-bit and floating-point
-//      shared atomics are emulated on sm_100): each point adds the unsigned low
-//      13 bits and the signed high part of r_q (its centred flux*weight
-//      quantised to 24-27 bits of the curve's largest, by its length) to two
-//      words and 1 to the bin's count.  With per-point
-//      weights the two sums stay FP64.  A lane holds 8 time-consecutive points
-//      (the lanes of a warp 8 points apart, so their bins rarely collide);
-//   2. per period: applies the reference's wrap pad (_bls_core.py:377-381),
-//      turns the bins into prefix sums in place and writes an FP32 screen copy;
-//   3. sweeps every (duration, start) box.  An FP32 bound on the box objective
-//      -- maximising snr (or the log-likelihood) is maximising
-//      t^2 / (iv_in iv_out) (or t^2 / (iv_in iv_out^2)) with t = y_in - ybar iv_in
-//      -- discards every box that provably cannot be the period's best; the few
-//      that remain are evaluated with the reference's FP64 formulas
-//      (_bls_core.py:410-426) on the exact sums, and the winner is the first in
-//      (duration index, start) order among equals, as in the reference;
+//      FP64 path (FoldConst) whose result is used only when it is provably the
+//      reference's; otherwise the reference's own IEEE chain runs.  Bin sums are
+//      exact integers built with native 32-bit shared reductions only (64-bit and
+//      floating-point shared atomics are emulated on sm_100), except for curves of
+//      more than 2^17 points or of extreme scale, whose sums stay FP64.  A lane holds
+//      8 time-consecutive points (the lanes of a warp 8 points apart, so their bins
+//      rarely collide);
+//   2. per period: applies the reference's wrap pad (_bls_core.py:377-381), turns the
+//      bins into prefix sums in place and writes an FP32 screen copy;
+//   3. sweeps every (duration, start) box.  Each lane keeps the largest FP32 upper bound
+//      of the box objective it meets and where; the boxes that provably cannot be the
+//      period's best drop out against the largest lower bound, and the few left are
+//      evaluated with the reference's FP64 formulas (_bls_core.py:410-426) on the exact
+//      sums, the winner the first in (duration index, start) order among equals, as in
+//      the reference;
 //   4. writes the reference's seven per-period fields (_bls_core.py:443-460).
+// A period takes two CTA barriers: one between the scan's two passes (which also ends
+// the previous period's sweep), one before its sweep.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -52,10 +48,16 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr float kRel = 1.0f / 262144.0f;    // 2^-18: relative slack of FP32 key bounds
 constexpr int kCasLimit = 1 << 16;          // retries of one FP64 shared add
 constexpr int kNoBox = 1 << 29;             // duration slot past the last real duration
-// WIDE: the FP32 screen holds weights scaled by 2^-13 (fixed-point weights are
-// below 2^37 per point), the range of the FP64 mode's, so that the likelihood's
-// iv_in * iv_out^2 stays finite in FP32
-constexpr int kWideScreenShift = 13;
+constexpr int kList = 256;                  // candidates of one tile's periods
+constexpr int kRegBins = 9;                 // bins a lane holds in registers while scanning
+constexpr int kBoxBits = 20;                // box key: duration index << kBoxBits | start
+// Per-point weights: the FP32 screen holds them scaled by 2^-shift, their sum (below
+// 2^54, 2^60 and 2^54) at most 2^41, so that the likelihood's iv_in * iv_out^2 stays
+// below 2^126
+template <int MODE>
+__device__ __host__ constexpr int screen_shift() {
+    return MODE == MODE_WIDE ? 13 : (MODE == MODE_EXACT || MODE == MODE_GENERAL) ? 20 : 0;
+}
 
 struct TileShared {
     WorkItem item;
@@ -66,20 +68,19 @@ struct TileShared {
     uint32_t scale[kMaxTile];
     int32_t nb[kMaxTile];
     alignas(16) int32_t dur[kMaxDur + 4];   // padded with kNoBox; read four at a time
-    double win_v[kMaxTile];         // per period of the tile: the best box
-    int32_t win_di[kMaxTile];
-    int32_t win_n[kMaxTile];
-    uint32_t tot_w[6][kWarps];      // integer prefix scan: per-warp totals of each word
-    double tot_rd[kWarps];
-    double tot_wd[kWarps];
-    float red_f[kWarps];
+    uint32_t thr_bits[kMaxTile];    // per period: a lower bound of its best key (bits of a
+                                    // float >= 0)
+    int32_t win[kMaxTile];          // per period: the best box's key, -1 when there is none
+    long long tot[2][2][kWarps];    // scan: per-warp totals (by block parity, value)
+    double tot_d[2][kWarps];
     float red_t[kWarps];
     double red_v[kWarps];
-    int red_di[kWarps];
-    int red_n[kWarps];
+    int red_box[kWarps];
     int red_ne[kWarps];             // GENERAL scan: last non-empty bin per warp
+    uint32_t list[kList];           // candidates: period << 25 | box, standing for the four
+    int list_n;                     // widths of the box's group at its start
+    uint32_t rescan;                // bit q: period q needs every box in FP64
     int next;
-    uint32_t thr_bits;              // the sweep's shared threshold (bits of a float >= 0)
 };
 
 // Shared-memory accesses by 32-bit shared-space address (the hot loops compute
@@ -87,9 +88,8 @@ struct TileShared {
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
-template <int OFF>
 __device__ __forceinline__ void red_add_u32(uint32_t a, uint32_t v) {
-    asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(a), "r"(v), "n"(OFF) : "memory");
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_u32(uint32_t a) {
     uint32_t v;
@@ -112,14 +112,24 @@ __device__ __forceinline__ float2 ld_f2(uint32_t a) {
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
-template <int OFF>
-__device__ __forceinline__ float2 ld_f2_off(uint32_t a) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2+%3];" : "=f"(v.x), "=f"(v.y) : "r"(a), "n"(OFF));
-    return v;
-}
 __device__ __forceinline__ void st_f2(uint32_t a, float2 v) {
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+// {b.x - a.x, b.y - a.y} in one packed add, given {-a.x, -a.y}.
+__device__ __forceinline__ float2 add_f2(float2 b, float2 na) {
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(b.x), "f"(b.y), "f"(na.x), "f"(na.y));
+    return r;
+}
+
+// 1 / x to an ulp (0 for x above 2^126).
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
 // FP64 add to a shared-memory word by a bounded compare-and-swap loop in the
@@ -153,17 +163,9 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// (v, di, n) is better than (w, dj, m): larger objective, then earlier
-// (duration index, start) -- the reference's first-wins order.
-__device__ __forceinline__ bool better(double v, int di, int n, double w, int dj, int m) {
-    if (v > w) return true;
-    if (v < w || !(v == w)) return false;
-    return di < dj || (di == dj && n < m);
-}
-
 // Sums of one box inside and outside, in the reference's units: the reference
-// forms the outside as sum_y - y_in and sum_ivar - iv_in; WIDE curves take them
-// from the exact quantised totals instead (CurveDesc::rq_total).
+// forms the outside as sum_y - y_in and sum_ivar - iv_in; WIDE and EXACT curves take
+// them from the exact quantised totals instead (CurveDesc::rq_total).
 struct BoxSums {
     double y_in, iv_in, y_out, iv_out;
 };
@@ -181,240 +183,126 @@ __device__ __forceinline__ double box_objective(const BoxSums& s, const CurveDes
     return 0.5 * s.iv_in * depth * depth;
 }
 
-// Histogram layout of one period: one record per bin, prefix sums in place.
-//  UNIFORM: {A, B, C}, 12 bytes -- sum of the low 13 bits of r_q, sum of its
-//           signed high part, count (32-bit words);
-//  GENERAL: {R, W}, 16 bytes -- FP64 sums of the scaled centred flux*weight and
-//           of the scaled weight;
-//  WIDE:    {R0, R1, R2, I0, I1, I2}, 24 bytes -- the three parts of the
-//           fixed-point centred flux*weight and of the weight (32-bit words).
-// A period's region is padded to 16 bytes.
+// ---- histogram layout ---------------------------------------------------------
+// Integer modes keep kW planes of 32-bit words per period, one word per bin in each
+// (a bin is one word of a bank in every plane, so 32 random bins fall on 32 banks;
+// records of 8 or 16 bytes would use half or a quarter of them).  A point adds one
+// word to each plane, a native 32-bit reduction without a return value:
+//  PAIR:    {v, (v >> 20) << 12 | 1}: the quantised centred flux*weight v (28 bits
+//           and sign) modulo 2^32, and its top part above a count.  The second plane
+//           gives the count (a bin holds at most kPairMax points, host bound) and
+//           H = sum of v >> 20; the sum of v is 2^20 H plus what the first plane
+//           holds above 2^20 H modulo 2^32 -- at most kPairMax * 2^20 < 2^32, so no
+//           carry is lost;
+//  UNIFORM: {low 13 bits of v, v >> 13, 1}: as PAIR for any number of points in a bin;
+//  WIDE:    {r, r >> 19, i, i >> 19} of the 38-bit flux*weight and weight, at most
+//           kWideMax points in a bin;
+//  EXACT:   {r, r >> 15, r >> 30, i, i >> 15, i >> 30} of 61-bit values, any number
+//           of points (the same argument twice: 2^17 points x 2^15 <= 2^32).
+// GENERAL keeps 16-byte records of two FP64 sums.  The scan leaves exact prefix sums
+// in place: 64-bit integers in the words' first planes (PAIR / UNIFORM one, packed
+// as sum << kCountShift | count; WIDE / EXACT two), or the FP64 record.  One bin past
+// the last takes what the reference never reads.
 template <int MODE>
-__device__ __host__ constexpr int bin_bytes() {
-    return MODE == MODE_UNIFORM ? 12 : (MODE == MODE_WIDE ? 24 : 16);
+__device__ __host__ constexpr int point_words() {
+    return MODE == MODE_PAIR ? 2 : MODE == MODE_UNIFORM ? 3 : MODE == MODE_WIDE ? 4
+           : MODE == MODE_EXACT ? 6 : 0;
 }
 template <int MODE>
-__device__ __host__ __forceinline__ size_t hist_period_bytes(int hl) {
-    return ((size_t)hl * bin_bytes<MODE>() + 15) & ~size_t(15);
+__device__ __host__ constexpr bool one_weight() {
+    return MODE == MODE_PAIR || MODE == MODE_UNIFORM;
+}
+template <int MODE>
+__device__ __host__ __forceinline__ uint32_t plane_bytes(int hl) {
+    return 4u * (uint32_t)((hl + 1 + 3) & ~3);
+}
+template <int MODE>
+__device__ __host__ __forceinline__ uint32_t hist_period_bytes(int hl) {
+    return MODE == MODE_GENERAL ? 16u * (uint32_t)(hl + 1)
+                                : (uint32_t)point_words<MODE>() * plane_bytes<MODE>(hl);
+}
+// planes of the weight's words start here (WIDE / EXACT)
+template <int MODE>
+__device__ __host__ constexpr int weight_plane() {
+    return MODE == MODE_EXACT ? 3 : 2;
 }
 
-template <int MODE>
-struct PointRegs {
-    double x[kPts];
-    uint32_t lo[MODE == MODE_UNIFORM ? kPts : 1], hi[MODE == MODE_UNIFORM ? kPts : 1];
-    double rv[MODE == MODE_GENERAL ? kPts : 1], iv[MODE == MODE_GENERAL ? kPts : 1];
-    long long rq[MODE == MODE_WIDE ? kPts : 1], iq[MODE == MODE_WIDE ? kPts : 1];
+// One period's histogram: its address and the distance between planes.
+struct Hist {
+    uint32_t base, plane;
 };
 
-// WIDE: the three 32-bit parts of a fixed-point value (|v| < 2^37): low and
-// middle 13 bits, and the signed high part.
-__device__ __forceinline__ uint32_t wide_part(long long v, int k) {
-    return k == 0 ? (uint32_t)(v & ((1ll << kWideBits) - 1))
-                  : (k == 1 ? (uint32_t)((v >> kWideBits) & ((1ll << kWideBits) - 1))
-                            : (uint32_t)(int32_t)(v >> (2 * kWideBits)));
+__device__ __forceinline__ long long ld_planes(uint32_t a, uint32_t plane) {
+    return (long long)(((unsigned long long)ld_u32(a + plane) << 32) | ld_u32(a));
 }
-// WIDE: the value of three prefix parts.
-__device__ __forceinline__ long long wide_value(uint32_t p0, uint32_t p1, uint32_t p2) {
-    return (long long)(int32_t)p2 * (1ll << (2 * kWideBits)) +
-           (long long)p1 * (1ll << kWideBits) + (long long)p0;
+__device__ __forceinline__ void st_planes(uint32_t a, uint32_t plane, long long v) {
+    st_u32(a, (uint32_t)v);
+    st_u32(a + plane, (uint32_t)((unsigned long long)v >> 32));
 }
+
+// A sum kept as its value modulo 2^32 (`low`) and the sum of its points' values
+// shifted right by S (`high`): exact while the points' remainders add up below 2^32.
+template <int S>
+__device__ __forceinline__ long long join_sum(long long high, uint32_t low) {
+    return high * (1ll << S) + (long long)(uint32_t)(low - ((uint32_t)high << S));
+}
+
+// The sums of bin i: flux*weight and weight (packed with its count when there is one
+// weight).
 template <int MODE>
-__device__ __forceinline__ void add_point(uint32_t rec, const PointRegs<MODE>& p, int r,
-                                          int32_t* flag);
-
-template <int MODE, bool TAIL>
-__device__ __forceinline__ void load_points(const BatchArgs& a, const CurveDesc& c, int base,
-                                            PointRegs<MODE>& p) {
-    const int tid = threadIdx.x;
-    const double* __restrict__ tau = a.tau + c.point_off;
-#pragma unroll
-    for (int r = 0; r < kPts; ++r) {
-        const int j = base + r * kThreads + tid;
-        const bool ok = !TAIL || j < c.n_points;
-        p.x[r] = ok ? __ldg(tau + j) : -1.0;
-        if (MODE == MODE_UNIFORM) {
-            const uint32_t w = ok ? __ldg(a.pay_r + c.point_off + j) : 0u;
-            p.lo[r] = w & 0xffffu;
-            p.hi[r] = (uint32_t)((int32_t)w >> 16);    // signed high part
-        } else if (MODE == MODE_WIDE) {
-            const long long* rq = reinterpret_cast<const long long*>(a.r64) + c.point_off;
-            const long long* iq = reinterpret_cast<const long long*>(a.iv64) + c.point_off;
-            p.rq[r] = ok ? __ldg(rq + j) : 0ll;
-            p.iq[r] = ok ? __ldg(iq + j) : 0ll;
-        } else {
-            p.rv[r] = ok ? __ldg(a.r64 + c.point_off + j) : 0.0;
-            p.iv[r] = ok ? __ldg(a.iv64 + c.point_off + j) : 0.0;
-        }
-    }
-}
-
-template <int MODE, bool TAIL>
-__device__ __forceinline__ void fold_points(const TileShared& s, uint32_t hist_s,
-                                            const PointRegs<MODE>& p, int pt, int hl,
-                                            int32_t* flag) {
-    const SegmentDesc& g = s.seg;
-    const int fb = g.frac_bits;
-    const uint32_t fmask = (1u << fb) - 1u;
-    const uint32_t mu = g.margin_u;
-    const uint32_t fr_span = (1u << fb) - 2u * mu;
-    const uint32_t mphi = g.margin_phi;
-    const uint32_t phi_span = 0u - 2u * mphi;
-    const bool fast = g.fast_fold != 0;
-    const double bin = g.bin_duration;
-    const int width = g.width;
-    const uint32_t pbytes = (uint32_t)hist_period_bytes<MODE>(hl);
-    constexpr uint32_t kB = (uint32_t)bin_bytes<MODE>();
-    for (int q = 0; q < pt; ++q) {
-        const double f = s.freq[q];
-        const uint32_t S = s.scale[q];
-        const uint32_t hq = hist_s + (uint32_t)q * pbytes;
-        if (!TAIL && fast) {
-            // common case: every point's fast fold (fold_fast, inlined here) is
-            // provably the reference's bin, and the records take their atomics
-            // with no per-point test
-            uint32_t rec[kPts];
-            bool all_ok = true;
-#pragma unroll
-            for (int r = 0; r < kPts; ++r) {
-                const double qm = __fma_rn(p.x[r], f, 1572864.0);
-                const uint32_t phi = (uint32_t)__double2loint(qm);
-                const uint32_t v = __umulhi(phi, S);
-                all_ok &= ((phi - mphi) < phi_span) & (((v & fmask) - mu) < fr_span);
-                rec[r] = hq + kB + (v >> fb) * kB;
-            }
-            if (all_ok) {
-                if (MODE == MODE_UNIFORM) {
-                    // a lane's points are consecutive in time, so dense curves in
-                    // the wide-bin segments put several in one bin: each run of
-                    // equal bins adds its exact sums once (low parts of at most 8
-                    // points stay below 2^16), and lanes without a flush at a
-                    // step sit out that step's atomics and their bank conflicts
-                    uint32_t s_lo = p.lo[0], s_hi = p.hi[0], s_c = 1u;
-#pragma unroll
-                    for (int r = 1; r < kPts; ++r) {
-                        if (rec[r] != rec[r - 1]) {
-                            red_add_u32<0>(rec[r - 1], s_lo);
-                            red_add_u32<4>(rec[r - 1], s_hi);
-                            red_add_u32<8>(rec[r - 1], s_c);
-                            s_lo = 0u;
-                            s_hi = 0u;
-                            s_c = 0u;
-                        }
-                        s_lo += p.lo[r];
-                        s_hi += p.hi[r];
-                        s_c += 1u;
-                    }
-                    red_add_u32<0>(rec[kPts - 1], s_lo);
-                    red_add_u32<4>(rec[kPts - 1], s_hi);
-                    red_add_u32<8>(rec[kPts - 1], s_c);
-                } else {
-#pragma unroll
-                    for (int r = 0; r < kPts; ++r) add_point<MODE>(rec[r], p, r, flag);
-                }
-                continue;
-            }
-        }
-        // 1. the fast fold of all points, straight-line (-1: near an edge, -2: skip)
-        int ind[kPts];
-        bool miss = false;
-#pragma unroll
-        for (int r = 0; r < kPts; ++r) {
-            ind[r] = fast ? fold_fast(p.x[r], f, S, fb, fmask, mu, fr_span, mphi, phi_span) : -1;
-            if (TAIL && p.x[r] < 0.0) ind[r] = -2;
-            miss |= ind[r] == -1;
-        }
-        // 2. rare: the reference's IEEE chain for points near a cycle or bin edge
-        if (miss) {
-            const double P = s.per[q];
-            const int nbq = s.nb[q];
-#pragma unroll
-            for (int r = 0; r < kPts; ++r) {
-                if (ind[r] == -1) {
-                    const int e = fold_exact(p.x[r], P, bin, width);
-                    ind[r] = e > nbq ? -2 : e;        // a bin the reference never reads
-                }
-            }
-        }
-        // 3. accumulate: one record address per point feeds all its atomics
-#pragma unroll
-        for (int r = 0; r < kPts; ++r) {
-            if (ind[r] < 0) continue;
-            add_point<MODE>(hq + (uint32_t)ind[r] * (uint32_t)bin_bytes<MODE>(), p, r, flag);
-        }
-    }
-}
-
-// One point's contribution to its bin record.
-template <int MODE>
-__device__ __forceinline__ void add_point(uint32_t rec, const PointRegs<MODE>& p, int r,
-                                          int32_t* flag) {
-    if (MODE == MODE_UNIFORM) {
-        red_add_u32<0>(rec, p.lo[r]);
-        red_add_u32<4>(rec, p.hi[r]);
-        red_add_u32<8>(rec, 1u);
+__device__ __forceinline__ void bin_sums(const Hist& h, int i, long long& r, long long& w) {
+    const uint32_t a = h.base + 4u * (uint32_t)i;
+    w = 0;
+    if (MODE == MODE_PAIR) {
+        const uint32_t lo = ld_u32(a), b = ld_u32(a + h.plane);
+        const long long sum = join_sum<32 - kPairBits>((int32_t)b >> kPairBits, lo);
+        r = (sum << kCountShift) + (long long)(b & ((1u << kPairBits) - 1u));
+    } else if (MODE == MODE_UNIFORM) {
+        const long long sum = (long long)(int32_t)ld_u32(a + h.plane) * (1ll << kHalfBits) +
+                              (long long)ld_u32(a);
+        r = (sum << kCountShift) + (long long)ld_u32(a + 2 * h.plane);
     } else if (MODE == MODE_WIDE) {
-        red_add_u32<0>(rec, wide_part(p.rq[r], 0));
-        red_add_u32<4>(rec, wide_part(p.rq[r], 1));
-        red_add_u32<8>(rec, wide_part(p.rq[r], 2));
-        red_add_u32<12>(rec, wide_part(p.iq[r], 0));
-        red_add_u32<16>(rec, wide_part(p.iq[r], 1));
-        red_add_u32<20>(rec, wide_part(p.iq[r], 2));
+        r = join_sum<kWideBits>((int32_t)ld_u32(a + h.plane), ld_u32(a));
+        w = join_sum<kWideBits>((int32_t)ld_u32(a + 3 * h.plane), ld_u32(a + 2 * h.plane));
     } else {
-        shared_add_f64(rec, p.rv[r], flag);
-        shared_add_f64(rec + 8, p.iv[r], flag);
+        // the middle sum modulo 2^32 is completed by the high one, then completes the low
+        r = join_sum<kExactBits>(join_sum<kExactBits>((int32_t)ld_u32(a + 2 * h.plane),
+                                                      ld_u32(a + h.plane)),
+                                 ld_u32(a));
+        w = join_sum<kExactBits>(join_sum<kExactBits>((int32_t)ld_u32(a + 5 * h.plane),
+                                                      ld_u32(a + 4 * h.plane)),
+                                 ld_u32(a + 3 * h.plane));
     }
 }
 
-// WIDE: exact prefixes at bin i of the centred flux*weight and of the weight.
-__device__ __forceinline__ long long wide_prefix_r(uint32_t hq, int i) {
-    const uint32_t rec = hq + (uint32_t)i * 24u;
-    return wide_value(ld_u32(rec), ld_u32(rec + 4), ld_u32(rec + 8));
+// Prefix sums at bin i, as the scan left them.
+__device__ __forceinline__ long long prefix_r(const Hist& h, int i) {
+    return ld_planes(h.base + 4u * (uint32_t)i, h.plane);
 }
-__device__ __forceinline__ long long wide_prefix_i(uint32_t hq, int i) {
-    const uint32_t rec = hq + (uint32_t)i * 24u + 12u;
-    return wide_value(ld_u32(rec), ld_u32(rec + 4), ld_u32(rec + 8));
-}
-
-// Exact prefix of r_q at bin i from a UNIFORM record's two prefix words.
-__device__ __forceinline__ long long prefix_r(uint32_t hq, int i) {
-    const uint32_t rec = hq + (uint32_t)i * 12u;
-    return (long long)(int32_t)ld_u32(rec + 4) * (1ll << kHalfBits) + (long long)ld_u32(rec);
-}
-__device__ __forceinline__ uint32_t prefix_c(uint32_t hq, int i) {
-    return ld_u32(hq + (uint32_t)i * 12u + 8u);
-}
-
-// Exact sums of box (n, d) in the reference's units from one period's prefixes
-// (hq: the period's region).
 template <int MODE>
-__device__ __forceinline__ BoxSums box_sums(uint32_t hq, const CurveDesc& cv, int n, int d);
-
-// The reference's objective of box (n, d), out of line: the sweep reaches it
-// rarely and keeps its own loop small.
-template <int MODE>
-__device__ __noinline__ double exact_objective(uint32_t hq, const CurveDesc* cv, int n, int d,
-                                               int obj) {
-    return box_objective(box_sums<MODE>(hq, *cv, n, d), *cv, obj);
+__device__ __forceinline__ long long prefix_w(const Hist& h, int i) {
+    return ld_planes(h.base + 4u * (uint32_t)i + weight_plane<MODE>() * h.plane, h.plane);
 }
 
+// Exact sums of box (n, d) in the reference's units from one period's prefixes.
 template <int MODE>
-__device__ __forceinline__ BoxSums box_sums(uint32_t hq, const CurveDesc& cv, int n, int d) {
+__device__ __forceinline__ BoxSums box_sums(const Hist& h, const CurveDesc& cv, int n, int d) {
     BoxSums b;
-    if (MODE == MODE_UNIFORM) {
-        const double cnt = (double)(prefix_c(hq, n + d) - prefix_c(hq, n));
+    if (one_weight<MODE>()) {
+        const long long v = prefix_r(h, n + d) - prefix_r(h, n);
+        const double cnt = (double)(v & ((1ll << kCountShift) - 1));
         b.iv_in = cnt * cv.w_uniform;
-        b.y_in = ldexp((double)(prefix_r(hq, n + d) - prefix_r(hq, n)), -cv.e_r) +
-                 cv.center * cnt;
-    } else if (MODE == MODE_WIDE) {
-        const long long qi = wide_prefix_i(hq, n + d) - wide_prefix_i(hq, n);
-        const long long qr = wide_prefix_r(hq, n + d) - wide_prefix_r(hq, n);
+        b.y_in = ldexp((double)(v >> kCountShift), -cv.e_r) + cv.center * cnt;
+    } else if (MODE != MODE_GENERAL) {
+        const long long qi = prefix_w<MODE>(h, n + d) - prefix_w<MODE>(h, n);
+        const long long qr = prefix_r(h, n + d) - prefix_r(h, n);
         b.iv_in = ldexp((double)qi, -cv.e_i);
         b.y_in = ldexp((double)qr, -cv.e_r) + cv.ybar * b.iv_in;
         b.iv_out = ldexp((double)(cv.iq_total - qi), -cv.e_i);
         b.y_out = ldexp((double)(cv.rq_total - qr), -cv.e_r) + cv.ybar * b.iv_out;
         return b;
     } else {
-        const uint32_t r1 = hq + (uint32_t)(n + d) * 16u, r0 = hq + (uint32_t)n * 16u;
+        const uint32_t r1 = h.base + (uint32_t)(n + d) * 16u, r0 = h.base + (uint32_t)n * 16u;
         b.iv_in = ldexp(ld_f64(r1 + 8) - ld_f64(r0 + 8), -cv.e_i);
         b.y_in = ldexp(ld_f64(r1) - ld_f64(r0), -cv.e_r) + cv.ybar * b.iv_in;
     }
@@ -423,8 +311,400 @@ __device__ __forceinline__ BoxSums box_sums(uint32_t hq, const CurveDesc& cv, in
     return b;
 }
 
+// The reference's objective of box (n, d), out of line: reached rarely.
 template <int MODE, int OBJ>
-__global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
+__device__ __noinline__ double exact_objective(uint32_t base, uint32_t plane, const CurveDesc* cv,
+                                               int n, int d) {
+    return box_objective(box_sums<MODE>(Hist{base, plane}, *cv, n, d), *cv, OBJ);
+}
+
+// The better of two boxes by exact objective: larger, then the earlier (duration
+// index, start) -- the reference's first-wins order.  key < 0: no box.
+__device__ __forceinline__ void keep_better(double& v, int& key, double ov, int okey) {
+    if (okey >= 0 && ov > -CUDART_INF && (key < 0 || ov > v || (ov == v && okey < key))) {
+        v = ov;
+        key = okey;
+    }
+}
+
+// ---- fold -----------------------------------------------------------------------
+
+// NR time-consecutive points of one lane: the time offset and, ready to add, the
+// words (or FP64 sums) of the point's contribution.
+template <int MODE, int NR>
+struct PointRegs {
+    static constexpr int kW = point_words<MODE>();
+    double x[NR];
+    uint32_t w[kW > 0 ? NR : 1][kW > 0 ? kW : 1];
+    double rv[kW > 0 ? 1 : NR], iv[kW > 0 ? 1 : NR];
+};
+
+// The points of this lane in the block of kThreads * NR points at `base`: slot
+// base + r * kThreads + tid of a full chunk (stored lane-interleaved), time index
+// base + tid * NR + r of the tail.  A tail slot past the last point repeats that
+// point's time with nothing to add.
+template <int MODE, int NR, bool TAIL>
+__device__ __forceinline__ void load_points(const BatchArgs& a, const CurveDesc& c, int base,
+                                            PointRegs<MODE, NR>& p) {
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        int j = TAIL ? base + tid * NR + r : base + r * kThreads + tid;
+        const bool ok = !TAIL || j < c.n_points;
+        if (TAIL) j = min(j, c.n_points - 1);
+        const int64_t slot = c.point_off + j;
+        p.x[r] = __ldg(a.tau + slot);
+        if constexpr (one_weight<MODE>()) {
+            const int32_t v = ok ? __ldg(a.pay_r + slot) : 0;
+            if constexpr (MODE == MODE_PAIR) {
+                p.w[r][0] = (uint32_t)v;
+                p.w[r][1] = ((uint32_t)(v >> (32 - kPairBits)) << kPairBits) | (ok ? 1u : 0u);
+            } else {
+                p.w[r][0] = (uint32_t)v & ((1u << kHalfBits) - 1u);
+                p.w[r][1] = (uint32_t)(v >> kHalfBits);
+                p.w[r][2] = ok ? 1u : 0u;
+            }
+        } else if constexpr (MODE != MODE_GENERAL) {
+            const long long rq = ok ? __ldg(reinterpret_cast<const long long*>(a.r64) + slot) : 0ll;
+            const long long iq =
+                ok ? __ldg(reinterpret_cast<const long long*>(a.iv64) + slot) : 0ll;
+            constexpr int kStep = MODE == MODE_WIDE ? kWideBits : kExactBits;
+            constexpr int kHalf = point_words<MODE>() / 2;
+#pragma unroll
+            for (int k = 0; k < kHalf; ++k) {
+                p.w[r][k] = (uint32_t)(rq >> (k * kStep));
+                p.w[r][kHalf + k] = (uint32_t)(iq >> (k * kStep));
+            }
+        } else {
+            p.rv[r] = ok ? __ldg(a.r64 + slot) : 0.0;
+            p.iv[r] = ok ? __ldg(a.iv64 + slot) : 0.0;
+        }
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void add_words(uint32_t rec, uint32_t plane, const uint32_t (&w)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) red_add_u32(rec + k * plane, w[k]);
+}
+
+// The bin of a point whose fast fold is not provably the reference's: the reference's
+// IEEE chain, out of line (2 points in 10^4 of a survey cadence); what the reference
+// never reads (past n_bins) goes to the bin past the last, hl.
+__device__ __noinline__ int exact_bin(double x, double P, double bin, int width, int nb, int hl) {
+    const int e = fold_exact(x, P, bin, width);
+    return e > nb ? hl : e;
+}
+
+// Fold this lane's NR points into the histograms of the tile's pt periods.
+// Bound by the shared-memory pipe (the reductions and their bank conflicts: 3.8
+// wavefronts each on a survey cadence), then by issue.
+// MERGE: a lane's points are consecutive in time, so where a bin is wider than the
+// sampling each run of equal bins adds its sums once; elsewhere the comparisons only
+// cost (one-weight batch of 16 curves, 50,000 periods: 27.7 ms without, 29.8 with).
+template <int MODE, int NR, bool TAIL, bool MERGE>
+__device__ __forceinline__ void fold_points(const TileShared& s, uint32_t hist_s,
+                                            const PointRegs<MODE, NR>& p, int pt, int hl,
+                                            int32_t* flag) {
+    const SegmentDesc& g = s.seg;
+    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, g.fast_fold != 0);
+    const uint32_t plane = plane_bytes<MODE>(hl);
+    const uint32_t pbytes = hist_period_bytes<MODE>(hl);
+    constexpr uint32_t kB = MODE == MODE_GENERAL ? 16u : 4u;
+    uint32_t hq = hist_s;
+    for (int q = 0; q < pt; ++q, hq += pbytes) {
+        const double f = s.freq[q];
+        const uint32_t S = s.scale[q];
+        uint32_t rec[NR], worst = 0u;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint32_t v = fc.position(p.x[r], f, S);
+            worst = max(worst, fc.edge(v));
+            rec[r] = hq + kB + (v >> fc.fb) * kB;
+        }
+        if (worst >= fc.limit) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                if (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit)
+                    rec[r] = hq + kB * (uint32_t)exact_bin(p.x[r], s.per[q], g.bin_duration,
+                                                           g.width, s.nb[q], hl);
+        }
+        if constexpr (MODE == MODE_GENERAL) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                shared_add_f64(rec[r], p.rv[r], flag);
+                shared_add_f64(rec[r] + 8, p.iv[r], flag);
+            }
+        } else if constexpr (!MERGE) {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) add_words(rec[r], plane, p.w[r]);
+        } else {
+            constexpr int kW = point_words<MODE>();
+            uint32_t run[kW];
+#pragma unroll
+            for (int k = 0; k < kW; ++k) run[k] = p.w[0][k];
+#pragma unroll
+            for (int r = 1; r < NR; ++r) {
+                if (rec[r] != rec[r - 1]) {
+                    add_words<kW>(rec[r - 1], plane, run);
+#pragma unroll
+                    for (int k = 0; k < kW; ++k) run[k] = 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < kW; ++k) run[k] += p.w[r][k];
+            }
+            add_words<kW>(rec[NR - 1], plane, run);
+        }
+    }
+}
+
+// Fold the block of kThreads * NR points at `base`; lanes past the tail's last
+// point sit it out.
+template <int MODE, int NR, bool TAIL, bool MERGE>
+__device__ __forceinline__ void fold_block(const BatchArgs& a, const TileShared& s,
+                                           uint32_t hist_s, int base, int pt, int hl) {
+    if (TAIL && base + (int)threadIdx.x * NR >= s.curve.n_points) return;
+    PointRegs<MODE, NR> p;
+    load_points<MODE, NR, TAIL>(a, s.curve, base, p);
+    fold_points<MODE, NR, TAIL, MERGE>(s, hist_s, p, pt, hl, a.error_flag);
+}
+
+// ---- prefix sums -----------------------------------------------------------------
+
+// The FP32 screen copy of one prefix: {t, weight} and, one weight, the magnitude that
+// bounds t's rounding error.
+template <int MODE>
+__device__ __forceinline__ float2 screen_record(long long r, long long w, float cfrac, float& tm) {
+    if (one_weight<MODE>()) {
+        // the screen's t is centred by ybar itself: the stored prefix minus
+        // center_frac per point, in FP32.  It is within 2^-23 tm of the exact value
+        // (pf and t round once each, cf <= 2^16 twice), so a box's t is within
+        // 1.5 * 2^-22 of the largest tm, inside Et
+        const float cnt = (float)(uint32_t)(r & ((1ll << kCountShift) - 1));
+        const float pf = (float)(r >> kCountShift);
+        const float cf = cfrac * cnt;
+        const float t = pf - cf;
+        tm = fmaxf(fabsf(pf), fabsf(t)) + fabsf(cf);
+        return make_float2(t, cnt);
+    }
+    const float t = (float)r;
+    tm = fabsf(t);
+    // exact scaling by a power of two
+    return make_float2(t, (float)w * (MODE == MODE_EXACT ? 0x1p-20f : 0x1p-13f));
+}
+
+// Integer modes: the wrap pad (bins 1..o repeated in nb-o..nb-1, _bls_core.py:377-381)
+// and prefix sums of one period, in place, with the FP32 screen copy.  Returns after
+// the period's second barrier; `first` runs after its first one (what the previous
+// period left to do once every warp has finished its sweep).  A lane owns K
+// consecutive bins, K odd so that the lanes' words sit in distinct banks, and holds
+// their running sums in registers between the two barriers, so each bin is read once
+// and written once; more than kThreads * kRegBins bins go in several such blocks.
+template <int MODE, typename F>
+__device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32_t scr_s, int L,
+                                            int o, F&& first) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nb = L - 1;
+    constexpr int kW = point_words<MODE>();
+    constexpr bool kTwo = !one_weight<MODE>();
+    const bool single = L <= kThreads * kRegBins;
+    // several blocks, or a pad that overlaps its source: copied before the scan (the
+    // overlapping one by one thread in the reference's order); else the lane that owns
+    // a pad bin reads the bin it repeats (no word changes before the first barrier)
+    const bool overlap = nb - o <= o;
+    const bool copied = overlap || !single;
+    if (copied) {
+        auto copy_bin = [&](int dst, int src) {
+            if (dst < 0 || dst >= s.seg.width || dst > s.seg.hist_len || src > s.seg.hist_len) return;
+            const uint32_t rd = h.base + 4u * (uint32_t)dst, rs = h.base + 4u * (uint32_t)src;
+#pragma unroll
+            for (int k = 0; k < kW; ++k) st_u32(rd + k * h.plane, ld_u32(rs + k * h.plane));
+        };
+        if (overlap) {
+            if (tid == 0)
+                for (int k = 0; k < o; ++k) copy_bin(nb - o + k, 1 + k);
+        } else {
+            for (int k = tid; k < o; k += kThreads) copy_bin(nb - o + k, 1 + k);
+        }
+        __syncthreads();
+    }
+    const int K = single ? (((L + kThreads - 1) / kThreads) | 1) : kRegBins;
+    const float cfrac = (float)s.curve.center_frac;
+    long long carry_r = 0, carry_w = 0;
+    float tmax = 0.0f;
+    int par = 0;
+    for (int b0 = 0; b0 < L; b0 += kThreads * K, par ^= 1) {
+        const int l0 = b0 + tid * K;
+        long long ar[kRegBins], aw[kTwo ? kRegBins : 1];
+        long long run_r = 0, run_w = 0;
+#pragma unroll
+        for (int r = 0; r < kRegBins; ++r) {
+            if (r < K) {
+                const int i = l0 + r;
+                if (i < L) {
+                    const int src = !copied && i >= nb - o && i < nb ? i - (nb - o) + 1 : i;
+                    long long br, bw;
+                    bin_sums<MODE>(h, src, br, bw);
+                    run_r += br;
+                    run_w += bw;
+                }
+                ar[r] = run_r;
+                if (kTwo) aw[kTwo ? r : 0] = run_w;
+            }
+        }
+        long long in_r = run_r, in_w = run_w;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const long long x = __shfl_up_sync(kFull, in_r, k);
+            if (lane >= k) in_r += x;
+            if (kTwo) {
+                const long long y = __shfl_up_sync(kFull, in_w, k);
+                if (lane >= k) in_w += y;
+            }
+        }
+        if (lane == 31) {
+            s.tot[par][0][warp] = in_r;
+            if (kTwo) s.tot[par][1][warp] = in_w;
+        }
+        __syncthreads();
+        if (b0 == 0) first();
+        long long off_r = carry_r + in_r - run_r, off_w = carry_w + in_w - run_w;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const long long t = s.tot[par][0][w];
+            carry_r += t;
+            if (w < warp) off_r += t;
+            if (kTwo) {
+                const long long u = s.tot[par][1][w];
+                carry_w += u;
+                if (w < warp) off_w += u;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRegBins; ++r) {
+            const int i = l0 + r;
+            if (r < K && i < L) {
+                const uint32_t a = h.base + 4u * (uint32_t)i;
+                const long long vr = off_r + ar[r], vw = kTwo ? off_w + aw[kTwo ? r : 0] : 0;
+                st_planes(a, h.plane, vr);
+                if (kTwo) st_planes(a + weight_plane<MODE>() * h.plane, h.plane, vw);
+                float tm;
+                st_f2(scr_s + 8u * (uint32_t)i, screen_record<MODE>(vr, vw, cfrac, tm));
+                tmax = fmaxf(tmax, tm);
+            }
+        }
+    }
+    tmax = warp_max(tmax);
+    if (lane == 0) s.red_t[warp] = tmax;
+    // sentinel records past the last bin: t = NaN fails every screen
+    if (tid < kScreenPad) st_f2(scr_s + 8u * (uint32_t)(L + tid), make_float2(CUDART_NAN_F, 0.0f));
+    __syncthreads();
+}
+
+// GENERAL: the same on FP64 sums.  The lanes' partial sums associate differently from
+// one running sum, so at a lane boundary an empty bin could move the FP64 prefix by a
+// rounding; the reference's running sum keeps it exactly constant, which makes boxes
+// that differ only by empty end bins tie exactly (first wins), so the lanes copy the
+// prefix of the last non-empty bin into their leading empty bins (a third barrier).
+template <typename F>
+__device__ __forceinline__ void scan_period_f64(TileShared& s, const Hist& h, uint32_t scr_s, int L,
+                                                int o, F&& first) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nb = L - 1;
+    auto copy_bin = [&](int dst, int src) {
+        if (dst < 0 || dst >= s.seg.width || dst > s.seg.hist_len || src > s.seg.hist_len) return;
+        const uint32_t rd = h.base + 16u * (uint32_t)dst, rs = h.base + 16u * (uint32_t)src;
+        st_f64(rd, ld_f64(rs));
+        st_f64(rd + 8, ld_f64(rs + 8));
+    };
+    if (nb - o <= o) {
+        if (tid == 0)
+            for (int k = 0; k < o; ++k) copy_bin(nb - o + k, 1 + k);
+    } else {
+        for (int k = tid; k < o; k += kThreads) copy_bin(nb - o + k, 1 + k);
+    }
+    __syncthreads();
+    const int K = ((L + kThreads - 1) / kThreads) | 1;
+    const int l0 = min(L, tid * K), l1 = min(L, l0 + K);
+    double ur = 0.0, uw = 0.0;
+    int lead = 0, last_ne = -1;     // leading empty bins, last non-empty bin of the lane
+    for (int i = l0; i < l1; ++i) {
+        const uint32_t rec = h.base + 16u * (uint32_t)i;
+        const double br = ld_f64(rec), bw = ld_f64(rec + 8);
+        ur += br;
+        uw += bw;
+        if (br != 0.0 || bw != 0.0) last_ne = i;
+        else if (last_ne < 0) ++lead;
+    }
+    double ir = ur, iw = uw;
+    int im = last_ne;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const double xr = __shfl_up_sync(kFull, ir, k);
+        const double xw = __shfl_up_sync(kFull, iw, k);
+        const int xm = __shfl_up_sync(kFull, im, k);
+        if (lane >= k) {
+            ir += xr;
+            iw += xw;
+            im = max(im, xm);
+        }
+    }
+    double rr = __shfl_up_sync(kFull, ir, 1), rw = __shfl_up_sync(kFull, iw, 1);
+    last_ne = __shfl_up_sync(kFull, im, 1);
+    if (lane == 0) {
+        rr = rw = 0.0;
+        last_ne = -1;
+    }
+    if (lane == 31) {
+        s.tot_d[0][warp] = ir;
+        s.tot_d[1][warp] = iw;
+        s.red_ne[warp] = im;
+    }
+    __syncthreads();
+    first();
+    for (int w = 0; w < warp; ++w) {
+        rr += s.tot_d[0][w];
+        rw += s.tot_d[1][w];
+        last_ne = max(last_ne, s.red_ne[w]);
+    }
+    float tmax = 0.0f;
+    for (int i = l0; i < l1; ++i) {
+        const uint32_t rec = h.base + 16u * (uint32_t)i;
+        rr += ld_f64(rec);
+        rw += ld_f64(rec + 8);
+        st_f64(rec, rr);
+        st_f64(rec + 8, rw);
+        st_f2(scr_s + 8u * (uint32_t)i, make_float2((float)rr, (float)(rw * 0x1p-20)));
+        tmax = fmaxf(tmax, fabsf((float)rr));
+    }
+    tmax = warp_max(tmax);
+    if (lane == 0) s.red_t[warp] = tmax;
+    if (tid < kScreenPad) st_f2(scr_s + 8u * (uint32_t)(L + tid), make_float2(CUDART_NAN_F, 0.0f));
+    __syncthreads();
+    if (lead > 0 && last_ne >= 0) {
+        const uint32_t rs = h.base + 16u * (uint32_t)last_ne;
+        const double pr = ld_f64(rs), pw = ld_f64(rs + 8);
+        for (int i = l0; i < l0 + lead; ++i) {
+            const uint32_t rec = h.base + 16u * (uint32_t)i;
+            st_f64(rec, pr);
+            st_f64(rec + 8, pw);
+            st_f2(scr_s + 8u * (uint32_t)i, make_float2((float)pr, (float)(pw * 0x1p-20)));
+        }
+    }
+    __syncthreads();
+}
+
+// ---- the search --------------------------------------------------------------------
+
+// Persistent search; see the head of this file.  One weight runs three CTAs an SM (80
+// registers), per-point weights two.  Bound by latency between its barriers with 24 (16)
+// resident warps: neither issue nor the shared-memory pipe is above two thirds busy.
+// 96 curves of the batched workload (mean 9,900 points, 50,000 periods): 152.8 ms with
+// three words a point, five barriers a period and a screened sweep, 128.3 ms as built;
+// 16 curves with per-point errors 52.7 -> 40.7 ms (38-bit weights), 8 with outlying
+// errors 56.2 -> 29.3 ms (FP64 sums by compare-and-swap before).
+template <int MODE, int OBJ>
+__global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
     bls_search_kernel(BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared s;
@@ -470,12 +750,15 @@ __global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
             w.p_count = min(cap, s.seg.n_periods - w.p_begin);
             s.item = w;
             s.curve = a.curves[w.curve];
+            s.list_n = 0;
+            s.rescan = 0u;
         }
         __syncthreads();
         const int pt = s.item.p_count;
         const int hl = s.seg.hist_len;
         const int n_dur = s.seg.n_dur;
-        if (pt < 1 || pt > kMaxTile || n_dur < 0 || n_dur > kMaxDur || hl < 2) {
+        if (pt < 1 || pt > kMaxTile || n_dur < 0 || n_dur > kMaxDur || hl < 2 ||
+            hl >= (1 << kBoxBits)) {
             if (tid == 0) atomicExch(a.error_flag, 1);
             continue;
         }
@@ -485,9 +768,9 @@ __global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
             s.freq[tid] = a.freq[g0 + tid];
             s.scale[tid] = a.scale[g0 + tid];
             s.nb[tid] = a.nbins[g0 + tid];
+            s.thr_bits[tid] = 0u;
         }
         if (tid < kMaxDur + 4) s.dur[tid] = tid < n_dur ? a.dur_bins[s.seg.dur_off + tid] : kNoBox;
-        __syncthreads();
 
         double* out = a.out + s.curve.out_off + g0;
         const int64_t ostride = a.out_stride;
@@ -500,7 +783,8 @@ __global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
         }
 
         // ---- 1. fold ---------------------------------------------------------
-        const size_t pbytes = hist_period_bytes<MODE>(hl);
+        const uint32_t pbytes = hist_period_bytes<MODE>(hl);
+        const uint32_t plane = plane_bytes<MODE>(hl);
         const uint32_t smem_s = smem_addr(smem);
         {
             const int n16 = (int)((pt * pbytes) / 16);
@@ -511,522 +795,299 @@ __global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
         {
             const int n = s.curve.n_points;
             int base = 0;
-            for (; base + kChunk <= n; base += kChunk) {
-                PointRegs<MODE> p;
-                load_points<MODE, false>(a, s.curve, base, p);
-                fold_points<MODE, false>(s, smem_s, p, pt, hl, a.error_flag);
-            }
-            if (base < n) {
-                PointRegs<MODE> p;
-                load_points<MODE, true>(a, s.curve, base, p);
-                fold_points<MODE, true>(s, smem_s, p, pt, hl, a.error_flag);
-            }
+            if (MODE != MODE_GENERAL && s.seg.bin_duration > 1.5f * s.curve.gap)
+                for (; base + kChunk <= n; base += kChunk)
+                    fold_block<MODE, kPts, false, true>(a, s, smem_s, base, pt, hl);
+            else
+                for (; base + kChunk <= n; base += kChunk)
+                    fold_block<MODE, kPts, false, false>(a, s, smem_s, base, pt, hl);
+            // the tail: fewer points a lane when few are left, so that more warps
+            // share them
+            const int left = n - base;
+            if (left > 4 * kThreads)
+                fold_block<MODE, kPts, true, false>(a, s, smem_s, base, pt, hl);
+            else if (left > 2 * kThreads)
+                fold_block<MODE, 4, true, false>(a, s, smem_s, base, pt, hl);
+            else if (left > 0)
+                fold_block<MODE, 2, true, false>(a, s, smem_s, base, pt, hl);
         }
         __syncthreads();
 
-        // ---- 2-3. per period: pad, prefix, sweep, reduce ------------------------
-        const size_t hist_bytes = (size_t)pt * pbytes;               // multiple of 16
-        const uint32_t scr_s = smem_s + (uint32_t)hist_bytes;        // FP32 screen copy
+        // ---- 2-3. per period: pad, prefix, sweep --------------------------------
+        const uint32_t scr_s = smem_s + (uint32_t)pt * pbytes;       // FP32 screen copy
         const CurveDesc& cv = s.curve;
-        constexpr int obj = OBJ;          // 0 snr, 1 log-likelihood
-        const int e_r = cv.e_r, e_i = cv.e_i;
         const int o = s.seg.oversample;
-        constexpr uint32_t kRec = (uint32_t)bin_bytes<MODE>();
-        constexpr int kNW = MODE == MODE_UNIFORM ? 3 : (MODE == MODE_WIDE ? 6 : 1);   // words
+        auto hist = [&](int q) { return Hist{smem_s + (uint32_t)q * pbytes, plane}; };
+
+        // what a lane keeps of its sweep of one period: its best and second-best group
+        // (four widths at one start) by screened key, and the best group's place
+        float best = -1.0f, second = -1.0f;
+        int place = 0;
+        // Once every sweep of period q is done its threshold is final: lanes whose best
+        // group reaches it are candidates.  A second group that reaches it too (ties
+        // across groups of one lane) or a full list leaves the period to the CTA.
+        auto submit = [&](int q) {
+            const float Lc = __uint_as_float(s.thr_bits[q]);
+            if (best >= Lc) {
+                const int pos = second >= Lc ? kList : atomicAdd(&s.list_n, 1);
+                if (pos < kList) s.list[pos] = ((uint32_t)q << 25) | (uint32_t)place;
+                else atomicOr(&s.rescan, 1u << q);
+            }
+            best = second = -1.0f;
+        };
 
         for (int q = 0; q < pt; ++q) {
             const int nb = s.nb[q];
             const int L = nb + 1;
-            const uint32_t hq = smem_s + (uint32_t)(q * pbytes);
-            auto copy_bin = [&](int dst, int src) {
-                if (dst >= 0 && dst < s.seg.width && dst < hl && src < hl) {
-                    const uint32_t rd = hq + (uint32_t)dst * kRec, rs = hq + (uint32_t)src * kRec;
-                    if (MODE != MODE_GENERAL) {
-#pragma unroll
-                        for (int w = 0; w < kNW; ++w) st_u32(rd + 4 * w, ld_u32(rs + 4 * w));
-                    } else {
-                        st_f64(rd, ld_f64(rs));
-                        st_f64(rd + 8, ld_f64(rs + 8));
-                    }
-                }
-            };
-
-            // wrap pad: bins 1..o copied to nb-o..nb-1 (_bls_core.py:377-381).  When
-            // the two ranges overlap one thread copies in the reference's order;
-            // otherwise the warp that owns each destination copies it in pass 1
-            // (the source bins are not written before pass 2).
-            const bool overlap = nb - o <= o;
-            if (overlap) {
-                if (tid == 0)
-                    for (int k = 0; k < o; ++k) copy_bin(nb - o + k, 1 + k);
-                __syncthreads();
-            }
-
-            // prefix scan.  Lane `lane` of warp `warp` owns K consecutive bins from
-            // (warp * 32 + lane) * K, K odd so that the lanes' 12-byte records sit
-            // in distinct banks.  Pass 1: each lane sums its bins, the warp scans
-            // the 32 lane totals once and publishes its own total.
-            const int K = ((L + kThreads - 1) / kThreads) | 1;
-            const int lo_i = warp * 32 * K;
-            const int hi_i = min(L, lo_i + 32 * K);
-            const int l0 = min(L, lo_i + lane * K), l1 = min(L, l0 + K);
-            if (tid == 0) s.thr_bits = 0u;      // every warp left the last sweep
-            if (!overlap) {
-                for (int k = lane; k < o; k += 32) {
-                    const int dst = nb - o + k;
-                    if (dst >= lo_i && dst < hi_i) copy_bin(dst, 1 + k);
-                }
-                __syncwarp();
-            }
-            uint32_t ex[kNW];                   // this lane's exclusive offsets in the warp
-#pragma unroll
-            for (int w = 0; w < kNW; ++w) ex[w] = 0u;
-            double er = 0.0, ew = 0.0;
-            // GENERAL: the lane's leading empty bins and its last non-empty bin
-            // (the FP64 prefix of a run of empty bins is made exactly constant)
-            int lead = 0, last_ne = -1;
-            {
-                uint32_t u[kNW];
-#pragma unroll
-                for (int w = 0; w < kNW; ++w) u[w] = 0u;
-                double ur = 0.0, uw = 0.0;
-                for (int i = l0; i < l1; ++i) {
-                    const uint32_t rec = hq + (uint32_t)i * kRec;
-                    if (MODE != MODE_GENERAL) {
-#pragma unroll
-                        for (int w = 0; w < kNW; ++w) u[w] += ld_u32(rec + 4 * w);
-                    } else {
-                        const double br = ld_f64(rec), bw = ld_f64(rec + 8);
-                        ur += br;
-                        uw += bw;
-                        const bool empty = (br == 0.0) & (bw == 0.0);
-                        if (!empty) last_ne = i;
-                        else if (last_ne < 0) ++lead;
-                    }
-                }
-                if (MODE != MODE_GENERAL) {
-                    // 32-bit words added modulo 2^32; every prefix fits its word
-                    uint32_t in[kNW];
-#pragma unroll
-                    for (int w = 0; w < kNW; ++w) in[w] = u[w];
-#pragma unroll
-                    for (int k = 1; k < 32; k <<= 1) {
-#pragma unroll
-                        for (int w = 0; w < kNW; ++w) {
-                            const uint32_t x = __shfl_up_sync(kFull, in[w], k);
-                            if (lane >= k) in[w] += x;
-                        }
-                    }
-#pragma unroll
-                    for (int w = 0; w < kNW; ++w) {
-                        ex[w] = in[w] - u[w];
-                        if (lane == 31) s.tot_w[w][warp] = in[w];
-                    }
-                } else {
-                    double ir = ur, iw = uw;
-#pragma unroll
-                    for (int k = 1; k < 32; k <<= 1) {
-                        const double xr = __shfl_up_sync(kFull, ir, k);
-                        const double xw = __shfl_up_sync(kFull, iw, k);
-                        if (lane >= k) { ir += xr; iw += xw; }
-                    }
-                    // the lane's offset as the sum of the lanes before it
-                    er = __shfl_up_sync(kFull, ir, 1);
-                    ew = __shfl_up_sync(kFull, iw, 1);
-                    if (lane == 0) { er = 0.0; ew = 0.0; }
-                    if (lane == 31) { s.tot_rd[warp] = ir; s.tot_wd[warp] = iw; }
-                    // last non-empty bin before this lane: exclusive max-scan
-                    int im = last_ne;
-#pragma unroll
-                    for (int k = 1; k < 32; k <<= 1) {
-                        const int x = __shfl_up_sync(kFull, im, k);
-                        if (lane >= k) im = max(im, x);
-                    }
-                    if (lane == 31) s.red_ne[warp] = im;
-                    last_ne = __shfl_up_sync(kFull, im, 1);
-                    if (lane == 0) last_ne = -1;
-                }
-            }
-            __syncthreads();
-            if (MODE == MODE_GENERAL)
-                for (int w = 0; w < warp; ++w) last_ne = max(last_ne, s.red_ne[w]);
-            // pass 2: the lane walks its bins again from its offset, writes the
-            // prefix in place and the FP32 screen copy {t prefix, weight prefix}
+            const Hist h = hist(q);
+            auto previous = [&] { if (q > 0) submit(q - 1); };
+            if constexpr (MODE == MODE_GENERAL) scan_period_f64(s, h, scr_s, L, o, previous);
+            else scan_period<MODE>(s, h, scr_s, L, o, previous);
             float tmax = 0.0f;
-            {
-                uint32_t run[kNW];
-#pragma unroll
-                for (int w = 0; w < kNW; ++w) run[w] = ex[w];
-                double rr = er, rw = ew;
-                for (int wp = 0; wp < warp; ++wp) {
-                    if (MODE != MODE_GENERAL) {
-#pragma unroll
-                        for (int w = 0; w < kNW; ++w) run[w] += s.tot_w[w][wp];
-                    } else {
-                        rr += s.tot_rd[wp];
-                        rw += s.tot_wd[wp];
-                    }
-                }
-                const float cfrac = (float)cv.center_frac;
-                for (int i = l0; i < l1; ++i) {
-                    const uint32_t rec = hq + (uint32_t)i * kRec;
-                    float tf, wf, tm = 0.0f;
-                    if (MODE != MODE_GENERAL) {
-#pragma unroll
-                        for (int w = 0; w < kNW; ++w) {
-                            run[w] += ld_u32(rec + 4 * w);
-                            st_u32(rec + 4 * w, run[w]);
-                        }
-                        if (MODE == MODE_UNIFORM) {
-                            // the screen's t is centred by ybar itself: the stored
-                            // prefix minus center_frac per point, in FP32.  tf is
-                            // within 2^-23 tm of the exact value (pf and tf round
-                            // once each, cf <= 2^16 twice), so a box's t is within
-                            // 1.5 * 2^-22 of the largest tm, inside Et
-                            const float pf = (float)((long long)(int32_t)run[1] *
-                                                         (1ll << kHalfBits) +
-                                                     (long long)run[0]);
-                            const float cf = cfrac * (float)run[2];
-                            tf = pf - cf;
-                            tm = fmaxf(fabsf(pf), fabsf(tf)) + fabsf(cf);
-                            wf = (float)run[2];
-                        } else {
-                            tf = (float)wide_value(run[0], run[1], run[2]);
-                            wf = (float)ldexp((double)wide_value(run[3], run[4], run[5]),
-                                              -kWideScreenShift);
-                        }
-                    } else {
-                        rr += ld_f64(rec);
-                        rw += ld_f64(rec + 8);
-                        st_f64(rec, rr);
-                        st_f64(rec + 8, rw);
-                        tf = (float)rr;
-                        wf = (float)rw;
-                    }
-                    st_f2(scr_s + (uint32_t)i * 8u, make_float2(tf, wf));
-                    tmax = fmaxf(tmax, MODE == MODE_UNIFORM ? tm : fabsf(tf));
-                }
-                tmax = warp_max(tmax);
-                if (lane == 0) s.red_t[warp] = tmax;
-            }
-            // sentinel records past the last bin: t = NaN fails every screen
-            for (int i = L + tid; i < L + kScreenPad; i += kThreads)
-                st_f2(scr_s + (uint32_t)i * 8u, make_float2(CUDART_NAN_F, 0.0f));
-            __syncthreads();
-            if (MODE == MODE_GENERAL) {
-                // The lanes' partial sums associate differently from one running
-                // sum, so at a lane boundary an empty bin could move the FP64
-                // prefix by a rounding.  The reference's running sum keeps it
-                // exactly constant, which makes boxes that differ only by empty
-                // end bins tie exactly (first wins); copy the prefix of the last
-                // non-empty bin into this lane's leading empty bins.
-                if (lead > 0 && last_ne >= 0) {
-                    const uint32_t rs = hq + (uint32_t)last_ne * kRec;
-                    const double pr = ld_f64(rs), pw = ld_f64(rs + 8);
-                    for (int i = l0; i < l0 + lead; ++i) {
-                        const uint32_t rec = hq + (uint32_t)i * kRec;
-                        st_f64(rec, pr);
-                        st_f64(rec + 8, pw);
-                        st_f2(scr_s + (uint32_t)i * 8u, make_float2((float)pr, (float)pw));
-                    }
-                }
-                __syncthreads();
-            }
-            tmax = 0.0f;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) tmax = fmaxf(tmax, s.red_t[w]);
 
-            auto iv_prefix = [&](int i) -> double {
-                return MODE == MODE_UNIFORM ? (double)prefix_c(hq, i) * cv.w_uniform
-                       : MODE == MODE_WIDE  ? ldexp((double)wide_prefix_i(hq, i), -e_i)
-                                            : ldexp(ld_f64(hq + (uint32_t)i * 16u + 8u), -e_i);
-            };
-            auto exact = [&](int n, int d) -> double {
-                return exact_objective<MODE>(hq, &cv, n, d, obj);
-            };
             if (a.debug_prefix != nullptr && q == 0) {   // test hook: this period's prefixes
                 for (int i = tid; i < L; i += kThreads) {
-                    const double r_i =
-                        MODE == MODE_UNIFORM ? ldexp((double)prefix_r(hq, i), -e_r)
-                        : MODE == MODE_WIDE  ? ldexp((double)wide_prefix_r(hq, i), -e_r)
-                                             : ldexp(ld_f64(hq + (uint32_t)i * 16u), -e_r);
-                    a.debug_prefix[i] =
-                        r_i + (MODE == MODE_UNIFORM ? cv.center * (double)prefix_c(hq, i)
-                                                    : cv.ybar * iv_prefix(i));
-                    a.debug_prefix[hl + i] = iv_prefix(i);
-                }
-            }
-
-            // ---- sweep: durations outer (the reference's order), two starts per lane ----
-            // bound on the FP32 error of a box's t: 2^-21 of the largest prefix
-            // (one rounding per prefix, one per difference: 2^-22, 2x slack; one
-            // weight: 1.5 * 2^-22 of the largest tm, 1.33x slack)
-            const float Et = cv.exact_all ? CUDART_INF_F : tmax * (1.0f / 2097152.0f);
-            const float Wt = MODE == MODE_UNIFORM ? (float)cv.n_points
-                             : MODE == MODE_WIDE  ? (float)ldexp(cv.i_total, -kWideScreenShift)
-                                                  : (float)cv.i_total;
-            const float Ei = MODE == MODE_UNIFORM ? 0.0f : Wt * (1.0f / 2097152.0f);
-            const float floor_q =
-                MODE != MODE_UNIFORM
-                    ? (float)ldexp(cv.ivar_floor,
-                                   MODE == MODE_WIDE ? e_i - kWideScreenShift : e_i) * (1.0f + 1e-3f)
-                    : 0.0f;
-
-            bool has = false, ex_ok = false;
-            int bn = 0, bdi = 0;
-            float lb = -1.0f, hb = -1.0f;
-            double ex_v = -CUDART_INF;
-            float thr = 0.0f;
-            const uint32_t thr_s = smem_addr(&s.thr_bits);
-
-            // one box that passed the screen: keep it if it may be this lane's best
-            auto consider = [&](int n, int di, int d, float t, float den_lo, float den_hi,
-                                bool sure_valid) -> bool {
-                const float th = fabsf(t) + Et;
-                const float tl = fmaxf(fabsf(t) - Et, 0.0f);
-                const float khi =
-                    den_lo > 0.0f ? __fdividef(th * th, den_lo) * (1.0f + kRel) : CUDART_INF_F;
-                const float klo = __fdividef(tl * tl, den_hi) * (1.0f - kRel);
-                const bool sure = (t < -Et) & sure_valid & (klo > 0.0f);
-                if (!has) {
-                    if (sure) {
-                        has = true; ex_ok = false; bn = n; bdi = di; lb = klo; hb = khi;
-                        return true;
-                    }
-                    const double v = exact(n, d);
-                    if (v > -CUDART_INF) {
-                        has = true; ex_ok = true; ex_v = v; bn = n; bdi = di; lb = klo; hb = khi;
-                        return true;
-                    }
-                    return false;
-                }
-                if (sure && klo > hb) {
-                    ex_ok = false; bn = n; bdi = di; lb = klo; hb = khi;
-                    return true;
-                }
-                if (khi >= lb) {
-                    if (!ex_ok) { ex_v = exact(bn, s.dur[bdi]); ex_ok = true; }
-                    const double v = exact(n, d);
-                    if (v > -CUDART_INF && better(v, di, n, ex_v, bdi, bn)) {
-                        ex_v = v; bn = n; bdi = di; lb = fmaxf(klo, lb); hb = khi;
-                        return true;
-                    }
-                }
-                return false;
-            };
-            // the screen of box (n, d) from its two screen records
-            auto screen = [&](float2 av, float2 bv, int n, int d, float& t, float& den_lo,
-                              float& den_hi, bool& sure_valid) -> bool {
-                t = bv.x - av.x;
-                const float iv = bv.y - av.y;              // count, or scaled weight
-                const float ov = Wt - iv;
-                bool ok;
-                if (MODE == MODE_UNIFORM) {
-                    den_lo = obj ? iv * ov * ov : iv * ov;  // exact counts: > 0 iff valid
-                    den_hi = den_lo;
-                    sure_valid = true;
-                    ok = den_lo > 0.0f;
-                } else {
-                    const float il = fmaxf(iv - Ei, 0.0f), ol = fmaxf(ov - Ei, 0.0f);
-                    const float ih = iv + Ei, oh = ov + Ei;
-                    den_lo = obj ? il * ol * ol : il * ol;
-                    den_hi = obj ? ih * oh * oh : ih * oh;
-                    sure_valid = (il >= floor_q) & (ol >= floor_q);
-                    ok = den_lo > 0.0f;
-                    // an empty box is exactly 0 in the FP64 prefix; t <= Et also
-                    // keeps sentinel boxes (t = NaN) away from these loads
-                    if (!ok && t <= Et) {
-                        ok = MODE == MODE_WIDE ? wide_prefix_i(hq, n + d) != wide_prefix_i(hq, n)
-                                               : ld_f64(hq + (uint32_t)(n + d) * 16u + 8u) !=
-                                                     ld_f64(hq + (uint32_t)n * 16u + 8u);
-                    }
-                }
-                const float th = fabsf(t) + Et;
-                return ok & (t <= Et) & !(th * th < thr * den_lo);
-            };
-
-            // Pilot: the lower key bounds of the warp's first chunk of the first
-            // admissible duration set the screen's threshold before any box is
-            // kept.  Each such box passes the screen again in the sweep below
-            // (its upper bound is at least its lower bound), so its lane keeps it
-            // or something better, and every box discarded against this
-            // threshold is worse than a box that is kept.  Without it a warp's
-            // first chunk of every period would pass the screen whole.
-            {
-                int dp = 0;
-                while (dp < n_dur && s.dur[dp] >= nb) ++dp;
-                if (dp < n_dur) {
-                    const int d = s.dur[dp];
-                    const int nmax = nb - d;
-                    float kbest = -1.0f;
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const int n = warp * 32 + lane + c * kThreads;
-                        if (n <= nmax) {
-                            const uint32_t sa = scr_s + (uint32_t)n * 8u;
-                            float t, den_lo, den_hi;
-                            bool sure_valid;
-                            // thr is still -1 here: the screen checks admissibility only
-                            const bool ok = screen(ld_f2(sa), ld_f2(sa + (uint32_t)d * 8u), n, d, t,
-                                                   den_lo, den_hi, sure_valid);
-                            const float tl = fmaxf(fabsf(t) - Et, 0.0f);
-                            const float klo = __fdividef(tl * tl, den_hi) * (1.0f - kRel);
-                            if (ok & (t < -Et) & sure_valid & (den_lo > 0.0f) & (klo > 0.0f) &
-                                (klo < CUDART_INF_F))
-                                kbest = fmaxf(kbest, klo);
-                        }
-                    }
-                    kbest = warp_max(kbest);
-                    if (kbest > 0.0f) {
-                        thr = kbest * (1.0f - 2.0f * kRel);
-                        if (lane == 0) atomicMax(&s.thr_bits, __float_as_uint(thr));
-                    }
-                }
-            }
-
-            // A cheaper screen in front of `screen`: th = Et - t bounds |t_exact|
-            // for every dip (t_exact < 0 and |t - t_exact| <= Et), and den is a
-            // lower bound of the box's exact denominator -- with one weight the
-            // counts are exact in FP32 and den = c (N - c) (times N - c for the
-            // likelihood); with per-point weights each side is lowered by the
-            // weights' FP32 error Ei.  So a box failing th |th| >= thr den cannot
-            // be the best; `screen` repeats its own test on the few that pass
-            // (and decides, exactly, whether a box with den = 0 is empty).  The
-            // threshold is shared by the CTA's warps through s.thr_bits
-            // (non-negative floats order as their bits), each value a lower bound
-            // of a box some lane keeps.
-            {
-                auto quick = [&](float2 av, float2 bv) -> bool {
-                    const float t = bv.x - av.x;
-                    const float th = Et - t;
-                    const float c = bv.y - av.y;
-                    if (MODE == MODE_UNIFORM) {
-                        const float oc = Wt - c;
-                        const float den = OBJ ? c * oc * oc : c * oc;
-                        return (den > 0.0f) & (th * fabsf(th) >= thr * den);
+                    double r_i, w_i;
+                    if constexpr (one_weight<MODE>()) {
+                        const long long v = prefix_r(h, i);
+                        const double cnt = (double)(v & ((1ll << kCountShift) - 1));
+                        r_i = ldexp((double)(v >> kCountShift), -cv.e_r) + cv.center * cnt;
+                        w_i = cnt * cv.w_uniform;
+                    } else if constexpr (MODE == MODE_GENERAL) {
+                        w_i = ldexp(ld_f64(h.base + 16u * (uint32_t)i + 8u), -cv.e_i);
+                        r_i = ldexp(ld_f64(h.base + 16u * (uint32_t)i), -cv.e_r) + cv.ybar * w_i;
                     } else {
-                        const float il = fmaxf(c - Ei, 0.0f), ol = fmaxf(Wt - c - Ei, 0.0f);
-                        const float den = OBJ ? il * ol * ol : il * ol;
-                        return (th >= 0.0f) & ((den <= 0.0f) | (th * fabsf(th) >= thr * den));
+                        w_i = ldexp((double)prefix_w<MODE>(h, i), -cv.e_i);
+                        r_i = ldexp((double)prefix_r(h, i), -cv.e_r) + cv.ybar * w_i;
                     }
-                };
-                // Starts outer: each lane's two start records (n, n + kThreads) load
-                // once per chunk; widths inner in groups of four (one broadcast
-                // load), so a lane screens eight independent boxes per step and
-                // the warp votes once.  A width with no admissible start in the
-                // chunk (too wide, past the chunk, or a kNoBox slot) reads the
-                // sentinel record instead and fails.  Ties are ordered explicitly
-                // by (duration index, start) in `consider` and the reductions.
+                    a.debug_prefix[i] = r_i;
+                    a.debug_prefix[hl + i] = w_i;
+                }
+            }
+
+            // Bound on the FP32 error of a box's t: 2^-21 of the largest prefix
+            // (one rounding per prefix, one per difference: 2^-22, 2x slack; one
+            // weight: 1.5 * 2^-22 of the largest tm, 1.33x slack), and never 0, so
+            // that a box of exactly the mean counts as the dip it is.  Ei: the same of
+            // the weight (half an ulp per prefix, 2^-24 of the total; 2x slack).
+            const float Et =
+                cv.exact_all ? CUDART_INF_F : tmax * (1.0f / 2097152.0f) + 0.0625f;
+            constexpr int kShift = screen_shift<MODE>();
+            const float Wt = one_weight<MODE>() ? (float)cv.n_points
+                                                : (float)ldexp(cv.i_total, -kShift);
+            const float Ei = one_weight<MODE>() ? 0.0f : Wt * (1.0f / 8388608.0f);
+
+            // Sweep: starts outer, 32 per warp and step; widths inner in groups of four
+            // (one broadcast load).  Maximising snr (likelihood) is maximising the key
+            // t^2 / (iv_in iv_out) (t^2 / (iv_in iv_out^2)) over dips, t = y_in - ybar
+            // iv_in.  th = Et - t bounds |t_exact| for every dip and den is at most the
+            // box's exact denominator, so th |th| / den bounds its key from above: a
+            // lane keeps the largest per group, and its place.  One weight: counts are
+            // exact in FP32, and th = c Et - t is 0 for an empty box (key NaN, which
+            // the maximum drops).  Per-point weights: each side is lowered by the
+            // weights' FP32 error; a box that this leaves without a bound, and that is
+            // not certainly empty, is evaluated in FP64 at once.  A width with no
+            // admissible start in the step (too wide, or a kNoBox slot) reads the
+            // sentinel record and its key is NaN.
+            // Screened in order with a shared threshold instead (what passes bounded and
+            // listed), the passing boxes alone took as long as the sweep itself.
+            double ex_v = -CUDART_INF;
+            int ex_box = -1;
+            {
                 int dmin = nb;
                 for (int k = 0; k < n_dur; ++k) dmin = min(dmin, s.dur[k]);
                 const int nmax_all = nb - dmin;
-                const int n_groups = (n_dur + 3) >> 2;
-                const uint32_t sent = scr_s + (uint32_t)L * 8u;    // first sentinel record
-                constexpr int kHalf = kThreads * 8;                 // bytes to the second start
-                uint32_t sa = scr_s + (uint32_t)(warp * 32 + lane) * 8u;
-                for (int n0 = warp * 32; n0 <= nmax_all; n0 += 2 * kThreads, sa += 2u * kHalf) {
-                    thr = fmaxf(thr, __uint_as_float(ld_u32(thr_s)));
-                    const float2 a1 = ld_f2(sa), a2 = ld_f2_off<kHalf>(sa);
-                    for (int g = 0; g < n_groups; ++g) {
-                        const int4 dg = *reinterpret_cast<const int4*>(&s.dur[4 * g]);
+                const uint32_t sent = scr_s + 8u * (uint32_t)L;    // first sentinel record
+                for (int n0 = warp * 32; n0 <= nmax_all; n0 += kThreads) {
+                    const uint32_t sa = scr_s + 8u * (uint32_t)(n0 + lane);
+                    const float2 x = ld_f2(sa);
+                    const float2 na = make_float2(-x.x, -x.y);
+                    for (int g = 0; g < n_dur; g += 4) {
+                        const int4 dg = *reinterpret_cast<const int4*>(&s.dur[g]);
                         const int dk[4] = {dg.x, dg.y, dg.z, dg.w};
-                        uint32_t m = 0u;
+                        float m = -1.0f, den_min = 1.0f;
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
-                            const int d = dk[k];
-                            const bool fits = (d < nb) & (n0 <= nb - d);
-                            const uint32_t sb = fits ? sa + (uint32_t)d * 8u : sent;
-                            const float2 b1 = ld_f2(sb), b2 = ld_f2_off<kHalf>(sb);
-                            m |= (quick(a1, b1) ? 1u : 0u) << (2 * k);
-                            m |= (quick(a2, b2) ? 2u : 0u) << (2 * k);
-                        }
-                        if (__any_sync(kFull, m != 0u)) {
-                            const int n1 = n0 + lane, n2 = n1 + kThreads;
-                            bool upd = false;
-#pragma unroll 1
-                            for (int k = 0; k < 4; ++k) {
-                                if ((m >> (2 * k) & 3u) == 0u) continue;
-                                const int di = 4 * g + k;
-                                const int d = s.dur[di];
-                                const int nmax = nb - d;
-                                float t, l, h;
-                                bool v;
-                                if ((m >> (2 * k) & 1u) && n1 <= nmax &&
-                                    screen(a1, ld_f2(sa + (uint32_t)d * 8u), n1, d, t, l, h, v))
-                                    upd |= consider(n1, di, d, t, l, h, v);
-                                if ((m >> (2 * k) & 2u) && n2 <= nmax &&
-                                    screen(a2, ld_f2_off<kHalf>(sa + (uint32_t)d * 8u), n2, d, t,
-                                           l, h, v))
-                                    upd |= consider(n2, di, d, t, l, h, v);
+                            const bool fits = (dk[k] < nb) & (n0 <= nb - dk[k]);
+                            const uint32_t sb = fits ? sa + 8u * (uint32_t)dk[k] : sent;
+                            const float2 diff = add_f2(ld_f2(sb), na);
+                            const float t = diff.x, c = diff.y;
+                            float th, den;
+                            if constexpr (one_weight<MODE>()) {
+                                th = fmaf(c, Et, -t);
+                                const float oc = Wt - c;
+                                den = OBJ ? c * oc * oc : c * oc;
+                            } else {
+                                th = Et - t;
+                                const float il = c - Ei, ol = fmaxf(Wt - c - Ei, 0.0f);
+                                den = OBJ ? il * ol * ol : il * ol;
+                                if (c > cv.w_small) den_min = fminf(den_min, den);
                             }
-                            if (__any_sync(kFull, upd)) {
-                                thr = fmaxf(thr,
-                                            warp_max(has ? lb * (1.0f - 2.0f * kRel) : -1.0f));
-                                if (lane == 0) atomicMax(&s.thr_bits, __float_as_uint(thr));
+                            m = fmaxf(m, th * fabsf(th) * rcp_approx(den));
+                        }
+                        second = fmaxf(second, fminf(m, best));
+                        if (m > best) {
+                            best = m;
+                            place = (g << kBoxBits) | (n0 + lane);
+                        }
+                        if constexpr (!one_weight<MODE>()) {
+                            if (!(den_min > 0.0f)) {
+                                const int n = n0 + lane;
+#pragma unroll 1
+                                for (int k = 0; k < 4; ++k) {
+                                    const int d = s.dur[g + k];
+                                    if (d >= nb || n > nb - d) continue;
+                                    const float2 diff = add_f2(ld_f2(sa + 8u * (uint32_t)d), na);
+                                    const float il = diff.y - Ei;
+                                    if (il * (Wt - diff.y - Ei) > 0.0f && il > 0.0f) continue;
+                                    // an empty box is exactly 0 in the prefix
+                                    bool holds;
+                                    if constexpr (MODE == MODE_GENERAL)
+                                        holds = ld_f64(h.base + 16u * (uint32_t)(n + d) + 8u) !=
+                                                ld_f64(h.base + 16u * (uint32_t)n + 8u);
+                                    else holds = prefix_w<MODE>(h, n + d) != prefix_w<MODE>(h, n);
+                                    if (holds)
+                                        keep_better(ex_v, ex_box,
+                                                    exact_objective<MODE, OBJ>(h.base, h.plane, &cv,
+                                                                               n, d),
+                                                    ((g + k) << kBoxBits) | n);
+                                }
                             }
                         }
                     }
                 }
             }
 
-            // ---- reduce: lanes whose best may be the CTA's maximum --------------
-            // After the barrier s.thr_bits is final: the largest published lower
-            // bound (times 1 - 2 kRel), at most the CTA's best lower bound, so a
-            // lane whose upper bound is below it cannot hold the best box.  The
-            // lane holding that largest lower bound is always a candidate; when
-            // it is the only one its box is the period's best and needs no FP64
-            // comparison (the epilogue evaluates it).  Several candidates (near
-            // ties, or every box in exact mode) are compared in FP64 with the
-            // reference's first-wins order.
-            __syncthreads();
-            const float Lc = __uint_as_float(ld_u32(thr_s));
-            const bool cand = has && hb >= Lc;
-            const int n_cand = __syncthreads_count(cand);
-            if (n_cand == 1) {
-                if (cand) { s.win_v[q] = 0.0; s.win_di[q] = bdi; s.win_n[q] = bn; }
-            } else {
-                double v = -CUDART_INF;
-                int vdi = 1 << 30, vn = 1 << 30;
-                if (cand) {
-                    if (!ex_ok) { ex_v = exact(bn, s.dur[bdi]); ex_ok = true; }
-                    v = ex_v; vdi = bdi; vn = bn;
+            // The warp's best group publishes the largest key lower bound of its boxes
+            // that are certainly admissible dips.
+            {
+                const float top = warp_max(best);
+                if (best == top && top > 0.0f) {
+                    const int g = place >> kBoxBits, n = place & ((1 << kBoxBits) - 1);
+                    const uint32_t sa = scr_s + 8u * (uint32_t)n;
+                    const float2 x = ld_f2(sa);
+                    float lo = 0.0f;
+#pragma unroll 1
+                    for (int k = 0; k < 4; ++k) {
+                        const int d = s.dur[g + k];
+                        if (d >= nb || n > nb - d) continue;
+                        const float2 diff = add_f2(ld_f2(sa + 8u * (uint32_t)d),
+                                                   make_float2(-x.x, -x.y));
+                        const float t = diff.x, c = diff.y, ov = Wt - c;
+                        const float ih = c + Ei, oh = ov + Ei;
+                        const float den = OBJ ? ih * oh * oh : ih * oh;
+                        bool valid = (c > 0.0f) & (ov > 0.0f);
+                        if constexpr (!one_weight<MODE>()) {
+                            const float floor_q =
+                                (float)ldexp(cv.ivar_floor, cv.e_i - kShift) * (1.0f + 1e-3f);
+                            valid = (c - Ei >= floor_q) & (ov - Ei >= floor_q) & (c > Ei) & (ov > Ei);
+                        }
+                        const float tl = fmaxf(-t - Et, 0.0f);
+                        const float key = tl * tl * rcp_approx(den) * (1.0f - 2.0f * kRel);
+                        if (valid & (key < CUDART_INF_F)) lo = fmaxf(lo, key);
+                    }
+                    if (lo > 0.0f) atomicMax(&s.thr_bits[q], __float_as_uint(lo));
                 }
-                if (__any_sync(kFull, cand)) {
+            }
+            if constexpr (!one_weight<MODE>()) {
+                // the warp's best box without a bound is a candidate as it stands
+                if (__any_sync(kFull, ex_box >= 0)) {
 #pragma unroll
                     for (int k = 16; k > 0; k >>= 1) {
-                        const double ov = __shfl_xor_sync(kFull, v, k);
-                        const int odi = __shfl_xor_sync(kFull, vdi, k);
-                        const int on = __shfl_xor_sync(kFull, vn, k);
-                        if (better(ov, odi, on, v, vdi, vn)) { v = ov; vdi = odi; vn = on; }
+                        const double ov = __shfl_xor_sync(kFull, ex_v, k);
+                        const int ob = __shfl_xor_sync(kFull, ex_box, k);
+                        keep_better(ex_v, ex_box, ov, ob);
+                    }
+                    if (lane == 0 && ex_box >= 0) {
+                        const int pos = atomicAdd(&s.list_n, 1);
+                        if (pos < kList)
+                            s.list[pos] = ((uint32_t)q << 25) | (uint32_t)(ex_box & ~(3 << kBoxBits));
+                        else atomicOr(&s.rescan, 1u << q);
                     }
                 }
-                if (lane == 0) { s.red_v[warp] = v; s.red_di[warp] = vdi; s.red_n[warp] = vn; }
+            }
+        }
+        __syncthreads();
+        submit(pt - 1);
+        __syncthreads();
+
+        // Each period's winner: the boxes of its candidate groups (one or two, more in
+        // near ties) with the reference's formulas on the exact sums, a box a lane, in
+        // its first-wins order.
+        const int n_list = min(s.list_n, kList);
+        for (int q = warp; q < pt; q += kWarps) {
+            double v = -CUDART_INF;
+            int key = -1;
+            const Hist h = hist(q);
+            const int nb = s.nb[q];
+            for (int e = lane >> 2; e < n_list; e += 8) {
+                const uint32_t c = s.list[e];
+                if ((int)(c >> 25) != q) continue;
+                const int box = (int)(c & ((1u << 25) - 1u)) + ((lane & 3) << kBoxBits);
+                const int d = s.dur[box >> kBoxBits], n = box & ((1 << kBoxBits) - 1);
+                if (d < nb && n <= nb - d)
+                    keep_better(v, key, exact_objective<MODE, OBJ>(h.base, h.plane, &cv, n, d), box);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 16; k > 0; k >>= 1) {
+                const double ov = __shfl_xor_sync(kFull, v, k);
+                const int ok = __shfl_xor_sync(kFull, key, k);
+                keep_better(v, key, ov, ok);
+            }
+            if (lane == 0) s.win[q] = key;
+        }
+        __syncthreads();
+
+        // periods of more candidates than that (a constant flux, sums outside FP32's
+        // range): every box in FP64, by the whole CTA
+        if (s.rescan != 0u) {
+            for (int q = 0; q < pt; ++q) {
+                if (!(s.rescan >> q & 1u)) continue;
+                const Hist h = hist(q);
+                const int nb = s.nb[q];
+                double v = -CUDART_INF;
+                int key = -1;
+                for (int k = 0; k < n_dur; ++k) {
+                    const int d = s.dur[k];
+                    for (int n = tid; d < nb && n <= nb - d; n += kThreads)
+                        keep_better(v, key, exact_objective<MODE, OBJ>(h.base, h.plane, &cv, n, d),
+                                    (k << kBoxBits) | n);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 16; k > 0; k >>= 1) {
+                    const double ov = __shfl_xor_sync(kFull, v, k);
+                    const int ok = __shfl_xor_sync(kFull, key, k);
+                    keep_better(v, key, ov, ok);
+                }
+                if (lane == 0) {
+                    s.red_v[warp] = v;
+                    s.red_box[warp] = key;
+                }
                 __syncthreads();
                 if (tid == 0) {
-                    for (int w = 1; w < kWarps; ++w)
-                        if (better(s.red_v[w], s.red_di[w], s.red_n[w], v, vdi, vn)) {
-                            v = s.red_v[w]; vdi = s.red_di[w]; vn = s.red_n[w];
-                        }
-                    s.win_v[q] = v;
-                    s.win_di[q] = vdi;
-                    s.win_n[q] = vn;
+                    for (int w = 1; w < kWarps; ++w) keep_better(v, key, s.red_v[w], s.red_box[w]);
+                    s.win[q] = key;
                 }
+                __syncthreads();
             }
         }
 
         // ---- 4. the tile's seven output fields, one thread per period ----------
-        __syncthreads();
         if (tid < pt) {
             const int q = tid;
-            const uint32_t hq = smem_s + (uint32_t)(q * pbytes);
             double* op = out + q;
-            if (!(s.win_v[q] > -CUDART_INF)) {
+            const int box = s.win[q];
+            if (box < 0) {
                 op[0] = -CUDART_INF;
                 for (int f = 1; f < kFields; ++f) op[f * ostride] = 0.0;
             } else {
-                const int vn = s.win_n[q];
-                const int d = s.dur[s.win_di[q]];
-                const BoxSums b = box_sums<MODE>(hq, cv, vn, d);
+                const int vn = box & ((1 << kBoxBits) - 1);
+                const int d = s.dur[box >> kBoxBits];
+                const BoxSums b = box_sums<MODE>(hist(q), cv, vn, d);
                 const double iv_out = b.iv_out;
                 const double yin = b.y_in / b.iv_in;
                 const double yout = b.y_out / iv_out;
@@ -1036,7 +1097,7 @@ __global__ void __launch_bounds__(kThreads, MODE == MODE_UNIFORM ? 3 : 2)
                 const double ll = 0.5 * b.iv_in * depth * depth;
                 const double bin = s.seg.bin_duration;
                 const double dur = (double)d * bin;
-                op[0] = obj == 0 ? dsnr : ll;
+                op[0] = OBJ == 0 ? dsnr : ll;
                 op[1 * ostride] = depth;
                 op[2 * ostride] = derr;
                 op[3 * ostride] = dsnr;
@@ -1305,10 +1366,7 @@ __global__ void fold_bins_kernel(const double* tau, int n, double P, double f, u
                                  int fast, int32_t* out, int32_t* used_fast) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const uint32_t fmask = (1u << fb) - 1u;
-    int ind = fast ? fold_fast(tau[j], f, S, fb, fmask, mu, (1u << fb) - 2u * mu, mphi,
-                               0u - 2u * mphi)
-                   : -1;
+    int ind = fold_fast(tau[j], f, S, FoldConst(fb, mu, mphi, fast != 0));
     used_fast[j] = ind >= 0;
     if (ind < 0) ind = fold_exact(tau[j], P, bin, width);
     out[j] = ind;
@@ -1376,11 +1434,19 @@ __global__ void best_kernel(const double* power, const int64_t* spec_off, int64_
 }  // namespace
 
 namespace {
+using SearchKernel = void (*)(BatchArgs);
 template <int OBJ>
-const void* search_fn(int mode) {
-    return mode == MODE_UNIFORM ? (const void*)bls_search_kernel<MODE_UNIFORM, OBJ>
-           : mode == MODE_WIDE  ? (const void*)bls_search_kernel<MODE_WIDE, OBJ>
-                                : (const void*)bls_search_kernel<MODE_GENERAL, OBJ>;
+SearchKernel search_fn(int mode) {
+    switch (mode) {
+        case MODE_UNIFORM: return bls_search_kernel<MODE_UNIFORM, OBJ>;
+        case MODE_PAIR: return bls_search_kernel<MODE_PAIR, OBJ>;
+        case MODE_WIDE: return bls_search_kernel<MODE_WIDE, OBJ>;
+        case MODE_EXACT: return bls_search_kernel<MODE_EXACT, OBJ>;
+        default: return bls_search_kernel<MODE_GENERAL, OBJ>;
+    }
+}
+const void* search_ptr(int mode, int obj) {
+    return (const void*)(obj ? search_fn<1>(mode) : search_fn<0>(mode));
 }
 }  // namespace
 
@@ -1399,8 +1465,8 @@ cudaError_t raise_smem_limit(const void* fn, size_t smem) {
 }
 
 cudaError_t configure_search(int mode, size_t smem) {
-    for (const void* f : {search_fn<0>(mode), search_fn<1>(mode)}) {
-        const cudaError_t e = raise_smem_limit(f, smem);
+    for (int obj = 0; obj < 2; ++obj) {
+        const cudaError_t e = raise_smem_limit(search_ptr(mode, obj), smem);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1408,17 +1474,8 @@ cudaError_t configure_search(int mode, size_t smem) {
 
 cudaError_t launch_search(const BatchArgs& args, int mode, int n_ctas, size_t smem,
                           cudaStream_t stream) {
-    const bool ll = args.obj_flag != 0;
-    if (mode == MODE_UNIFORM) {
-        if (ll) bls_search_kernel<MODE_UNIFORM, 1><<<n_ctas, kThreads, smem, stream>>>(args);
-        else bls_search_kernel<MODE_UNIFORM, 0><<<n_ctas, kThreads, smem, stream>>>(args);
-    } else if (mode == MODE_WIDE) {
-        if (ll) bls_search_kernel<MODE_WIDE, 1><<<n_ctas, kThreads, smem, stream>>>(args);
-        else bls_search_kernel<MODE_WIDE, 0><<<n_ctas, kThreads, smem, stream>>>(args);
-    } else {
-        if (ll) bls_search_kernel<MODE_GENERAL, 1><<<n_ctas, kThreads, smem, stream>>>(args);
-        else bls_search_kernel<MODE_GENERAL, 0><<<n_ctas, kThreads, smem, stream>>>(args);
-    }
+    const SearchKernel k = args.obj_flag != 0 ? search_fn<1>(mode) : search_fn<0>(mode);
+    k<<<n_ctas, kThreads, smem, stream>>>(args);
     return cudaGetLastError();
 }
 
@@ -1477,16 +1534,26 @@ cudaError_t static_scratch_address(int device, void** ptr) {
 int search_threads() { return kThreads; }
 
 size_t period_hist_bytes(int mode, int hl) {
-    return mode == MODE_UNIFORM ? hist_period_bytes<MODE_UNIFORM>(hl)
-           : mode == MODE_WIDE  ? hist_period_bytes<MODE_WIDE>(hl)
-                                : hist_period_bytes<MODE_GENERAL>(hl);
+    switch (mode) {
+        case MODE_UNIFORM: return hist_period_bytes<MODE_UNIFORM>(hl);
+        case MODE_PAIR: return hist_period_bytes<MODE_PAIR>(hl);
+        case MODE_WIDE: return hist_period_bytes<MODE_WIDE>(hl);
+        case MODE_EXACT: return hist_period_bytes<MODE_EXACT>(hl);
+        default: return hist_period_bytes<MODE_GENERAL>(hl);
+    }
+}
+
+int screen_shift(int mode) {
+    return mode == MODE_WIDE ? screen_shift<MODE_WIDE>()
+           : mode == MODE_EXACT ? screen_shift<MODE_EXACT>() : 0;
 }
 
 size_t search_static_smem(int mode) {
     size_t most = 0;
-    for (const void* f : {search_fn<0>(mode), search_fn<1>(mode)}) {
+    for (int obj = 0; obj < 2; ++obj) {
         cudaFuncAttributes at{};
-        if (cudaFuncGetAttributes(&at, f) == cudaSuccess) most = std::max(most, at.sharedSizeBytes);
+        if (cudaFuncGetAttributes(&at, search_ptr(mode, obj)) == cudaSuccess)
+            most = std::max(most, at.sharedSizeBytes);
     }
     return most;
 }
@@ -1494,8 +1561,8 @@ size_t search_static_smem(int mode) {
 int max_resident_ctas(int mode, size_t smem) {
     // the smaller of the two objectives' occupancies
     int b0 = 0, b1 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, search_fn<0>(mode), kThreads, smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, search_fn<1>(mode), kThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, search_ptr(mode, 0), kThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, search_ptr(mode, 1), kThreads, smem);
     return b0 < b1 ? b0 : b1;
 }
 

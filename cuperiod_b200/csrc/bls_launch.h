@@ -60,6 +60,8 @@ cudaError_t launch_rows(const double* out, int64_t out_stride, int n_curves,
 
 // Bytes of one period's histogram in the kernel's layout.
 size_t period_hist_bytes(int mode, int hl);
+// WIDE / EXACT: the FP32 screen holds the fixed-point weights times 2^-screen_shift.
+int screen_shift(int mode);
 
 // Joint-ephemeris multi-band search (bls_joint.cu): static shared memory of one
 // CTA, CTAs resident per SM (histograms in `smem` bytes of dynamic shared memory,
