@@ -107,13 +107,6 @@ struct CurveDesc {
     float gap;              // mean time between points
 };
 
-struct WorkItem {
-    int32_t curve;
-    int32_t segment;
-    int32_t p_begin;        // first period of the tile, within the segment
-    int32_t p_count;        // periods in the tile (<= kMaxTile)
-};
-
 // One launch may search several trial grids (each curve has one).  The curves
 // of one accumulation mode and one grid form a group whose work is regular:
 // every curve of the group is cut into the same tiles (segment s of the grid:

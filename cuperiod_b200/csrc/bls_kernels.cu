@@ -32,6 +32,7 @@
 #include <cfloat>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "bls_device.h"
@@ -47,9 +48,10 @@ constexpr int kPts = kChunkPts;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kRel = 1.0f / 262144.0f;    // 2^-18: relative slack of FP32 key bounds
 constexpr int kCasLimit = 1 << 16;          // retries of one FP64 shared add
-constexpr int kNoBox = 1 << 29;             // duration slot past the last real duration
-constexpr int kList = 256;                  // candidates of one tile's periods
+constexpr int kList = 512;                  // open points, then candidates, of one tile
 constexpr int kRegBins = 9;                 // bins a lane holds in registers while scanning
+constexpr int kOpenBits = 28;               // open point: period << kOpenBits | index
+constexpr uint32_t kNoPoint = 0xffffffffu;  // (of a 17th period)
 constexpr int kBoxBits = 20;                // box key: duration index << kBoxBits | start
 // Per-point weights: the FP32 screen holds them scaled by 2^-shift, their sum (below
 // 2^54, 2^60 and 2^54) at most 2^41, so that the likelihood's iv_in * iv_out^2 stays
@@ -59,15 +61,23 @@ __device__ __host__ constexpr int screen_shift() {
     return MODE == MODE_WIDE ? 13 : (MODE == MODE_EXACT || MODE == MODE_GENERAL) ? 20 : 0;
 }
 
-struct TileShared {
-    WorkItem item;
+// One work item's inputs, copied to shared memory while the item before it is searched.
+struct Tile {
     CurveDesc curve;
     SegmentDesc seg;
     double per[kMaxTile];
     double freq[kMaxTile];
     uint32_t scale[kMaxTile];
     int32_t nb[kMaxTile];
-    alignas(16) int32_t dur[kMaxDur + 4];   // padded with kNoBox; read four at a time
+    alignas(16) int32_t dur[kMaxDur + 4];   // box widths, the last one repeated to a multiple
+                                            // of four (a repeated box only ties itself)
+    int32_t p_begin, p_count;
+    int32_t d_min, d_max;                   // smallest and largest width
+    int32_t item;                           // work item, >= n_items: none left
+};
+
+struct TileShared {
+    Tile tile[2];
     uint32_t thr_bits[kMaxTile];    // per period: a lower bound of its best key (bits of a
                                     // float >= 0)
     int32_t win[kMaxTile];          // per period: the best box's key, -1 when there is none
@@ -77,10 +87,13 @@ struct TileShared {
     double red_v[kWarps];
     int red_box[kWarps];
     int red_ne[kWarps];             // GENERAL scan: last non-empty bin per warp
-    uint32_t list[kList];           // candidates: period << 25 | box, standing for the four
-    int list_n;                     // widths of the box's group at its start
+    // after the sweeps, candidates: period << 25 | box, standing for the four widths of
+    // the box's group at its start; before them, while folding, open points: period <<
+    // kOpenBits | point
+    uint32_t list[kList];
+    int list_n;
+    int open_n;
     uint32_t rescan;                // bit q: period q needs every box in FP64
-    int next;
 };
 
 // Shared-memory accesses by 32-bit shared-space address (the hot loops compute
@@ -254,9 +267,13 @@ __device__ __forceinline__ void bin_sums(const Hist& h, int i, long long& r, lon
     const uint32_t a = h.base + 4u * (uint32_t)i;
     w = 0;
     if (MODE == MODE_PAIR) {
+        // 2^20 H as a 64-bit value: the second plane's top 20 bits, 8 up; the first plane
+        // is its low word plus the remainder modulo 2^32, so a low word above it carries
         const uint32_t lo = ld_u32(a), b = ld_u32(a + h.plane);
-        const long long sum = join_sum<32 - kPairBits>((int32_t)b >> kPairBits, lo);
-        r = (sum << kCountShift) + (long long)(b & ((1u << kPairBits) - 1u));
+        const uint32_t base = (b << (32 - 2 * kPairBits)) & ~((1u << (32 - kPairBits)) - 1u);
+        const uint32_t hi = (uint32_t)((int32_t)b >> (2 * kPairBits)) + (lo < base ? 1u : 0u);
+        r = (long long)(((unsigned long long)__funnelshift_l(lo, hi, kCountShift) << 32) |
+                        ((lo << kCountShift) | (b & ((1u << kPairBits) - 1u))));
     } else if (MODE == MODE_UNIFORM) {
         const long long sum = (long long)(int32_t)ld_u32(a + h.plane) * (1ll << kHalfBits) +
                               (long long)ld_u32(a);
@@ -339,46 +356,55 @@ struct PointRegs {
     double rv[kW > 0 ? 1 : NR], iv[kW > 0 ? 1 : NR];
 };
 
-// The points of this lane in the block of kThreads * NR points at `base`: slot
-// base + r * kThreads + tid of a full chunk (stored lane-interleaved), time index
-// base + tid * NR + r of the tail.  A tail slot past the last point repeats that
-// point's time with nothing to add.
+// The words of the point in slot `i`, nothing when !ok.
+template <int MODE, int NR>
+__device__ __forceinline__ void load_words(const BatchArgs& a, int64_t i, bool ok,
+                                           PointRegs<MODE, NR>& p, int r) {
+    if constexpr (one_weight<MODE>()) {
+        const int32_t v = ok ? __ldg(a.pay_r + i) : 0;
+        if constexpr (MODE == MODE_PAIR) {
+            p.w[r][0] = (uint32_t)v;
+            p.w[r][1] = ((uint32_t)(v >> (32 - kPairBits)) << kPairBits) | (ok ? 1u : 0u);
+        } else {
+            p.w[r][0] = (uint32_t)v & ((1u << kHalfBits) - 1u);
+            p.w[r][1] = (uint32_t)(v >> kHalfBits);
+            p.w[r][2] = ok ? 1u : 0u;
+        }
+    } else if constexpr (MODE != MODE_GENERAL) {
+        const long long rq = ok ? __ldg(reinterpret_cast<const long long*>(a.r64) + i) : 0ll;
+        const long long iq = ok ? __ldg(reinterpret_cast<const long long*>(a.iv64) + i) : 0ll;
+        constexpr int kStep = MODE == MODE_WIDE ? kWideBits : kExactBits;
+        constexpr int kHalf = point_words<MODE>() / 2;
+#pragma unroll
+        for (int w = 0; w < kHalf; ++w) {
+            p.w[r][w] = (uint32_t)(rq >> (w * kStep));
+            p.w[r][kHalf + w] = (uint32_t)(iq >> (w * kStep));
+        }
+    } else {
+        p.rv[r] = ok ? __ldg(a.r64 + i) : 0.0;
+        p.iv[r] = ok ? __ldg(a.iv64 + i) : 0.0;
+    }
+}
+
+// This lane's r-th point of the block of kThreads * NR points at `base` (may lie past the
+// last point): slot base + r * kThreads + tid of a full chunk (stored lane-interleaved),
+// time index base + tid * NR + r of the tail.
+template <int NR, bool TAIL>
+__device__ __forceinline__ int point_index(int base, int r) {
+    return TAIL ? base + (int)threadIdx.x * NR + r : base + r * kThreads + (int)threadIdx.x;
+}
+
+// The lane's points; a tail slot past the last point repeats that point's time with
+// nothing to add.
 template <int MODE, int NR, bool TAIL>
 __device__ __forceinline__ void load_points(const BatchArgs& a, const CurveDesc& c, int base,
                                             PointRegs<MODE, NR>& p) {
-    const int tid = threadIdx.x;
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        int j = TAIL ? base + tid * NR + r : base + r * kThreads + tid;
-        const bool ok = !TAIL || j < c.n_points;
-        if (TAIL) j = min(j, c.n_points - 1);
-        const int64_t slot = c.point_off + j;
-        p.x[r] = __ldg(a.tau + slot);
-        if constexpr (one_weight<MODE>()) {
-            const int32_t v = ok ? __ldg(a.pay_r + slot) : 0;
-            if constexpr (MODE == MODE_PAIR) {
-                p.w[r][0] = (uint32_t)v;
-                p.w[r][1] = ((uint32_t)(v >> (32 - kPairBits)) << kPairBits) | (ok ? 1u : 0u);
-            } else {
-                p.w[r][0] = (uint32_t)v & ((1u << kHalfBits) - 1u);
-                p.w[r][1] = (uint32_t)(v >> kHalfBits);
-                p.w[r][2] = ok ? 1u : 0u;
-            }
-        } else if constexpr (MODE != MODE_GENERAL) {
-            const long long rq = ok ? __ldg(reinterpret_cast<const long long*>(a.r64) + slot) : 0ll;
-            const long long iq =
-                ok ? __ldg(reinterpret_cast<const long long*>(a.iv64) + slot) : 0ll;
-            constexpr int kStep = MODE == MODE_WIDE ? kWideBits : kExactBits;
-            constexpr int kHalf = point_words<MODE>() / 2;
-#pragma unroll
-            for (int k = 0; k < kHalf; ++k) {
-                p.w[r][k] = (uint32_t)(rq >> (k * kStep));
-                p.w[r][kHalf + k] = (uint32_t)(iq >> (k * kStep));
-            }
-        } else {
-            p.rv[r] = ok ? __ldg(a.r64 + slot) : 0.0;
-            p.iv[r] = ok ? __ldg(a.iv64 + slot) : 0.0;
-        }
+        const int j = point_index<NR, TAIL>(base, r);
+        const int64_t i = c.point_off + (TAIL ? min(j, c.n_points - 1) : j);
+        p.x[r] = __ldg(a.tau + i);
+        load_words<MODE, NR>(a, i, !TAIL || j < c.n_points, p, r);
     }
 }
 
@@ -388,12 +414,53 @@ __device__ __forceinline__ void add_words(uint32_t rec, uint32_t plane, const ui
     for (int k = 0; k < N; ++k) red_add_u32(rec + k * plane, w[k]);
 }
 
-// The bin of a point whose fast fold is not provably the reference's: the reference's
-// IEEE chain, out of line (2 points in 10^4 of a survey cadence); what the reference
-// never reads (past n_bins) goes to the bin past the last, hl.
-__device__ __noinline__ int exact_bin(double x, double P, double bin, int width, int nb, int hl) {
-    const int e = fold_exact(x, P, bin, width);
-    return e > nb ? hl : e;
+// One point's contribution to the record at shared address `rec`.
+template <int MODE, int NR>
+__device__ __forceinline__ void add_point(uint32_t rec, uint32_t plane,
+                                          const PointRegs<MODE, NR>& p, int r, int32_t* flag) {
+    if constexpr (MODE == MODE_GENERAL) {
+        shared_add_f64(rec, p.rv[r], flag);
+        shared_add_f64(rec + 8, p.iv[r], flag);
+    } else {
+        add_words(rec, plane, p.w[r]);
+    }
+}
+
+template <int MODE>
+__device__ __host__ constexpr uint32_t bin_stride() {
+    return MODE == MODE_GENERAL ? 16u : 4u;
+}
+
+// Point j of the curve at period q, whose fast fold is not provably the reference's bin:
+// by the reference's IEEE chain.  What the reference never reads, bins past n_bins, is
+// dropped.
+template <int MODE>
+__device__ __noinline__ void fold_exactly(const BatchArgs* a, const Tile* tl, int j, int q,
+                                          uint32_t hist_s) {
+    if (j >= tl->curve.n_points) return;
+    const uint32_t hq = hist_s + (uint32_t)q * hist_period_bytes<MODE>(tl->seg.hist_len);
+    const uint32_t plane = plane_bytes<MODE>(tl->seg.hist_len);
+    const int64_t i = tl->curve.point_off + j;
+    const int e = fold_exact(__ldg(a->tau + i), tl->per[q], tl->seg.bin_duration, tl->seg.width);
+    if (e > tl->nb[q]) return;
+    PointRegs<MODE, 1> p;
+    load_words<MODE, 1>(*a, i, true, p, 0);
+    add_point<MODE, 1>(hq + bin_stride<MODE>() * (uint32_t)e, plane, p, 0, a->error_flag);
+}
+
+// The open points of one lane's block at period q, when the list is full.
+template <int MODE, int NR, bool TAIL>
+__device__ __noinline__ void fold_lane_exactly(const BatchArgs* a, const Tile* tl, int base, int q,
+                                               uint32_t hist_s) {
+    const SegmentDesc& g = tl->seg;
+    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, g.fast_fold != 0);
+    for (int r = 0; r < NR; ++r) {
+        const int j = point_index<NR, TAIL>(base, r);
+        if (j >= tl->curve.n_points) return;
+        const double x = __ldg(a->tau + tl->curve.point_off + j);
+        if (fc.edge(fc.position(x, tl->freq[q], tl->scale[q])) >= fc.limit)
+            fold_exactly<MODE>(a, tl, j, q, hist_s);
+    }
 }
 
 // Fold this lane's NR points into the histograms of the tile's pt periods.
@@ -402,16 +469,24 @@ __device__ __noinline__ int exact_bin(double x, double P, double bin, int width,
 // MERGE: a lane's points are consecutive in time, so where a bin is wider than the
 // sampling each run of equal bins adds its sums once; elsewhere the comparisons only
 // cost (one-weight batch of 16 curves, 50,000 periods: 27.7 ms without, 29.8 with).
+//
+// Open points (not decided by the fast fold: 2 in 10^4 of a survey cadence, those on bin
+// edges) go to the bin past the last, which nothing reads, and to a list that the CTA
+// folds exactly at the end.  Folding them here, in whatever form, took a call inside the
+// loop, whose calling convention halves the registers that stay live: words were spilled
+// or formed again at every period (4 four-year curves 53.7 ms so, 48.7 ms with the list;
+// 16 curves of the batched workload 18.3 -> 16.7 ms).
 template <int MODE, int NR, bool TAIL, bool MERGE>
-__device__ __forceinline__ void fold_points(const TileShared& s, uint32_t hist_s,
-                                            const PointRegs<MODE, NR>& p, int pt, int hl,
-                                            int32_t* flag) {
+__device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& sh, const Tile& s,
+                                                uint32_t hist_s, const PointRegs<MODE, NR>& p,
+                                                int base, int pt, int hl) {
     const SegmentDesc& g = s.seg;
     const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, g.fast_fold != 0);
     const uint32_t plane = plane_bytes<MODE>(hl);
     const uint32_t pbytes = hist_period_bytes<MODE>(hl);
-    constexpr uint32_t kB = MODE == MODE_GENERAL ? 16u : 4u;
+    constexpr uint32_t kB = bin_stride<MODE>();
     uint32_t hq = hist_s;
+    uint32_t lost = 0u;             // periods whose open points found the list full
     for (int q = 0; q < pt; ++q, hq += pbytes) {
         const double f = s.freq[q];
         const uint32_t S = s.scale[q];
@@ -423,18 +498,28 @@ __device__ __forceinline__ void fold_points(const TileShared& s, uint32_t hist_s
             rec[r] = hq + kB + (v >> fc.fb) * kB;
         }
         if (worst >= fc.limit) {
+            uint32_t open = 0u;
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-                if (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit)
-                    rec[r] = hq + kB * (uint32_t)exact_bin(p.x[r], s.per[q], g.bin_duration,
-                                                           g.width, s.nb[q], hl);
+                if (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit) {
+                    open |= 1u << r;
+                    rec[r] = hq + kB * (uint32_t)hl;
+                }
+            int pos = atomicAdd(&sh.open_n, __popc(open));
+            const bool fits = pos + __popc(open) <= kList &&
+                              point_index<NR, TAIL>(base, NR) < (1 << kOpenBits);
+            if (!fits) lost |= 1u << q;
+            for (; open != 0u && pos < kList; ++pos) {
+                const int r = __ffs(open) - 1;
+                open &= open - 1u;
+                sh.list[pos] = fits ? ((uint32_t)q << kOpenBits) |
+                                          (uint32_t)point_index<NR, TAIL>(base, r)
+                                    : kNoPoint;
+            }
         }
         if constexpr (MODE == MODE_GENERAL) {
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                shared_add_f64(rec[r], p.rv[r], flag);
-                shared_add_f64(rec[r] + 8, p.iv[r], flag);
-            }
+            for (int r = 0; r < NR; ++r) add_point<MODE, NR>(rec[r], plane, p, r, a.error_flag);
         } else if constexpr (!MERGE) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) add_words(rec[r], plane, p.w[r]);
@@ -456,35 +541,69 @@ __device__ __forceinline__ void fold_points(const TileShared& s, uint32_t hist_s
             add_words<kW>(rec[NR - 1], plane, run);
         }
     }
+    return lost;
 }
 
 // Fold the block of kThreads * NR points at `base`; lanes past the tail's last
 // point sit it out.
 template <int MODE, int NR, bool TAIL, bool MERGE>
-__device__ __forceinline__ void fold_block(const BatchArgs& a, const TileShared& s,
+__device__ __forceinline__ void fold_block(const BatchArgs& a, TileShared& sh, const Tile& s,
                                            uint32_t hist_s, int base, int pt, int hl) {
     if (TAIL && base + (int)threadIdx.x * NR >= s.curve.n_points) return;
-    PointRegs<MODE, NR> p;
-    load_points<MODE, NR, TAIL>(a, s.curve, base, p);
-    fold_points<MODE, NR, TAIL, MERGE>(s, hist_s, p, pt, hl, a.error_flag);
+    uint32_t lost;
+    {
+        PointRegs<MODE, NR> p;
+        load_points<MODE, NR, TAIL>(a, s.curve, base, p);
+        lost = fold_points<MODE, NR, TAIL, MERGE>(a, sh, s, hist_s, p, base, pt, hl);
+    }
+    for (; lost != 0u; lost &= lost - 1u)
+        fold_lane_exactly<MODE, NR, TAIL>(&a, &s, base, __ffs(lost) - 1, hist_s);
+}
+
+// Fold the curve into the histograms of the tile.
+template <int MODE>
+__device__ __forceinline__ void fold_curve(const BatchArgs& a, TileShared& s, const Tile& tl,
+                                           uint32_t smem_s) {
+    const int pt = tl.p_count, hl = tl.seg.hist_len, n = tl.curve.n_points;
+    int base = 0;
+    if (MODE != MODE_GENERAL && tl.seg.bin_duration > 1.5f * tl.curve.gap)
+        for (; base + kChunk <= n; base += kChunk)
+            fold_block<MODE, kPts, false, true>(a, s, tl, smem_s, base, pt, hl);
+    else
+        for (; base + kChunk <= n; base += kChunk)
+            fold_block<MODE, kPts, false, false>(a, s, tl, smem_s, base, pt, hl);
+    // the tail: fewer points a lane when few are left, so that more warps share them
+    const int left = n - base;
+    if (left > 4 * kThreads)
+        fold_block<MODE, kPts, true, false>(a, s, tl, smem_s, base, pt, hl);
+    else if (left > 2 * kThreads)
+        fold_block<MODE, 4, true, false>(a, s, tl, smem_s, base, pt, hl);
+    else if (left > 0)
+        fold_block<MODE, 2, true, false>(a, s, tl, smem_s, base, pt, hl);
+    __syncthreads();
+    const int open = min(s.open_n, kList);
+    for (int e = threadIdx.x; e < open; e += kThreads) {
+        const uint32_t p = s.list[e];
+        if (p != kNoPoint)
+            fold_exactly<MODE>(&a, &tl, (int)(p & ((1u << kOpenBits) - 1u)), (int)(p >> kOpenBits),
+                               smem_s);
+    }
 }
 
 // ---- prefix sums -----------------------------------------------------------------
 
-// The FP32 screen copy of one prefix: {t, weight} and, one weight, the magnitude that
-// bounds t's rounding error.
+// The FP32 screen copy of one prefix: {t, weight}, and the magnitude that bounds t's
+// rounding error.
 template <int MODE>
 __device__ __forceinline__ float2 screen_record(long long r, long long w, float cfrac, float& tm) {
     if (one_weight<MODE>()) {
         // the screen's t is centred by ybar itself: the stored prefix minus
-        // center_frac per point, in FP32.  It is within 2^-23 tm of the exact value
-        // (pf and t round once each, cf <= 2^16 twice), so a box's t is within
-        // 1.5 * 2^-22 of the largest tm, inside Et
+        // center_frac per point, in FP32.  It is within 2^-23 (|pf| + 2 |cf|) of the
+        // exact value (pf and t round once each, cf twice), |pf| <= |t| + |cf|, and
+        // |cf| <= |cfrac| n over a whole scan (2 n with the pad): the caller adds that
         const float cnt = (float)(uint32_t)(r & ((1ll << kCountShift) - 1));
-        const float pf = (float)(r >> kCountShift);
-        const float cf = cfrac * cnt;
-        const float t = pf - cf;
-        tm = fmaxf(fabsf(pf), fabsf(t)) + fabsf(cf);
+        const float t = fmaf(-cfrac, cnt, (float)(r >> kCountShift));
+        tm = fabsf(t);
         return make_float2(t, cnt);
     }
     const float t = (float)r;
@@ -501,7 +620,7 @@ __device__ __forceinline__ float2 screen_record(long long r, long long w, float 
 // their running sums in registers between the two barriers, so each bin is read once
 // and written once; more than kThreads * kRegBins bins go in several such blocks.
 template <int MODE, typename F>
-__device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32_t scr_s, int L,
+__device__ __forceinline__ void scan_period(TileShared& s, const Tile& tl, const Hist& h, uint32_t scr_s, int L,
                                             int o, F&& first) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = L - 1;
@@ -515,7 +634,7 @@ __device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32
     const bool copied = overlap || !single;
     if (copied) {
         auto copy_bin = [&](int dst, int src) {
-            if (dst < 0 || dst >= s.seg.width || dst > s.seg.hist_len || src > s.seg.hist_len) return;
+            if (dst < 0 || dst >= tl.seg.width || dst > tl.seg.hist_len || src > tl.seg.hist_len) return;
             const uint32_t rd = h.base + 4u * (uint32_t)dst, rs = h.base + 4u * (uint32_t)src;
 #pragma unroll
             for (int k = 0; k < kW; ++k) st_u32(rd + k * h.plane, ld_u32(rs + k * h.plane));
@@ -529,7 +648,7 @@ __device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32
         __syncthreads();
     }
     const int K = single ? (((L + kThreads - 1) / kThreads) | 1) : kRegBins;
-    const float cfrac = (float)s.curve.center_frac;
+    const float cfrac = (float)tl.curve.center_frac;
     long long carry_r = 0, carry_w = 0;
     float tmax = 0.0f;
     int par = 0;
@@ -568,18 +687,30 @@ __device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32
         }
         __syncthreads();
         if (b0 == 0) first();
-        long long off_r = carry_r + in_r - run_r, off_w = carry_w + in_w - run_w;
+        // the warps before this one: lane w takes warp w's total
+        long long off_r = lane < kWarps ? s.tot[par][0][lane] : 0ll, off_w = 0ll;
+        if (kTwo) off_w = lane < kWarps ? s.tot[par][1][lane] : 0ll;
+        if (!single) {          // the block's total, for the next one
+            long long all_r = off_r, all_w = off_w;
+            all_r = warp_sum(all_r);
+            if (kTwo) all_w = warp_sum(all_w);
+            if (lane >= warp) off_r = off_w = 0ll;
+            off_r = warp_sum(off_r) + carry_r;
+            if (kTwo) off_w = warp_sum(off_w) + carry_w;
+            carry_r += all_r;
+            carry_w += all_w;
+        } else {
+            if (lane >= warp) off_r = off_w = 0ll;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const long long t = s.tot[par][0][w];
-            carry_r += t;
-            if (w < warp) off_r += t;
-            if (kTwo) {
-                const long long u = s.tot[par][1][w];
-                carry_w += u;
-                if (w < warp) off_w += u;
+            for (int k = kWarps / 2; k > 0; k >>= 1) {
+                off_r += __shfl_xor_sync(kFull, off_r, k);
+                if (kTwo) off_w += __shfl_xor_sync(kFull, off_w, k);
             }
+            off_r = __shfl_sync(kFull, off_r, 0);
+            if (kTwo) off_w = __shfl_sync(kFull, off_w, 0);
         }
+        off_r += in_r - run_r;
+        off_w += in_w - run_w;
 #pragma unroll
         for (int r = 0; r < kRegBins; ++r) {
             const int i = l0 + r;
@@ -607,12 +738,12 @@ __device__ __forceinline__ void scan_period(TileShared& s, const Hist& h, uint32
 // that differ only by empty end bins tie exactly (first wins), so the lanes copy the
 // prefix of the last non-empty bin into their leading empty bins (a third barrier).
 template <typename F>
-__device__ __forceinline__ void scan_period_f64(TileShared& s, const Hist& h, uint32_t scr_s, int L,
+__device__ __forceinline__ void scan_period_f64(TileShared& s, const Tile& tl, const Hist& h, uint32_t scr_s, int L,
                                                 int o, F&& first) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = L - 1;
     auto copy_bin = [&](int dst, int src) {
-        if (dst < 0 || dst >= s.seg.width || dst > s.seg.hist_len || src > s.seg.hist_len) return;
+        if (dst < 0 || dst >= tl.seg.width || dst > tl.seg.hist_len || src > tl.seg.hist_len) return;
         const uint32_t rd = h.base + 16u * (uint32_t)dst, rs = h.base + 16u * (uint32_t)src;
         st_f64(rd, ld_f64(rs));
         st_f64(rd + 8, ld_f64(rs + 8));
@@ -696,127 +827,143 @@ __device__ __forceinline__ void scan_period_f64(TileShared& s, const Hist& h, ui
 
 // ---- the search --------------------------------------------------------------------
 
+// The last i in [0, n) with a[i * stride] <= v (a[0] <= v), by one warp, 32 at a time.
+__device__ __forceinline__ int last_at_most(const int32_t* a, int stride, int n, int v) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    while (n > 1) {
+        const int step = (n + 31) / 32;
+        const int i = lane * step;
+        const bool le = i < n && __ldg(a + (int64_t)(lo + i) * stride) <= v;
+        const int k = __popc(__ballot_sync(kFull, le)) - 1;
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
+}
+
+template <typename T>
+__device__ __forceinline__ void copy_words(T* to, const T* from, int lane) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
+    for (int i = lane; i < (int)(sizeof(T) / 4); i += 32)
+        reinterpret_cast<uint32_t*>(to)[i] = __ldg(reinterpret_cast<const uint32_t*>(from) + i);
+}
+
 // Persistent search; see the head of this file.  One weight runs three CTAs an SM (80
 // registers), per-point weights two.  Bound by latency between its barriers with 24 (16)
 // resident warps: neither issue nor the shared-memory pipe is above two thirds busy.
 // 96 curves of the batched workload (mean 9,900 points, 50,000 periods): 152.8 ms with
-// three words a point, five barriers a period and a screened sweep, 128.3 ms as built;
-// 16 curves with per-point errors 52.7 -> 40.7 ms (38-bit weights), 8 with outlying
-// errors 56.2 -> 29.3 ms (FP64 sums by compare-and-swap before).
+// three words a point, five barriers a period and a screened sweep; 104.3 ms as built.
+// 16 curves with per-point errors 52.7 -> 33.7 ms (38-bit weights), 8 with outlying
+// errors 56.2 -> 24.8 ms (FP64 sums by compare-and-swap before).
 template <int MODE, int OBJ>
 __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
-    bls_search_kernel(BatchArgs a) {
+    bls_search_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileShared s;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
 
-    for (;;) {
+    // Claims the next work item and copies its inputs to tile slot `to`: one warp, while
+    // the others search (the chain of dependent loads takes a few microseconds).
+    auto fetch = [&](int to) {
+        Tile& t = s.tile[to];
+        const int it = __shfl_sync(kFull, lane == 0 ? atomicAdd(a.work_counter, 1) : 0, 0);
+        if (it >= a.n_items) {
+            if (lane == 0) t.item = it;
+            return;
+        }
+        // one grid: the group is a launch parameter; several: a search
+        WorkGroup gr = a.group0;
+        if (a.n_groups > 1)
+            gr = a.groups[last_at_most(&a.groups[0].item_begin, sizeof(WorkGroup) / 4, a.n_groups,
+                                       it)];
+        const int local = it - gr.item_begin;
+        const int r = local / gr.tiles_per_curve;
+        const int j = local - r * gr.tiles_per_curve;
+        const int32_t* tiles = a.seg_tiles + gr.tiles_begin;
+        const int lo = last_at_most(tiles, 1, gr.n_segments, j);
+        const int sg = gr.seg_begin + lo;
+        const int cap = __ldg(a.seg_cap + sg);
+        const int curve = __ldg(a.order + gr.order_begin + r);
+        const int p_begin = (j - __ldg(tiles + lo)) * cap;
+        copy_words(&t.seg, a.segments + sg, lane);
+        copy_words(&t.curve, a.curves + curve, lane);
+        __syncwarp();
+        const int p_count = min(cap, t.seg.n_periods - p_begin);
+        const int64_t g0 = t.seg.period_off + p_begin;
+        if (lane < p_count && lane < kMaxTile) {
+            t.per[lane] = __ldg(a.period + g0 + lane);
+            t.freq[lane] = __ldg(a.freq + g0 + lane);
+            t.scale[lane] = __ldg(a.scale + g0 + lane);
+            t.nb[lane] = __ldg(a.nbins + g0 + lane);
+        }
+        const int n_dur = t.seg.n_dur;
+        int d = 0;
+        if (n_dur > 0 && n_dur <= kMaxDur) d = __ldg(a.dur_bins + t.seg.dur_off + min(lane, n_dur - 1));
+        t.dur[lane] = d;
+        if (lane < 4) t.dur[kMaxDur + lane] = 0;
+        const int d_min = __reduce_min_sync(kFull, d), d_max = __reduce_max_sync(kFull, d);
+        if (lane == 0) {
+            t.p_begin = p_begin;
+            t.p_count = p_count;
+            t.d_min = d_min;
+            t.d_max = d_max;
+            t.item = it;
+        }
+    };
+    constexpr int kFetcher = kWarps - 1;    // its share of a sweep is the smallest
+    if (warp == kFetcher) fetch(0);
+
+    for (int slot = 0;; slot ^= 1) {
         __syncthreads();
-        if (tid == 0) s.next = atomicAdd(a.work_counter, 1);
-        __syncthreads();
-        const int it = s.next;
-        if (it >= a.n_items) break;
+        const Tile& tl = s.tile[slot];
+        if (tl.item >= a.n_items) break;
         if (tid == 0) {
-            // one grid: the group is a launch parameter; several: a search
-            WorkGroup gr = a.group0;
-            if (a.n_groups > 1) {
-                int glo = 0, ghi = a.n_groups;      // groups[glo].item_begin <= it
-                while (ghi - glo > 1) {
-                    const int mid = (glo + ghi) >> 1;
-                    if (__ldg(&a.groups[mid].item_begin) <= it) glo = mid;
-                    else ghi = mid;
-                }
-                gr = a.groups[glo];
-            }
-            const int local = it - gr.item_begin;
-            const int r = local / gr.tiles_per_curve;
-            const int j = local - r * gr.tiles_per_curve;
-            const int32_t* tiles = a.seg_tiles + gr.tiles_begin;
-            int lo = 0, hi = gr.n_segments;         // tiles[lo] <= j < tiles[hi]
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (__ldg(tiles + mid) <= j) lo = mid;
-                else hi = mid;
-            }
-            const int sg = gr.seg_begin + lo;
-            const int cap = __ldg(a.seg_cap + sg);
-            s.seg = a.segments[sg];
-            WorkItem w;
-            w.curve = __ldg(a.order + gr.order_begin + r);
-            w.segment = sg;
-            w.p_begin = (j - __ldg(tiles + lo)) * cap;
-            w.p_count = min(cap, s.seg.n_periods - w.p_begin);
-            s.item = w;
-            s.curve = a.curves[w.curve];
             s.list_n = 0;
+            s.open_n = 0;
             s.rescan = 0u;
         }
-        __syncthreads();
-        const int pt = s.item.p_count;
-        const int hl = s.seg.hist_len;
-        const int n_dur = s.seg.n_dur;
-        if (pt < 1 || pt > kMaxTile || n_dur < 0 || n_dur > kMaxDur || hl < 2 ||
-            hl >= (1 << kBoxBits)) {
-            if (tid == 0) atomicExch(a.error_flag, 1);
-            continue;
-        }
-        const int64_t g0 = s.seg.period_off + s.item.p_begin;
-        if (tid < pt) {
-            s.per[tid] = a.period[g0 + tid];
-            s.freq[tid] = a.freq[g0 + tid];
-            s.scale[tid] = a.scale[g0 + tid];
-            s.nb[tid] = a.nbins[g0 + tid];
-            s.thr_bits[tid] = 0u;
-        }
-        if (tid < kMaxDur + 4) s.dur[tid] = tid < n_dur ? a.dur_bins[s.seg.dur_off + tid] : kNoBox;
-
-        double* out = a.out + s.curve.out_off + g0;
-        const int64_t ostride = a.out_stride;
-        if (s.curve.skip || n_dur == 0) {       // nothing admissible anywhere
-            if (tid < pt) {
-                out[tid] = -CUDART_INF;
-                for (int f = 1; f < kFields; ++f) out[f * ostride + tid] = 0.0;
+        // (what the fold needs is read here and again below, so that little stays in
+        // registers over it)
+        bool search;
+        {
+            const int pt = tl.p_count, hl = tl.seg.hist_len, n_dur = tl.seg.n_dur;
+            const bool bad = pt < 1 || pt > kMaxTile || n_dur < 0 || n_dur > kMaxDur || hl < 2 ||
+                             hl >= (1 << kBoxBits);
+            if (bad && tid == 0) atomicExch(a.error_flag, 1);
+            search = !bad && !tl.curve.skip && n_dur > 0;
+            if (!search) {
+                if (!bad && tid < pt) {         // nothing admissible anywhere
+                    double* out = a.out + tl.curve.out_off + tl.seg.period_off + tl.p_begin + tid;
+                    out[0] = -CUDART_INF;
+                    for (int f = 1; f < kFields; ++f) out[f * a.out_stride] = 0.0;
+                }
+                if (warp == kFetcher) fetch(slot ^ 1);
+                continue;
             }
-            continue;
+            if (tid < pt) s.thr_bits[tid] = 0u;
         }
 
         // ---- 1. fold ---------------------------------------------------------
-        const uint32_t pbytes = hist_period_bytes<MODE>(hl);
-        const uint32_t plane = plane_bytes<MODE>(hl);
         const uint32_t smem_s = smem_addr(smem);
         {
-            const int n16 = (int)((pt * pbytes) / 16);
+            const int n16 = (int)(tl.p_count * hist_period_bytes<MODE>(tl.seg.hist_len) / 16u);
             uint4* z = reinterpret_cast<uint4*>(smem);
             for (int i = tid; i < n16; i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         __syncthreads();
-        {
-            const int n = s.curve.n_points;
-            int base = 0;
-            if (MODE != MODE_GENERAL && s.seg.bin_duration > 1.5f * s.curve.gap)
-                for (; base + kChunk <= n; base += kChunk)
-                    fold_block<MODE, kPts, false, true>(a, s, smem_s, base, pt, hl);
-            else
-                for (; base + kChunk <= n; base += kChunk)
-                    fold_block<MODE, kPts, false, false>(a, s, smem_s, base, pt, hl);
-            // the tail: fewer points a lane when few are left, so that more warps
-            // share them
-            const int left = n - base;
-            if (left > 4 * kThreads)
-                fold_block<MODE, kPts, true, false>(a, s, smem_s, base, pt, hl);
-            else if (left > 2 * kThreads)
-                fold_block<MODE, 4, true, false>(a, s, smem_s, base, pt, hl);
-            else if (left > 0)
-                fold_block<MODE, 2, true, false>(a, s, smem_s, base, pt, hl);
-        }
+        fold_curve<MODE>(a, s, tl, smem_s);
         __syncthreads();
 
         // ---- 2-3. per period: pad, prefix, sweep --------------------------------
+        const int pt = tl.p_count, hl = tl.seg.hist_len, n_dur = tl.seg.n_dur;
+        const uint32_t pbytes = hist_period_bytes<MODE>(hl);
+        const uint32_t plane = plane_bytes<MODE>(hl);
         const uint32_t scr_s = smem_s + (uint32_t)pt * pbytes;       // FP32 screen copy
-        const CurveDesc& cv = s.curve;
-        const int o = s.seg.oversample;
+        const CurveDesc& cv = tl.curve;
+        const int o = tl.seg.oversample;
         auto hist = [&](int q) { return Hist{smem_s + (uint32_t)q * pbytes, plane}; };
 
         // what a lane keeps of its sweep of one period: its best and second-best group
@@ -837,12 +984,12 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
         };
 
         for (int q = 0; q < pt; ++q) {
-            const int nb = s.nb[q];
+            const int nb = tl.nb[q];
             const int L = nb + 1;
             const Hist h = hist(q);
             auto previous = [&] { if (q > 0) submit(q - 1); };
-            if constexpr (MODE == MODE_GENERAL) scan_period_f64(s, h, scr_s, L, o, previous);
-            else scan_period<MODE>(s, h, scr_s, L, o, previous);
+            if constexpr (MODE == MODE_GENERAL) scan_period_f64(s, tl, h, scr_s, L, o, previous);
+            else scan_period<MODE>(s, tl, h, scr_s, L, o, previous);
             float tmax = 0.0f;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) tmax = fmaxf(tmax, s.red_t[w]);
@@ -872,12 +1019,15 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             // weight: 1.5 * 2^-22 of the largest tm, 1.33x slack), and never 0, so
             // that a box of exactly the mean counts as the dip it is.  Ei: the same of
             // the weight (half an ulp per prefix, 2^-24 of the total; 2x slack).
+            if (one_weight<MODE>())
+                tmax += 4.0f * fabsf((float)cv.center_frac) * (float)cv.n_points;
             const float Et =
                 cv.exact_all ? CUDART_INF_F : tmax * (1.0f / 2097152.0f) + 0.0625f;
             constexpr int kShift = screen_shift<MODE>();
             const float Wt = one_weight<MODE>() ? (float)cv.n_points
                                                 : (float)ldexp(cv.i_total, -kShift);
             const float Ei = one_weight<MODE>() ? 0.0f : Wt * (1.0f / 8388608.0f);
+            const float small = cv.w_small;
 
             // Sweep: starts outer, 32 per warp and step; widths inner in groups of four
             // (one broadcast load).  Maximising snr (likelihood) is maximising the key
@@ -888,45 +1038,53 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             // exact in FP32, and th = c Et - t is 0 for an empty box (key NaN, which
             // the maximum drops).  Per-point weights: each side is lowered by the
             // weights' FP32 error; a box that this leaves without a bound, and that is
-            // not certainly empty, is evaluated in FP64 at once.  A width with no
-            // admissible start in the step (too wide, or a kNoBox slot) reads the
-            // sentinel record and its key is NaN.
+            // not certainly empty, is evaluated in FP64 at once.  In a step that some
+            // width does not fit, it reads the sentinel record and its key is NaN.
             // Screened in order with a shared threshold instead (what passes bounded and
             // listed), the passing boxes alone took as long as the sweep itself.
             double ex_v = -CUDART_INF;
             int ex_box = -1;
             {
-                int dmin = nb;
-                for (int k = 0; k < n_dur; ++k) dmin = min(dmin, s.dur[k]);
-                const int nmax_all = nb - dmin;
+                const int nmax_all = nb - tl.d_min;
+                const int n_all = nb - tl.d_max;    // every width fits a step below this
                 const uint32_t sent = scr_s + 8u * (uint32_t)L;    // first sentinel record
+                // the largest key of four widths at this lane's start
+                auto group = [&](auto fits_all, int n0, int g, uint32_t sa, float2 na,
+                                 float& den_min) -> float {
+                    const int4 dg = *reinterpret_cast<const int4*>(&tl.dur[g]);
+                    const int dk[4] = {dg.x, dg.y, dg.z, dg.w};
+                    float m = -1.0f;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        uint32_t sb = sa + 8u * (uint32_t)dk[k];
+                        if (!decltype(fits_all)::value)
+                            sb = (dk[k] < nb) & (n0 <= nb - dk[k]) ? sb : sent;
+                        const float2 diff = add_f2(ld_f2(sb), na);
+                        const float t = diff.x, c = diff.y;
+                        float th, den;
+                        if constexpr (one_weight<MODE>()) {
+                            th = fmaf(c, Et, -t);
+                            const float oc = Wt - c;
+                            den = OBJ ? c * oc * oc : c * oc;
+                        } else {
+                            th = Et - t;
+                            const float il = c - Ei, ol = fmaxf(Wt - c - Ei, 0.0f);
+                            den = OBJ ? il * ol * ol : il * ol;
+                            if (c > small) den_min = fminf(den_min, den);
+                        }
+                        m = fmaxf(m, th * fabsf(th) * rcp_approx(den));
+                    }
+                    return m;
+                };
                 for (int n0 = warp * 32; n0 <= nmax_all; n0 += kThreads) {
                     const uint32_t sa = scr_s + 8u * (uint32_t)(n0 + lane);
                     const float2 x = ld_f2(sa);
                     const float2 na = make_float2(-x.x, -x.y);
                     for (int g = 0; g < n_dur; g += 4) {
-                        const int4 dg = *reinterpret_cast<const int4*>(&s.dur[g]);
-                        const int dk[4] = {dg.x, dg.y, dg.z, dg.w};
-                        float m = -1.0f, den_min = 1.0f;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const bool fits = (dk[k] < nb) & (n0 <= nb - dk[k]);
-                            const uint32_t sb = fits ? sa + 8u * (uint32_t)dk[k] : sent;
-                            const float2 diff = add_f2(ld_f2(sb), na);
-                            const float t = diff.x, c = diff.y;
-                            float th, den;
-                            if constexpr (one_weight<MODE>()) {
-                                th = fmaf(c, Et, -t);
-                                const float oc = Wt - c;
-                                den = OBJ ? c * oc * oc : c * oc;
-                            } else {
-                                th = Et - t;
-                                const float il = c - Ei, ol = fmaxf(Wt - c - Ei, 0.0f);
-                                den = OBJ ? il * ol * ol : il * ol;
-                                if (c > cv.w_small) den_min = fminf(den_min, den);
-                            }
-                            m = fmaxf(m, th * fabsf(th) * rcp_approx(den));
-                        }
+                        float den_min = 1.0f;
+                        const float m = n0 < n_all
+                                            ? group(std::true_type{}, n0, g, sa, na, den_min)
+                                            : group(std::false_type{}, n0, g, sa, na, den_min);
                         second = fmaxf(second, fminf(m, best));
                         if (m > best) {
                             best = m;
@@ -937,7 +1095,7 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
                                 const int n = n0 + lane;
 #pragma unroll 1
                                 for (int k = 0; k < 4; ++k) {
-                                    const int d = s.dur[g + k];
+                                    const int d = tl.dur[g + k];
                                     if (d >= nb || n > nb - d) continue;
                                     const float2 diff = add_f2(ld_f2(sa + 8u * (uint32_t)d), na);
                                     const float il = diff.y - Ei;
@@ -960,22 +1118,21 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
                 }
             }
 
-            // The warp's best group publishes the largest key lower bound of its boxes
-            // that are certainly admissible dips.
+            // A warp whose best group may be the period's publishes the largest key lower
+            // bound of its boxes that are certainly admissible dips.
             {
-                const float top = warp_max(best);
-                if (best == top && top > 0.0f) {
-                    const int g = place >> kBoxBits, n = place & ((1 << kBoxBits) - 1);
-                    const uint32_t sa = scr_s + 8u * (uint32_t)n;
-                    const float2 x = ld_f2(sa);
+                const uint32_t top =
+                    __reduce_max_sync(kFull, __float_as_uint(fmaxf(best, 0.0f)));
+                if (top > *reinterpret_cast<volatile uint32_t*>(&s.thr_bits[q])) {
+                    const unsigned at = __ballot_sync(kFull, __float_as_uint(best) == top);
+                    const int pl = __shfl_sync(kFull, place, __ffs(at) - 1);
+                    const int n = pl & ((1 << kBoxBits) - 1);
+                    const int d = tl.dur[(pl >> kBoxBits) + (lane & 3)];
                     float lo = 0.0f;
-#pragma unroll 1
-                    for (int k = 0; k < 4; ++k) {
-                        const int d = s.dur[g + k];
-                        if (d >= nb || n > nb - d) continue;
-                        const float2 diff = add_f2(ld_f2(sa + 8u * (uint32_t)d),
-                                                   make_float2(-x.x, -x.y));
-                        const float t = diff.x, c = diff.y, ov = Wt - c;
+                    if (d < nb && n <= nb - d) {
+                        const uint32_t sa = scr_s + 8u * (uint32_t)n;
+                        const float2 x = ld_f2(sa), y = ld_f2(sa + 8u * (uint32_t)d);
+                        const float t = y.x - x.x, c = y.y - x.y, ov = Wt - c;
                         const float ih = c + Ei, oh = ov + Ei;
                         const float den = OBJ ? ih * oh * oh : ih * oh;
                         bool valid = (c > 0.0f) & (ov > 0.0f);
@@ -984,13 +1141,15 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
                                 (float)ldexp(cv.ivar_floor, cv.e_i - kShift) * (1.0f + 1e-3f);
                             valid = (c - Ei >= floor_q) & (ov - Ei >= floor_q) & (c > Ei) & (ov > Ei);
                         }
-                        const float tl = fmaxf(-t - Et, 0.0f);
-                        const float key = tl * tl * rcp_approx(den) * (1.0f - 2.0f * kRel);
-                        if (valid & (key < CUDART_INF_F)) lo = fmaxf(lo, key);
+                        const float tl_ = fmaxf(-t - Et, 0.0f);
+                        const float key = tl_ * tl_ * rcp_approx(den) * (1.0f - 2.0f * kRel);
+                        if (valid & (key < CUDART_INF_F)) lo = key;
                     }
-                    if (lo > 0.0f) atomicMax(&s.thr_bits[q], __float_as_uint(lo));
+                    const uint32_t lo_top = __reduce_max_sync(kFull, __float_as_uint(lo));
+                    if (lane == 0 && lo_top > 0u) atomicMax(&s.thr_bits[q], lo_top);
                 }
             }
+            if (q == 0 && warp == kFetcher) fetch(slot ^ 1);
             if constexpr (!one_weight<MODE>()) {
                 // the warp's best box without a bound is a candidate as it stands
                 if (__any_sync(kFull, ex_box >= 0)) {
@@ -1021,12 +1180,12 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             double v = -CUDART_INF;
             int key = -1;
             const Hist h = hist(q);
-            const int nb = s.nb[q];
+            const int nb = tl.nb[q];
             for (int e = lane >> 2; e < n_list; e += 8) {
                 const uint32_t c = s.list[e];
                 if ((int)(c >> 25) != q) continue;
                 const int box = (int)(c & ((1u << 25) - 1u)) + ((lane & 3) << kBoxBits);
-                const int d = s.dur[box >> kBoxBits], n = box & ((1 << kBoxBits) - 1);
+                const int d = tl.dur[box >> kBoxBits], n = box & ((1 << kBoxBits) - 1);
                 if (d < nb && n <= nb - d)
                     keep_better(v, key, exact_objective<MODE, OBJ>(h.base, h.plane, &cv, n, d), box);
             }
@@ -1047,11 +1206,11 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             for (int q = 0; q < pt; ++q) {
                 if (!(s.rescan >> q & 1u)) continue;
                 const Hist h = hist(q);
-                const int nb = s.nb[q];
+                const int nb = tl.nb[q];
                 double v = -CUDART_INF;
                 int key = -1;
                 for (int k = 0; k < n_dur; ++k) {
-                    const int d = s.dur[k];
+                    const int d = tl.dur[k];
                     for (int n = tid; d < nb && n <= nb - d; n += kThreads)
                         keep_better(v, key, exact_objective<MODE, OBJ>(h.base, h.plane, &cv, n, d),
                                     (k << kBoxBits) | n);
@@ -1079,14 +1238,15 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
         // ---- 4. the tile's seven output fields, one thread per period ----------
         if (tid < pt) {
             const int q = tid;
-            double* op = out + q;
+            double* op = a.out + tl.curve.out_off + tl.seg.period_off + tl.p_begin + q;
+            const int64_t ostride = a.out_stride;
             const int box = s.win[q];
             if (box < 0) {
                 op[0] = -CUDART_INF;
                 for (int f = 1; f < kFields; ++f) op[f * ostride] = 0.0;
             } else {
                 const int vn = box & ((1 << kBoxBits) - 1);
-                const int d = s.dur[box >> kBoxBits];
+                const int d = tl.dur[box >> kBoxBits];
                 const BoxSums b = box_sums<MODE>(hist(q), cv, vn, d);
                 const double iv_out = b.iv_out;
                 const double yin = b.y_in / b.iv_in;
@@ -1095,14 +1255,14 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
                 const double derr = sqrt(1.0 / b.iv_in + 1.0 / iv_out);
                 const double dsnr = depth / derr;
                 const double ll = 0.5 * b.iv_in * depth * depth;
-                const double bin = s.seg.bin_duration;
+                const double bin = tl.seg.bin_duration;
                 const double dur = (double)d * bin;
                 op[0] = OBJ == 0 ? dsnr : ll;
                 op[1 * ostride] = depth;
                 op[2 * ostride] = derr;
                 op[3 * ostride] = dsnr;
                 op[4 * ostride] = dur;
-                op[5 * ostride] = fmod((double)vn * bin + 0.5 * dur, s.per[q]) + cv.t_min;
+                op[5 * ostride] = fmod((double)vn * bin + 0.5 * dur, tl.per[q]) + cv.t_min;
                 op[6 * ostride] = ll;
             }
         }
