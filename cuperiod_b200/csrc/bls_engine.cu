@@ -544,6 +544,9 @@ void parallel_for(int n, F&& fn) {
 constexpr size_t kDefaultSmem[kModes] = {70 * 1024, 108 * 1024, 108 * 1024, 70 * 1024,
                                          108 * 1024};
 
+// A grid segment of at least this many periods may be cut by bin count (do_prepare).
+constexpr int kSplitPeriods = 512;
+
 size_t screen_bytes(int hl) { return ((size_t)hl + kScreenPad) * 8; }
 size_t period_bytes(int mode, int hl) { return period_hist_bytes(mode, hl); }
 
@@ -797,17 +800,49 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     for (int k = 0; k < n_grids; ++k)
         if (grid_err[k]) return fail(grid_err[k], "%s", grid_msg[k].c_str());
     std::vector<int32_t> dur_all;
-    int max_hl = 2;
     int fast_segments = 0;
     for (int s = 0; s < ns; ++s) {
         SegmentHost& sh = segs[s];
         sh.d.dur_off = (int32_t)dur_all.size();
         if (sh.empty_periods) continue;
         fast_segments += sh.d.fast_fold;
-        max_hl = std::max<int>(max_hl, sh.d.hist_len);
         dur_all.insert(dur_all.end(), sh.dur.begin(), sh.dur.end());
     }
-    (void)max_hl;
+    // The segments as the kernel sees them: a segment whose periods ascend (or descend) is
+    // cut where the phase bins of a period have grown by a quarter, so that tiles of its
+    // shorter periods take more of them (a tile's histograms are as long as its longest);
+    // the binning, widths and fold stay the whole segment's.
+    std::vector<SegmentDesc> dsegs;
+    std::vector<int> dbase(n_grids + 1, 0);
+    for (int k = 0; k < n_grids; ++k) {
+        for (int s = sbase[k]; s < sbase[k + 1]; ++s) {
+            const SegmentDesc& d = segs[s].d;
+            const PeriodConst* c = pc.data() + d.period_off;
+            bool up = true, down = true;
+            for (int32_t i = 1; i < d.n_periods; ++i) {
+                up = up && c[i].nb >= c[i - 1].nb;
+                down = down && c[i].nb <= c[i - 1].nb;
+            }
+            int32_t i0 = 0;
+            while (d.n_periods >= kSplitPeriods && (up || down) && i0 < d.n_periods) {
+                int32_t i1 = i0 + 1;
+                while (i1 < d.n_periods &&
+                       (i1 - i0 < kSplitPeriods / 8 || d.n_periods - i1 < kSplitPeriods / 8 ||
+                        4 * (int64_t)std::max(c[i1].nb, c[i0].nb) <=
+                            5 * (int64_t)std::min(c[i1].nb, c[i0].nb)))
+                    ++i1;
+                SegmentDesc part = d;
+                part.period_off = d.period_off + i0;
+                part.n_periods = i1 - i0;
+                part.hist_len = std::max(c[i0].nb, c[i1 - 1].nb) + 1;
+                dsegs.push_back(part);
+                i0 = i1;
+            }
+            if (i0 == 0) dsegs.push_back(d);
+        }
+        dbase[k + 1] = (int)dsegs.size();
+    }
+    const int nds = (int)dsegs.size();
     std::vector<int> seg_grid(ns, 0);
     for (int k = 0; k < n_grids; ++k)
         for (int s = sbase[k]; s < sbase[k + 1]; ++s) seg_grid[s] = k;
@@ -843,11 +878,19 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     int64_t n_items_mode[kModes] = {};
     std::vector<std::vector<int32_t>> members(n_grids);
     for (int m = 0; m < kModes; ++m) {
-        plan_cap[m].assign(std::max(ns, 1), 1);
+        plan_cap[m].assign(std::max(nds, 1), 1);
         if (!modes[m]) continue;
         for (auto& v : members) v.clear();
         for (int c = 0; c < nc; ++c)
             if (curves[c].d.mode == m) members[gid[c]].push_back(c);
+        // few periods in all: tiles that give every resident CTA one (1,000 periods of
+        // one 300-point curve: 23 us in tiles of 3, 42 in tiles of 16, 28 in tiles of 1)
+        int64_t searched = 0;
+        for (int k = 0; k < n_grids; ++k)
+            searched += (int64_t)members[k].size() * (pbase[k + 1] - pbase[k]);
+        const int64_t slots = (int64_t)e->n_sm * std::max(1, max_resident_ctas(m, smem_mode[m]));
+        const int spread = (int)std::min<int64_t>(
+            kMaxTile, std::max<int64_t>(1, (searched + slots - 1) / slots));
         struct Cand {
             int grid;
             int64_t tiles;
@@ -857,19 +900,21 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         std::vector<Cand> cands;
         for (int k = 0; k < n_grids; ++k) {
             if (members[k].empty()) continue;
-            Cand q{k, 0, 0.0, std::vector<int32_t>(grids[k].n_segments + 1, 0)};
+            const int n_seg = dbase[k + 1] - dbase[k];
+            Cand q{k, 0, 0.0, std::vector<int32_t>(n_seg + 1, 0)};
             int64_t acc = 0;
-            for (int sl = 0; sl < grids[k].n_segments; ++sl) {
-                const int s = sbase[k] + sl;
+            for (int sl = 0; sl < n_seg; ++sl) {
+                const int s = dbase[k] + sl;
                 q.prefix[sl] = (int32_t)acc;
-                if (segs[s].empty_periods) continue;
-                const int cap = tile_cap(m, segs[s].d.hist_len, smem_mode[m], e->tune.max_tile);
+                if (dsegs[s].n_periods == 0) continue;
+                const int cap = std::min(
+                    spread, tile_cap(m, dsegs[s].hist_len, smem_mode[m], e->tune.max_tile));
                 if (cap < 1) return fail(BLS_E_RESOURCE, "segment %d does not fit shared memory", s);
                 plan_cap[m][s] = cap;
-                acc += (segs[s].d.n_periods + cap - 1) / cap;
+                acc += (dsegs[s].n_periods + cap - 1) / cap;
                 if (acc > INT32_MAX) return fail(BLS_E_RESOURCE, "too many period tiles per curve");
             }
-            q.prefix[grids[k].n_segments] = (int32_t)acc;
+            q.prefix[n_seg] = (int32_t)acc;
             q.tiles = acc;
             if (acc == 0) continue;                  // no trial period: nothing to search
             std::stable_sort(members[k].begin(), members[k].end(), [&](int x, int y) {
@@ -886,8 +931,8 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             WorkGroup w;
             w.item_begin = (int32_t)items;
             w.tiles_per_curve = (int32_t)q.tiles;
-            w.seg_begin = sbase[q.grid];
-            w.n_segments = grids[q.grid].n_segments;
+            w.seg_begin = dbase[q.grid];
+            w.n_segments = dbase[q.grid + 1] - dbase[q.grid];
             w.order_begin = (int32_t)plan_order[m].size();
             w.tiles_begin = (int32_t)plan_tiles[m].size();
             plan_groups[m].push_back(w);
@@ -920,7 +965,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     for (int m = 0; m < kModes; ++m)
         plan_words += plan_groups[m].size() * (sizeof(WorkGroup) / 4) + plan_order[m].size() +
                       plan_tiles[m].size() + plan_cap[m].size();
-    const size_t meta_bytes = sizeof(CurveDesc) * nc + sizeof(SegmentDesc) * std::max(ns, 1) +
+    const size_t meta_bytes = sizeof(CurveDesc) * nc + sizeof(SegmentDesc) * std::max(nds, 1) +
                               sizeof(int64_t) * (2 * (size_t)nc + 1) +
                               sizeof(int32_t) * plan_words + 64;
     if ((rc = e->h_grid.ensure(grid_bytes))) return rc;
@@ -941,11 +986,11 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     char* mp = e->h_meta.as<char>();
     CurveDesc* hcur = reinterpret_cast<CurveDesc*>(mp);
     SegmentDesc* hseg = reinterpret_cast<SegmentDesc*>(hcur + nc);
-    int64_t* hspec = reinterpret_cast<int64_t*>(hseg + std::max(ns, 1));
+    int64_t* hspec = reinterpret_cast<int64_t*>(hseg + std::max(nds, 1));
     int64_t* hgbase = hspec + nc + 1;
     int32_t* hplan = reinterpret_cast<int32_t*>(hgbase + nc);
     for (int c = 0; c < nc; ++c) hcur[c] = curves[c].d;
-    for (int s = 0; s < ns; ++s) hseg[s] = segs[s].d;
+    for (int s = 0; s < nds; ++s) hseg[s] = dsegs[s];
     std::copy(spec_off.begin(), spec_off.end(), hspec);
     for (int c = 0; c < nc; ++c) hgbase[c] = pbase[gid[c]];
     size_t plan_off[kModes][4];     // per mode: groups, order, seg_tiles, seg_cap (in words)
@@ -1011,7 +1056,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     const char* dmp = e->d_curves.as<char>();
     const CurveDesc* dcur = reinterpret_cast<const CurveDesc*>(dmp);
     const SegmentDesc* dseg = reinterpret_cast<const SegmentDesc*>(dcur + nc);
-    const int64_t* dspec = reinterpret_cast<const int64_t*>(dseg + std::max(ns, 1));
+    const int64_t* dspec = reinterpret_cast<const int64_t*>(dseg + std::max(nds, 1));
     const int64_t* dgbase = dspec + nc + 1;
     const int32_t* dplan = reinterpret_cast<const int32_t*>(dgbase + nc);
     int32_t* ctl = e->d_ctl.as<int32_t>();
