@@ -39,6 +39,20 @@ N_CLASSES = 1024        # log-period bins of the grid
 IN_CHANNELS = 2
 
 _p, _i32, _i64, _f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+
+
+class _Params(ctypes.Structure):
+    """``PnNet`` / ``PnGrads`` of ``include/bls_proposal.h``: device pointers."""
+    _fields_ = [("conv_w", _p * N_CONV), ("conv_b", _p * N_CONV), ("w1", _p), ("b1", _p),
+                ("w2", _p), ("b2", _p)]
+
+    @classmethod
+    def of(cls, arrays) -> "_Params":
+        a = [_ptr(x) for x in arrays]
+        return cls((_p * N_CONV)(*a[:N_CONV]), (_p * N_CONV)(*a[N_CONV:2 * N_CONV]),
+                   *a[2 * N_CONV:])
+
+
 _bound = False
 
 
@@ -56,7 +70,12 @@ def _lib_pn() -> ctypes.CDLL:
         lib.pn_softmax_xent.argtypes = [_p, _i32, _i32, _p, _f32, _f32, _p, _p, _p]
         lib.pn_adam.argtypes = [_p, _p, _p, _p, _p, _i64, _f32, _f32, _f32, _f32, _f32, _i32, _p]
         lib.pn_topk.argtypes = [_p, _i32, _i32, _i32, _p, _p, _p]
-        for name in ("pn_gemm", "pn_bin_curves", "pn_im2col", "pn_col2im", "pn_transpose",
+        lib.pn_forward.argtypes = [_p, _p, _i32, _p, _p, _p, _p]
+        lib.pn_backward.argtypes = [_p, _p, _p, _i32, _p, _p, _p, _p, _p]
+        lib.pn_workspace.argtypes = [_i32]
+        lib.pn_scratch.argtypes = [_i32]
+        lib.pn_workspace.restype = lib.pn_scratch.restype = _i64
+        for name in ("pn_forward", "pn_backward", "pn_gemm", "pn_bin_curves", "pn_im2col", "pn_col2im", "pn_transpose",
                      "pn_colsum", "pn_softmax_xent", "pn_adam", "pn_topk"):
             getattr(lib, name).restype = ctypes.c_int
         _bound = True
@@ -215,7 +234,12 @@ class ProposalNet:
         if train:
             self.m = [torch.zeros_like(p) for p in self.master]
             self.v = [torch.zeros_like(p) for p in self.master]
-            self.g = [torch.zeros_like(p) for p in self.master]
+            # the gradients are views of one array, so that one fill clears them
+            self._g = torch.zeros(sum(p.numel() for p in self.master), device=dev)
+            self.g, at = [], 0
+            for p in self.master:
+                self.g.append(self._g[at:at + p.numel()].view_as(p))
+                at += p.numel()
             self.step = 0
 
     def weights(self, meta: dict | None = None) -> Weights:
@@ -227,29 +251,13 @@ class ProposalNet:
         """x: (B, N_BINS, IN_CHANNELS) bf16 -> logits (B, N_CLASSES) fp32."""
         torch, ops = self.torch, self.ops
         B = int(x.shape[0])
-        cache = {"x": x, "cols": [], "acts": []}
-        act, L, C = x, N_BINS, IN_CHANNELS
-        for layer in range(N_CONV):
-            k = kp(layer)
-            R = B * (L // 2)
-            col = torch.empty((R, k), dtype=torch.bfloat16, device="cuda")
-            ops.im2col(act, col, B, L, C, k)
-            y = torch.empty((R, CHANNELS), dtype=torch.bfloat16, device="cuda")
-            ops.gemm(col, self.half[layer], y, M=R, N=CHANNELS, K=k, lda=k, ldb=k,
-                     ldo=CHANNELS, mode=0, bias=self.master[N_CONV + layer], relu=True)
-            if self.train:
-                cache["cols"].append(col)
-                cache["acts"].append(y)
-            act, L, C = y, L // 2, CHANNELS
-        flat_n = CHANNELS * L
-        h = torch.empty((B, HIDDEN), dtype=torch.bfloat16, device="cuda")
-        ops.gemm(act, self.half[2 * N_CONV], h, M=B, N=HIDDEN, K=flat_n, lda=flat_n, ldb=flat_n,
-                 ldo=HIDDEN, mode=0, bias=self.master[2 * N_CONV + 1], relu=True)
+        # the activations: one buffer, kept for backward
+        ws = torch.empty(int(ops.lib.pn_workspace(B)), dtype=torch.uint8, device="cuda")
         logits = torch.empty((B, N_CLASSES), dtype=torch.float32, device="cuda")
-        ops.gemm(h, self.half[2 * N_CONV + 2], logits, M=B, N=N_CLASSES, K=HIDDEN, lda=HIDDEN,
-                 ldb=HIDDEN, ldo=N_CLASSES, mode=1, bias=self.master[2 * N_CONV + 3])
-        cache["flat"], cache["h"] = act, h
-        self._cache = cache
+        net = _Params.of([self.half.get(i, p) for i, p in enumerate(self.master)])
+        _ok(ops.lib.pn_forward(ctypes.byref(net), _ptr(x), B, _ptr(ws), _ptr(logits),
+                               _ptr(ops.err), ops._st), "pn_forward")
+        self._cache = {"x": x, "ws": ws} if self.train else None
         return logits
 
     # ---- backward and update ------------------------------------------------------------
@@ -258,63 +266,15 @@ class ProposalNet:
         torch, ops = self.torch, self.ops
         c = self._cache
         B = int(dlogits.shape[0])
-        h, flat = c["h"], c["flat"]
-        flat_n = CHANNELS * (N_BINS >> N_CONV)
-        iw1, ib1, iw2, ib2 = 2 * N_CONV, 2 * N_CONV + 1, 2 * N_CONV + 2, 2 * N_CONV + 3
-
-        def T(x, R, C):
-            out = torch.empty((C, R), dtype=torch.bfloat16, device="cuda")
-            ops.transpose(x, C, out, R, R, C)
-            return out
-
-        def splits(K, tiles):
-            return max(1, min(64, (148 * 2) // max(tiles, 1), (K + 63) // 64))
-
-        # logits = h W2^T + b2
-        dT = T(dlogits, B, N_CLASSES)                 # (N_CLASSES, B)
-        hT = T(h, B, HIDDEN)                          # (HIDDEN, B)
-        ops.gemm(dT, hT, self.g[iw2], M=N_CLASSES, N=HIDDEN, K=B, lda=B, ldb=B, ldo=HIDDEN,
-                 mode=2, splits=splits(B, 8))
-        ops.colsum(dlogits, N_CLASSES, B, N_CLASSES, self.g[ib2])
-        w2T = T(self.half[iw2], N_CLASSES, HIDDEN)    # (HIDDEN, N_CLASSES)
-        dh = torch.empty((B, HIDDEN), dtype=torch.bfloat16, device="cuda")
-        ops.gemm(dlogits, w2T, dh, M=B, N=HIDDEN, K=N_CLASSES, lda=N_CLASSES, ldb=N_CLASSES,
-                 ldo=HIDDEN, mode=0, mask=h)
-        # h = relu(flat W1^T + b1)
-        dhT = T(dh, B, HIDDEN)
-        flatT = T(flat, B, flat_n)
-        ops.gemm(dhT, flatT, self.g[iw1], M=HIDDEN, N=flat_n, K=B, lda=B, ldb=B, ldo=flat_n,
-                 mode=2, splits=splits(B, 2 * (flat_n // 256)))
-        ops.colsum(dh, HIDDEN, B, HIDDEN, self.g[ib1])
-        w1T = T(self.half[iw1], HIDDEN, flat_n)
-        dy = torch.empty((B, flat_n), dtype=torch.bfloat16, device="cuda")
-        ops.gemm(dh, w1T, dy, M=B, N=flat_n, K=HIDDEN, lda=HIDDEN, ldb=HIDDEN, ldo=flat_n,
-                 mode=0, mask=flat)
-        # the convolutions, last to first; dy is the pre-activation gradient
-        L = N_BINS >> (N_CONV - 1)
-        for layer in reversed(range(N_CONV)):
-            k = kp(layer)
-            R = B * (L // 2)
-            col = c["cols"][layer]
-            colT = T(col, R, k)                       # (k, R)
-            dyT = T(dy, R, CHANNELS)                  # (CHANNELS, R)
-            ops.gemm(colT, dyT, self.g[layer], M=k, N=CHANNELS, K=R, lda=R, ldb=R, ldo=k,
-                     mode=2, transpose=True, splits=splits(R, (k + 127) // 128))
-            ops.colsum(dy, CHANNELS, R, CHANNELS, self.g[N_CONV + layer])
-            if layer > 0:
-                wT = T(self.half[layer], CHANNELS, k)     # (k, CHANNELS)
-                dcol = torch.empty((R, k), dtype=torch.bfloat16, device="cuda")
-                ops.gemm(dy, wT, dcol, M=R, N=k, K=CHANNELS, lda=CHANNELS, ldb=CHANNELS, ldo=k,
-                         mode=0)
-                prev = c["acts"][layer - 1]           # the ReLU output this layer read
-                dx = torch.empty((B * L, CHANNELS), dtype=torch.bfloat16, device="cuda")
-                ops.col2im(dcol, prev, dx, B, L, CHANNELS, k)
-                dy = dx
-            L *= 2
+        dws = torch.empty(int(ops.lib.pn_scratch(B)), dtype=torch.uint8, device="cuda")
+        net = _Params.of([self.half.get(i, p) for i, p in enumerate(self.master)])
+        grads = _Params.of(self.g)
+        _ok(ops.lib.pn_backward(ctypes.byref(net), ctypes.byref(grads), _ptr(c["x"]), B,
+                                _ptr(c["ws"]), _ptr(dlogits), _ptr(dws), _ptr(ops.err), ops._st),
+            "pn_backward")
 
     def zero_grad(self):
-        for g in self.g:
-            g.zero_()
+        self._g.zero_()
 
     def adam(self, lr: float, *, b1=0.9, b2=0.999, eps=1e-8, wd=1e-4):
         self.step += 1

@@ -85,6 +85,45 @@ int pn_adam(float* w, float* m, float* v, const float* g, void* w16, long long n
 int pn_topk(const float* logits, int rows, int n_cls, int k, int* index, float* mass,
             void* stream);
 
+/* The network's parameters (matrices bf16, biases fp32): convolution l's weights
+ * [64][kp] with column k * C + c for tap k of input channel c (kp = 16 for the first
+ * layer, 448 after it), w1 [256][4096], w2 [1024][256]; 16-byte aligned. */
+typedef struct PnNet {
+    const void* conv_w[6];
+    const float* conv_b[6];
+    const void* w1;
+    const float* b1;
+    const void* w2;
+    const float* b2;
+} PnNet;
+
+/* Their gradients (fp32, same shapes); pn_backward adds to them. */
+typedef struct PnGrads {
+    float* conv_w[6];
+    float* conv_b[6];
+    float* w1;
+    float* b1;
+    float* w2;
+    float* b2;
+} PnGrads;
+
+/* No counterpart in the reference.  Bytes of pn_forward's workspace (the activations of B
+ * curves) and of pn_backward's scratch (their gradients, and partial sums). */
+long long pn_workspace(int B);
+long long pn_scratch(int B);
+
+/* No counterpart in the reference.  The network's logits (fp32, B x 1024) of x (bf16,
+ * B x 4096 x 2); the activations stay in ws (pn_workspace(B) bytes, 16-byte aligned)
+ * for pn_backward. */
+int pn_forward(const PnNet* net, const void* x, int B, void* ws, float* logits, int* error_flag,
+               void* stream);
+
+/* No counterpart in the reference.  From the activations of pn_forward and dlogits
+ * (bf16, B x 1024) the gradients of every parameter, added to *grads; B a multiple of
+ * 8; dws: pn_scratch(B) bytes, 16-byte aligned. */
+int pn_backward(const PnNet* net, const PnGrads* grads, const void* x, int B, const void* ws,
+                const void* dlogits, void* dws, int* error_flag, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
