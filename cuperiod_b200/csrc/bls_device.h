@@ -241,6 +241,7 @@ struct TlsCurveDesc {
     double w_total;         // the reference's float sum of w
     double y_unit;          // reference units of one quantum of yw (2^-e)
     double w_unit;          // reference units of one quantum of w
+    double merge_period;    // periods above this have bins wider than the sampling
 };
 
 struct TlsArgs {
@@ -258,7 +259,7 @@ struct TlsArgs {
     int64_t n_periods;
     int32_t* work_counter;
     int32_t* error_flag;
-    uint32_t margin_u;          // fast fold: bin-edge margin, units of 2^-32 bins
+    uint32_t margin_u;          // fast fold: edge margin (TlsFold), units of 2^-32 bins
     uint32_t margin_phi;        // fast fold: cycle-edge margin, units of 2^-32 cycles
     int32_t fast_fold;          // 1: the fast fold's error bound holds for the batch
     int32_t pad;

@@ -1524,8 +1524,10 @@ int do_prepare_tls(BlsEngine* e, const BlsTlsInputs* in, const double* periods, 
 
     // one work item: a tile of periods, each one histogram of n_bins + max_w - 1 bins
     const int ext = nb + max_w - 1;
-    const int64_t per_period = 16 * (int64_t)ext + 16 * (int64_t)nb;
-    int tile = (int)std::max<int64_t>(1, (64 * 1024 - 8 * (int64_t)n_tmpl) / per_period);
+    // (and the words of one more: tls_smem_bytes)
+    const int64_t per_period = 16 * (int64_t)ext;
+    int tile = (int)std::max<int64_t>(
+        1, (64 * 1024 - 8 * (int64_t)n_tmpl - 16 * (int64_t)nb) / per_period);
     tile = std::min<int>(tile, kTlsMaxTile);
     const size_t smem = tls_smem_bytes(nb, max_w, tile, n_tmpl);
     if (smem + 1024 > e->smem_optin)
@@ -1585,6 +1587,12 @@ int do_prepare_tls(BlsEngine* e, const BlsTlsInputs* in, const double* periods, 
         d.w_total = in->w_total[c];
         d.y_unit = std::ldexp(1.0, -e_y);
         d.w_unit = std::ldexp(1.0, -e_w);
+        double t_lo = INFINITY, t_hi = -INFINITY;
+        for (int64_t j = 0; j < n; ++j) {
+            t_lo = std::min(t_lo, in->tau[b + j]);
+            t_hi = std::max(t_hi, in->tau[b + j]);
+        }
+        d.merge_period = 1.5 * (double)nb * (t_hi - t_lo) / (double)n;
     });
     std::memcpy(h + o_per, periods, 8 * (size_t)P);
     // fast fold: the phase frac(tau * RN(1/P)) on a 2^-32 grid is within e_phi
@@ -1613,9 +1621,13 @@ int do_prepare_tls(BlsEngine* e, const BlsTlsInputs* in, const double* periods, 
             const double m_u =
                 std::ceil(((double)nb * (e_phi + e_ref) + (double)nb * std::ldexp(1.0, -52)) *
                           two32) + 2.0;
-            if (m_phi < 1e6 && m_u < 268435456.0) {
+            // TlsFold's one margin: the bin-edge error past the shift of mphi, and the
+            // 2 mphi that phases next to a cycle edge land in
+            const double shift = m_phi * (double)nb;
+            const double m_all = std::max(m_u + shift, 2.0 * shift) + 4.0;
+            if (m_phi < 1e6 && m_all < 268435456.0) {
                 fast = true;
-                mu = (uint32_t)m_u;
+                mu = (uint32_t)m_all;
                 mphi = (uint32_t)m_phi;
             }
         }
