@@ -178,6 +178,7 @@ struct JointBand {
     double y_unit;          // reference units of one quantum of y*ivar (2^-e)
     double i_unit;          // reference units of one quantum of ivar
     long long qi_total;     // sum of the band's quantised weights
+    long long qi_min;       // the smallest of them
     int32_t full_skip;      // 1: a box holding qi_total fails the floor test
     int32_t pad;
 };

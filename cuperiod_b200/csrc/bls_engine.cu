@@ -14,6 +14,7 @@
 #include <array>
 #include <atomic>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -1196,11 +1197,12 @@ int pack_joint_bands(const BlsCurves* bv, double* tau, long long* qy, long long*
             return std::max(-1000, std::min(1000, 61 - x));
         };
         const int e_y = exponent(abs_y), e_i = exponent(abs_i);
-        long long qi_total = 0;
+        long long qi_total = 0, qi_min = LLONG_MAX;
         for (int64_t j = 0; j < n; ++j) {
             qy[b + j] = std::llrint(std::ldexp(yw[j], e_y));
             qi[b + j] = std::llrint(std::ldexp(iv[j], e_i));
             qi_total += qi[b + j];
+            qi_min = std::min(qi_min, qi[b + j]);
             band_of[b + j] = (uint8_t)k;
         }
         JointBand& d = jb[k];
@@ -1214,12 +1216,12 @@ int pack_joint_bands(const BlsCurves* bv, double* tau, long long* qy, long long*
         d.ivar_floor = floor_v;
         d.y_unit = std::ldexp(1.0, -e_y);
         d.i_unit = std::ldexp(1.0, -e_i);
-        // a box holding every quantum of the band's weight: the kernel's FP64
+        // a box holding every quantum of the band's weight, or more: the kernel's FP64
         // floor test on it, operation for operation (the product is exact)
         d.qi_total = qi_total;
+        d.qi_min = qi_min;
         const double iv_all = (double)qi_total * d.i_unit;
-        const double out_all = d.sum_ivar - iv_all;
-        d.full_skip = (iv_all < d.ivar_floor || out_all < d.ivar_floor) ? 1 : 0;
+        d.full_skip = d.sum_ivar - iv_all < d.ivar_floor ? 1 : 0;
         // screen constants (the kernel's joint_screen); out of range or NaN
         // turns the screen off for the star
         const double ybar = d.sum_ivar > 0.0 ? d.sum_y / d.sum_ivar : NAN;
@@ -1362,6 +1364,7 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
     }
 
     // ---- where the histograms live ---------------------------------------------
+    hist_stride += hist_stride & 1;     // both halves whole 16-byte words
     const size_t hist_bytes = (size_t)2 * K * hist_stride * sizeof(long long);
     const bool in_smem = hist_bytes + joint_static_smem() + 1024 <= e->smem_optin;
     if (in_smem) CUDA_TRY(configure_joint(hist_bytes), "shared-memory opt-in");
