@@ -182,11 +182,9 @@ FoldParams fold_params(int64_t width, double bin, double tau_max, double f_max, 
     return fp;
 }
 
-struct PeriodConst {
-    double f;
-    uint32_t S;
-    int32_t nb;
-};
+// x to a whole number, ties to even, without a call; an x of 2^51 or more need not be exact
+// where it is used (it is out of range there).
+inline double round_even(double x) { return (x + 6755399441055744.0) - 6755399441055744.0; }
 
 // The reference's n_bins of one period (_bls_core.py:358-360 / 525-526).
 inline int64_t period_bins(double P, double bin, int oversample, int64_t width) {
@@ -197,7 +195,9 @@ inline int64_t period_bins(double P, double bin, int oversample, int64_t width) 
 struct SegmentHost {
     SegmentDesc d;
     std::vector<int32_t> dur;
+    double pmin = 0.0, pmax = 0.0;
     bool empty_periods = false;
+    bool up = true, down = true;        // phase bins per period: never fall, never rise
 };
 
 struct CurveHost {
@@ -221,7 +221,7 @@ struct BlsEngine {
         d_segments, d_rows, d_out, d_ctl, d_best, d_joint, d_tls;
     // pinned staging
     HostBuf h_tau, h_pay_r, h_r64, h_iv64, h_grid, h_meta, h_ctl, h_best, h_rows, h_joint,
-        h_tls;
+        h_tls, h_down;
 
     // the prepared batch
     bool prepared = false;
@@ -269,7 +269,7 @@ struct BlsEngine {
                           &d_joint, &d_tls})
             b->release();
         for (HostBuf* b : {&h_tau, &h_pay_r, &h_r64, &h_iv64, &h_grid, &h_meta, &h_ctl, &h_best,
-                           &h_rows, &h_joint, &h_tls})
+                           &h_rows, &h_joint, &h_tls, &h_down})
             b->release();
         if (stream) cudaStreamDestroy(stream);
     }
@@ -522,25 +522,23 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, const GridBins& gb, dou
     ch.tau_max = tau_max;
 }
 
+// fn(i, worker) for i in 0..n-1 on up to `most` of the host's threads, the caller's one of
+// them (a thread costs about 10 us to start).  fn must not throw.
 template <typename F>
-void parallel_for(int n, F&& fn) {
-    int hw = (int)std::thread::hardware_concurrency();
-    int nt = std::max(1, std::min(hw, n));
-    if (nt <= 1) {
-        for (int i = 0; i < n; ++i) fn(i, 0);
-        return;
-    }
-    std::atomic<int> next{0};
+void parallel_for(int64_t n, F&& fn, int64_t most = INT32_MAX) {
+    const int64_t hw = std::max(1, (int)std::thread::hardware_concurrency());
+    const int nt = (int)std::max<int64_t>(1, std::min({hw, n, most}));
+    std::atomic<int64_t> next{0};
+    auto work = [&](int w) {
+        for (int64_t i; (i = next.fetch_add(1)) < n;) fn((int)i, w);
+    };
     std::vector<std::thread> th;
-    th.reserve(nt);
-    for (int w = 0; w < nt; ++w)
-        th.emplace_back([&, w] {
-            for (;;) {
-                int i = next.fetch_add(1);
-                if (i >= n) break;
-                fn(i, w);
-            }
-        });
+    try {
+        th.reserve(nt - 1);
+        for (int w = 1; w < nt; ++w) th.emplace_back(work, w);
+    } catch (const std::exception&) {       // no more threads: those there do the work
+    }
+    work(0);
     for (auto& x : th) x.join();
 }
 
@@ -620,11 +618,29 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     const int64_t n_pts = cv->offsets[nc] - cv->offsets[0];
     if (cv->offsets[0] != 0 || n_pts < 0) return fail(BLS_E_INVALID, "offsets[0] must be 0");
 
-    // ---- segments (reference binning), grids in parallel ------------------------------
+    // ---- segments (reference binning) --------------------------------------------------
+    // The per-period tables are written once, into the buffer they are uploaded from, by
+    // pieces of at most kPiece periods over the host threads: 1,024 default grids took 47 ms
+    // through vectors of their own (first touches, 16 bytes a period) and a serial copy, 6 ms
+    // so; the 92,000 periods of one star's grid 1.6 ms and 0.4.
     int rc;
+    constexpr int64_t kPiece = 8192;
+    const size_t grid_bytes = (size_t)P_total * (8 + 8 + 4 + 4) + 64;
+    if ((rc = e->h_grid.ensure(grid_bytes))) return rc;
+    double* hper = e->h_grid.as<double>();
+    double* hfreq = hper + P_total;
+    uint32_t* hscale = reinterpret_cast<uint32_t*>(hfreq + P_total);
+    int32_t* hnb = reinterpret_cast<int32_t*>(hscale + P_total);
+    struct Piece {
+        int grid, seg;
+        int64_t begin, end;                     // of the concatenated periods
+        double pmin = INFINITY, pmax = 0.0, boxes = 0.0;
+        int32_t nb_max = 1;
+        bool bad = false, fast = true, up = true, down = true;
+    };
+    enum { SEG_OK, SEG_OFFSETS, SEG_NO_DUR, SEG_DUR, SEG_PERIODS, SEG_WIDTHS, SEG_BINS };
     std::vector<SegmentHost> segs(ns);
-    std::vector<double> per(P_total);
-    std::vector<PeriodConst> pc(P_total);
+    std::vector<char> seg_err(ns, SEG_OK);
     std::vector<double> grid_boxes(n_grids, 0.0), grid_trials(n_grids, 0.0);
     std::vector<int> grid_err(n_grids, BLS_OK);
     std::vector<std::string> grid_msg(n_grids);
@@ -634,56 +650,33 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     parallel_for(n_grids, [&](int k, int /*w*/) {
       try {                         // a worker thread: nothing may escape it
         const BlsGrid& g = grids[k];
-        auto bad = [&](int code, std::string msg) {
-            grid_err[k] = code;
-            grid_msg[k] = std::move(msg);
-        };
-        char buf[256];
-        int widest = 2;
+        const int64_t n_per = pbase[k + 1] - pbase[k];
         for (int sl = 0; sl < g.n_segments; ++sl) {
             const int s = sbase[k] + sl;
             const int64_t q0 = g.seg_offsets[sl], q1 = g.seg_offsets[sl + 1];   // this grid's
             const int64_t d0 = g.dur_offsets[sl], d1 = g.dur_offsets[sl + 1];
-            if (q1 < q0 || d1 < d0) {
-                std::snprintf(buf, sizeof buf, "segment %d: bad offsets", s);
-                return bad(BLS_E_INVALID, buf);
+            if (q1 < q0 || q1 > n_per || d1 < d0) {
+                seg_err[s] = SEG_OFFSETS;
+                return;
             }
-            const int64_t p0 = pbase[k] + q0, p1 = pbase[k] + q1;                // concatenated
             SegmentHost& sh = segs[s];
             SegmentDesc& sd = sh.d;
             std::memset(&sd, 0, sizeof(sd));
-            sd.period_off = p0;
-            sd.n_periods = (int32_t)(p1 - p0);
+            sd.period_off = pbase[k] + q0;                                      // concatenated
+            sd.n_periods = (int32_t)(q1 - q0);
             sd.oversample = o;
-            if (p1 == p0) {
+            if (q1 == q0) {
                 sh.empty_periods = true;
                 continue;
             }
-            if (d1 == d0) {
-                std::snprintf(buf, sizeof buf, "segment %d has no durations", s);
-                return bad(BLS_E_INVALID, buf);
-            }
-            double dmin = INFINITY, pmax = 0.0, pmin = INFINITY;
+            double dmin = INFINITY;
+            seg_err[s] = d1 == d0 ? SEG_NO_DUR : SEG_OK;
             for (int64_t i = d0; i < d1; ++i) {
                 const double d = g.durations[i];
-                if (!(std::isfinite(d) && d > 0.0)) {
-                    std::snprintf(buf, sizeof buf,
-                                  "segment %d: durations must be finite and > 0", s);
-                    return bad(BLS_E_INVALID, buf);
-                }
+                if (!(std::isfinite(d) && d > 0.0)) seg_err[s] = SEG_DUR;
                 dmin = std::min(dmin, d);
             }
-            for (int64_t i = q0; i < q1; ++i) {
-                const double P = g.periods[i];
-                if (!(std::isfinite(P) && P > 0.0)) {
-                    std::snprintf(buf, sizeof buf,
-                                  "BLS: trial periods must be finite and > 0 (segment %d)", s);
-                    return bad(BLS_E_INVALID, buf);
-                }
-                pmax = std::max(pmax, P);
-                pmin = std::min(pmin, P);
-                per[pbase[k] + i] = P;
-            }
+            if (seg_err[s] != SEG_OK) return;
             const double bin = dmin / (double)o;                              // _search_spec
             for (int64_t i = d0; i < d1; ++i) {                               // _duration_bins
                 const double kd = std::floor(g.durations[i] / bin + 0.5);
@@ -693,36 +686,118 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
                         sh.dur.push_back(kk);
                 }
             }
-            if ((int)sh.dur.size() > kMaxDur) {
-                std::snprintf(buf, sizeof buf, "segment %d: more than %d distinct box widths", s,
-                              kMaxDur);
-                return bad(BLS_E_INVALID, buf);
-            }
-            const double wmax = std::ceil(pmax / bin) + (double)o + 1.0;
-            if (!(wmax < 1073741824.0)) {
-                std::snprintf(buf, sizeof buf, "segment %d: %.3g phase bins per period", s, wmax);
-                return bad(BLS_E_RESOURCE, buf);
-            }
-            const int64_t width = (int64_t)wmax;
-            int64_t hl = 2;
-            for (int64_t i = p0; i < p1; ++i) {
-                pc[i].nb = (int32_t)period_bins(per[i], bin, o, width);
-                hl = std::max<int64_t>(hl, pc[i].nb + 1);
-            }
-            sd.width = (int32_t)width;
             sd.bin_duration = bin;
             sd.n_dur = (int32_t)sh.dur.size();
-            sd.hist_len = (int32_t)hl;
-            grid_bins[k].seg.emplace_back(bin, pmin);
-            widest = std::max<int>(widest, sd.hist_len);
+            if ((int)sh.dur.size() > kMaxDur) {         // (once its periods are looked at)
+                seg_err[s] = SEG_WIDTHS;
+                return;
+            }
         }
-        const size_t need = screen_bytes(widest) + 16 + period_hist_bytes(MODE_EXACT, widest);
-        grid_bins[k].exact_fits = need <= exact_limit;
       } catch (const std::bad_alloc&) {
         grid_err[k] = BLS_E_NOMEM;
         grid_msg[k] = "host allocation failed while preparing a grid";
       }
-    });
+    }, 1 + ns / 64);
+    std::vector<Piece> pieces;
+    for (int k = 0; k < n_grids; ++k)
+        for (int s = sbase[k]; s < sbase[k + 1] && !grid_err[k]; ++s) {
+            if (seg_err[s] != SEG_OK && seg_err[s] != SEG_WIDTHS) break;
+            const SegmentDesc& sd = segs[s].d;
+            for (int64_t i = 0; i < sd.n_periods; i += kPiece) {
+                Piece q{};
+                q.grid = k;
+                q.seg = s;
+                q.begin = sd.period_off + i;
+                q.end = sd.period_off + std::min<int64_t>(sd.n_periods, i + kPiece);
+                pieces.push_back(q);
+            }
+            if (seg_err[s] != SEG_OK) break;
+        }
+    const int64_t period_threads = 1 + P_total / (2 * kPiece);
+    parallel_for((int64_t)pieces.size(), [&](int i, int /*w*/) {
+        Piece& q = pieces[i];
+        const double bin = segs[q.seg].d.bin_duration;
+        const double* src = grids[q.grid].periods - pbase[q.grid];
+        for (int64_t j = q.begin; j < q.end; ++j) {
+            const double P = src[j];
+            q.bad |= !(std::isfinite(P) && P > 0.0);
+            q.pmax = std::max(q.pmax, P);
+            q.pmin = std::min(q.pmin, P);
+            hper[j] = P;
+            // the reference's n_bins of one period (_bls_core.py:358-360 / 525-526); its
+            // limit, the segment's width less one, is that of the longest period
+            const double nb = std::ceil(P / bin) + (double)o;
+            hnb[j] = nb < 1073741824.0 ? (int32_t)nb : 1073741824;
+            q.nb_max = std::max(q.nb_max, hnb[j]);
+        }
+    }, period_threads);
+    {
+        size_t at = 0;
+        for (int k = 0; k < n_grids; ++k) {
+            if (grid_err[k]) continue;
+            int widest = 2;
+            char buf[256];
+            auto bad = [&](int code, const char* msg) {
+                grid_err[k] = code;
+                grid_msg[k] = msg;
+            };
+            for (int s = sbase[k]; s < sbase[k + 1] && !grid_err[k]; ++s) {
+                SegmentHost& sh = segs[s];
+                SegmentDesc& sd = sh.d;
+                double pmin = INFINITY, pmax = 0.0;
+                int32_t nb_max = 1;
+                bool bad_period = false;
+                for (; at < pieces.size() && pieces[at].seg == s; ++at) {
+                    bad_period |= pieces[at].bad;
+                    pmin = std::min(pmin, pieces[at].pmin);
+                    pmax = std::max(pmax, pieces[at].pmax);
+                    nb_max = std::max(nb_max, pieces[at].nb_max);
+                }
+                switch (seg_err[s]) {
+                    case SEG_OFFSETS:
+                        std::snprintf(buf, sizeof buf, "segment %d: bad offsets", s);
+                        bad(BLS_E_INVALID, buf);
+                        continue;
+                    case SEG_NO_DUR:
+                        std::snprintf(buf, sizeof buf, "segment %d has no durations", s);
+                        bad(BLS_E_INVALID, buf);
+                        continue;
+                    case SEG_DUR:
+                        std::snprintf(buf, sizeof buf,
+                                      "segment %d: durations must be finite and > 0", s);
+                        bad(BLS_E_INVALID, buf);
+                        continue;
+                    default:
+                        break;
+                }
+                if (sh.empty_periods) continue;
+                const double wmax = std::ceil(pmax / sd.bin_duration) + (double)o + 1.0;
+                if (bad_period) {
+                    std::snprintf(buf, sizeof buf,
+                                  "BLS: trial periods must be finite and > 0 (segment %d)", s);
+                    bad(BLS_E_INVALID, buf);
+                } else if (seg_err[s] == SEG_WIDTHS) {
+                    std::snprintf(buf, sizeof buf,
+                                  "segment %d: more than %d distinct box widths", s, kMaxDur);
+                    bad(BLS_E_INVALID, buf);
+                } else if (!(wmax < 1073741824.0)) {
+                    std::snprintf(buf, sizeof buf, "segment %d: %.3g phase bins per period", s,
+                                  wmax);
+                    bad(BLS_E_RESOURCE, buf);
+                } else {
+                    sd.width = (int32_t)wmax;
+                    sd.hist_len = nb_max + 1;
+                    sh.pmin = pmin;
+                    sh.pmax = pmax;
+                    grid_bins[k].seg.emplace_back(sd.bin_duration, pmin);
+                    widest = std::max<int>(widest, sd.hist_len);
+                }
+            }
+            while (at < pieces.size() && pieces[at].grid == k) ++at;
+            const size_t need = screen_bytes(widest) + 16 + period_hist_bytes(MODE_EXACT, widest);
+            grid_bins[k].exact_fits = need <= exact_limit;
+        }
+    }
 
     // ---- curves ---------------------------------------------------------------
     if ((rc = e->h_tau.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
@@ -731,7 +806,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     if ((rc = e->h_iv64.ensure(sizeof(double) * std::max<int64_t>(n_pts, 1)))) return rc;
     std::vector<CurveHost> curves(nc);
     int hw = std::max(1, (int)std::thread::hardware_concurrency());
-    std::vector<std::vector<double>> scratch(hw);
+    std::vector<std::vector<double>> scratch(hw);     // one per worker of parallel_for
     double* htau = e->h_tau.as<double>();
     int32_t* hpr = e->h_pay_r.as<int32_t>();
     double* hr64 = e->h_r64.as<double>();
@@ -764,48 +839,62 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     }
 
     // ---- fold constants, which depend on the curves' time spans --------------------
-    parallel_for(n_grids, [&](int k, int /*w*/) {
-        if (grid_err[k]) return;
-        for (int sl = 0; sl < grids[k].n_segments; ++sl) {
-            const int s = sbase[k] + sl;
+    for (int k = 0; k < n_grids; ++k) {
+        if (grid_err[k]) continue;
+        for (int s = sbase[k]; s < sbase[k + 1]; ++s) {
             SegmentHost& sh = segs[s];
-            SegmentDesc& sd = sh.d;
             if (sh.empty_periods) continue;
-            const int64_t p0 = sd.period_off, p1 = p0 + sd.n_periods;
-            const double bin = sd.bin_duration;
-            double fmax = 0.0, smax = 0.0;
-            for (int64_t i = p0; i < p1; ++i) {
-                fmax = std::max(fmax, 1.0 / per[i]);
-                smax = std::max(smax, per[i] / bin);
-            }
-            FoldParams fp = fold_params(sd.width, bin, tau_max[k], fmax, smax);
-            const double scale = std::ldexp(1.0, fp.fb);
-            for (int64_t i = p0; i < p1 && fp.fast; ++i) {
-                const double P = per[i];
-                const double sc = std::nearbyint((P / bin) * scale);
-                if (!(sc >= 1.0 && sc < 4294967296.0)) { fp.fast = false; break; }
-                const uint32_t S = (uint32_t)sc;
-                // the fast fold's largest bin, ((S - 1) >> fb) + 1, must stay inside n_bins
-                if ((int64_t)((S - 1u) >> fp.fb) + 1 > pc[i].nb) { fp.fast = false; break; }
-            }
-            double boxes = 0.0;
-            for (int64_t i = p0; i < p1; ++i) {
-                const double P = per[i];
-                pc[i].f = 1.0 / P;
-                pc[i].S = fp.fast ? (uint32_t)std::nearbyint((P / bin) * scale) : 0u;
-                for (int32_t kk : sh.dur)
-                    if (kk < pc[i].nb) boxes += (double)(pc[i].nb - kk + 1);
-            }
-            sd.fast_fold = fp.fast;
-            sd.frac_bits = fp.fast ? fp.fb : 0;
-            sd.margin_u = fp.mu;
-            sd.margin_phi = fp.mphi;
-            grid_boxes[k] += boxes;                  // per curve of this grid
-            grid_trials[k] += (double)sd.n_periods * sh.dur.size();
+            // (rounding keeps the order: the largest quotients are the extreme periods')
+            const FoldParams fp = fold_params(sh.d.width, sh.d.bin_duration, tau_max[k],
+                                              1.0 / sh.pmin, sh.pmax / sh.d.bin_duration);
+            sh.d.fast_fold = fp.fast;
+            sh.d.frac_bits = fp.fb;
+            sh.d.margin_u = fp.mu;
+            sh.d.margin_phi = fp.mphi;
+            grid_trials[k] += (double)sh.d.n_periods * sh.dur.size();
         }
-    });
+    }
+    parallel_for((int64_t)pieces.size(), [&](int i, int /*w*/) {
+        Piece& q = pieces[i];
+        if (grid_err[q.grid]) return;
+        const SegmentHost& sh = segs[q.seg];
+        const SegmentDesc& sd = sh.d;
+        const double bin = sd.bin_duration, scale = std::ldexp(1.0, sd.frac_bits);
+        int64_t boxes = 0;
+        bool fast = sd.fast_fold != 0;
+        for (int64_t j = q.begin; j < q.end; ++j) {
+            const double P = hper[j];
+            const int32_t nb = hnb[j];
+            hfreq[j] = 1.0 / P;
+            const double sc = round_even((P / bin) * scale);
+            const bool in = sc >= 1.0 && sc < 4294967296.0;
+            const uint32_t S = in ? (uint32_t)(int64_t)sc : 0u;
+            // the fast fold's largest bin, ((S - 1) >> fb) + 1, must stay inside n_bins
+            fast = fast && in && (int64_t)((S - 1u) >> sd.frac_bits) + 1 <= nb;
+            hscale[j] = S;
+            for (int32_t kk : sh.dur) boxes += kk < nb ? nb - kk + 1 : 0;
+            if (j > sd.period_off) {
+                q.up = q.up && nb >= hnb[j - 1];
+                q.down = q.down && nb <= hnb[j - 1];
+            }
+        }
+        q.fast = fast;
+        q.boxes = (double)boxes;
+    }, period_threads);
     for (int k = 0; k < n_grids; ++k)
         if (grid_err[k]) return fail(grid_err[k], "%s", grid_msg[k].c_str());
+    for (const Piece& q : pieces) {
+        grid_boxes[q.grid] += q.boxes;              // per curve of this grid
+        SegmentHost& sh = segs[q.seg];
+        sh.up = sh.up && q.up;
+        sh.down = sh.down && q.down;
+        sh.d.fast_fold = sh.d.fast_fold && q.fast;
+    }
+    for (SegmentHost& sh : segs)
+        if (!sh.empty_periods && !sh.d.fast_fold) {
+            sh.d.frac_bits = 0;
+            std::fill_n(hscale + sh.d.period_off, sh.d.n_periods, 0u);
+        }
     std::vector<int32_t> dur_all;
     int fast_segments = 0;
     for (int s = 0; s < ns; ++s) {
@@ -824,24 +913,26 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     for (int k = 0; k < n_grids; ++k) {
         for (int s = sbase[k]; s < sbase[k + 1]; ++s) {
             const SegmentDesc& d = segs[s].d;
-            const PeriodConst* c = pc.data() + d.period_off;
-            bool up = true, down = true;
-            for (int32_t i = 1; i < d.n_periods; ++i) {
-                up = up && c[i].nb >= c[i - 1].nb;
-                down = down && c[i].nb <= c[i - 1].nb;
-            }
+            const int32_t* nb = hnb + d.period_off;
             int32_t i0 = 0;
-            while (d.n_periods >= kSplitPeriods && (up || down) && i0 < d.n_periods) {
-                int32_t i1 = i0 + 1;
-                while (i1 < d.n_periods &&
-                       (i1 - i0 < kSplitPeriods / 8 || d.n_periods - i1 < kSplitPeriods / 8 ||
-                        4 * (int64_t)std::max(c[i1].nb, c[i0].nb) <=
-                            5 * (int64_t)std::min(c[i1].nb, c[i0].nb)))
-                    ++i1;
+            while (d.n_periods >= kSplitPeriods && (segs[s].up || segs[s].down) &&
+                   i0 < d.n_periods) {
+                // the first period, kSplitPeriods / 8 on, that is a quarter away; the rest
+                // stays together when fewer than that are left
+                int32_t i1 = std::min(i0 + kSplitPeriods / 8, d.n_periods), hi = d.n_periods;
+                while (i1 < hi) {
+                    const int32_t mid = i1 + (hi - i1) / 2;
+                    if (4 * (int64_t)std::max(nb[mid], nb[i0]) <=
+                        5 * (int64_t)std::min(nb[mid], nb[i0]))
+                        i1 = mid + 1;
+                    else
+                        hi = mid;
+                }
+                if (d.n_periods - i1 < kSplitPeriods / 8) i1 = d.n_periods;
                 SegmentDesc part = d;
                 part.period_off = d.period_off + i0;
                 part.n_periods = i1 - i0;
-                part.hist_len = std::max(c[i0].nb, c[i1 - 1].nb) + 1;
+                part.hist_len = std::max(nb[i0], nb[i1 - 1]) + 1;
                 dsegs.push_back(part);
                 i0 = i1;
             }
@@ -965,31 +1056,18 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     // ---- stage metadata and upload ---------------------------------------------
     int64_t n_items = 0;
     for (int m = 0; m < kModes; ++m) n_items += n_items_mode[m];
-    const size_t grid_bytes = (size_t)P_total * (8 + 8 + 4 + 4) + dur_all.size() * 4 + 64;
     // descriptors, per-curve spectrum offsets and grid bases (int64), then per
-    // mode: groups, order, seg_tiles and seg_cap (int32 words)
+    // mode: groups, order, seg_tiles and seg_cap (int32 words), then the box widths
     size_t plan_words = 0;
     for (int m = 0; m < kModes; ++m)
         plan_words += plan_groups[m].size() * (sizeof(WorkGroup) / 4) + plan_order[m].size() +
                       plan_tiles[m].size() + plan_cap[m].size();
+    const size_t dur_word = plan_words;             // the box widths, last
+    plan_words += dur_all.size();
     const size_t meta_bytes = sizeof(CurveDesc) * nc + sizeof(SegmentDesc) * std::max(nds, 1) +
                               sizeof(int64_t) * (2 * (size_t)nc + 1) +
                               sizeof(int32_t) * plan_words + 64;
-    if ((rc = e->h_grid.ensure(grid_bytes))) return rc;
     if ((rc = e->h_meta.ensure(meta_bytes))) return rc;
-    char* gp = e->h_grid.as<char>();
-    double* hper = reinterpret_cast<double*>(gp);
-    double* hfreq = hper + P_total;
-    uint32_t* hscale = reinterpret_cast<uint32_t*>(hfreq + P_total);
-    int32_t* hnb = reinterpret_cast<int32_t*>(hscale + P_total);
-    int32_t* hdur = hnb + P_total;
-    for (int64_t i = 0; i < P_total; ++i) {
-        hper[i] = per[i];
-        hfreq[i] = pc[i].f;
-        hscale[i] = pc[i].S;
-        hnb[i] = pc[i].nb;
-    }
-    std::copy(dur_all.begin(), dur_all.end(), hdur);
     char* mp = e->h_meta.as<char>();
     CurveDesc* hcur = reinterpret_cast<CurveDesc*>(mp);
     SegmentDesc* hseg = reinterpret_cast<SegmentDesc*>(hcur + nc);
@@ -1018,6 +1096,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             w += plan_cap[m].size();
         }
     }
+    std::copy(dur_all.begin(), dur_all.end(), hplan + dur_word);
     for (int m = 0; m < kModes; ++m) e->n_items_mode[m] = (int32_t)n_items_mode[m];
 
     const size_t out_elems = (size_t)kFields * std::max<int64_t>(spec_total, 1);
@@ -1045,7 +1124,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
                  "upload weights");
         h2d += (int64_t)n_pts * 16;
     }
-    CUDA_TRY(cudaMemcpyAsync(e->d_period.p, gp, grid_bytes, cudaMemcpyHostToDevice, st),
+    CUDA_TRY(cudaMemcpyAsync(e->d_period.p, hper, grid_bytes, cudaMemcpyHostToDevice, st),
              "upload grid");
     CUDA_TRY(cudaMemcpyAsync(e->d_curves.p, mp, meta_bytes, cudaMemcpyHostToDevice, st),
              "upload descriptors");
@@ -1060,7 +1139,6 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     const double* dfreq = dper + P_total;
     const uint32_t* dscale = reinterpret_cast<const uint32_t*>(dfreq + P_total);
     const int32_t* dnb = reinterpret_cast<const int32_t*>(dscale + P_total);
-    const int32_t* ddur = dnb + P_total;
     const char* dmp = e->d_curves.as<char>();
     const CurveDesc* dcur = reinterpret_cast<const CurveDesc*>(dmp);
     const SegmentDesc* dseg = reinterpret_cast<const SegmentDesc*>(dcur + nc);
@@ -1088,7 +1166,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         a.freq = dfreq;
         a.scale = dscale;
         a.nbins = dnb;
-        a.dur_bins = ddur;
+        a.dur_bins = dplan + dur_word;
         a.out = e->d_out.as<double>();
         a.out_stride = spec_total;
         a.work_counter = ctl + m;
@@ -1168,6 +1246,44 @@ int ensure_graph(BlsEngine* e, cudaStream_t st) {
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) return cuda_fail(ce, "graph instantiate");
     e->graph_valid = true;
+    return BLS_OK;
+}
+
+// Copies `bytes` from the device to the caller's (pageable) memory.  A large copy goes through
+// pinned slots, one per thread, so that the slots' copies, the caller's page faults and the
+// copies out of the slots overlap: 22 MB of spectra took 9.4 ms as one pageable copy (the
+// driver's single thread), 2 ms so.  The copies stay in stream order; all have arrived on
+// return.
+int copy_out(BlsEngine* e, void* out, const void* src, size_t bytes, cudaStream_t st) {
+    constexpr size_t kSlot = 1 << 20;
+    constexpr int kSlots = 8;
+    const int64_t n = (int64_t)((bytes + kSlot - 1) / kSlot);
+    if (n < 2) {
+        CUDA_TRY(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, st), "download");
+        return BLS_OK;
+    }
+    int rc;
+    if ((rc = e->h_down.ensure(kSlot * kSlots))) return rc;
+    CUDA_TRY(cudaStreamSynchronize(st), "wait for the outputs");
+    std::atomic<int> err{(int)cudaSuccess};
+    std::atomic<int64_t> next{0};
+    auto work = [&](int, int slot) {
+        char* h = e->h_down.as<char>() + (size_t)slot * kSlot;
+        cudaEvent_t ev = nullptr;
+        cudaError_t ce = cudaSetDevice(e->device);
+        if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        for (int64_t i; ce == cudaSuccess && (i = next.fetch_add(1)) < n;) {
+            const size_t at = (size_t)i * kSlot, len = std::min(kSlot, bytes - at);
+            ce = cudaMemcpyAsync(h, (const char*)src + at, len, cudaMemcpyDeviceToHost, st);
+            if (ce == cudaSuccess) ce = cudaEventRecord(ev, st);
+            if (ce == cudaSuccess) ce = cudaEventSynchronize(ev);
+            if (ce == cudaSuccess) std::memcpy((char*)out + at, h, len);
+        }
+        if (ev) cudaEventDestroy(ev);
+        if (ce != cudaSuccess) err = (int)ce;
+    };
+    parallel_for(kSlots, work, std::min<int64_t>(kSlots, n));
+    if (err != (int)cudaSuccess) return cuda_fail((cudaError_t)err.load(), "download");
     return BLS_OK;
 }
 
@@ -1325,7 +1441,7 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
         sd.dur_off = (int32_t)dur_all.size();
         if (p1 == p0) continue;
         if (d1 == d0) return fail(BLS_E_INVALID, "segment %d has no durations", s);
-        double dmin = INFINITY, pmax = 0.0;
+        double dmin = INFINITY, pmax = 0.0, pmin = INFINITY;
         for (int64_t i = d0; i < d1; ++i) {
             const double d = g->durations[i];
             if (!(std::isfinite(d) && d > 0.0))
@@ -1338,6 +1454,7 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
                 return fail(BLS_E_INVALID,
                             "BLS: trial periods must be finite and > 0 (segment %d)", s);
             pmax = std::max(pmax, P);
+            pmin = std::min(pmin, P);
         }
         const double bin = dmin / (double)o;
         std::vector<int32_t> dur;
@@ -1366,24 +1483,19 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
         sd.hist_len = (int32_t)hl;
         hist_stride = std::max(hist_stride, hl);
         dur_all.insert(dur_all.end(), dur.begin(), dur.end());
-        // fast fold, with the single-band search's margins and checks
-        double fmax = 0.0, smax = 0.0;
-        for (int64_t i = p0; i < p1; ++i) {
-            fmax = std::max(fmax, 1.0 / g->periods[i]);
-            smax = std::max(smax, g->periods[i] / bin);
-        }
-        FoldParams fp = fold_params(width, bin, tau_max, fmax, smax);
+        // fast fold, with the single-band search's margins and checks (rounding keeps the
+        // order: the largest quotients are the extreme periods')
+        FoldParams fp = fold_params(width, bin, tau_max, 1.0 / pmin, pmax / bin);
         const double sc_unit = std::ldexp(1.0, fp.fb);
-        for (int64_t i = p0; i < p1 && fp.fast; ++i) {
-            const double sc = std::nearbyint((g->periods[i] / bin) * sc_unit);
-            if (!(sc >= 1.0 && sc < 4294967296.0)) { fp.fast = false; break; }
-            // the fast fold's largest bin, ((S - 1) >> fb) + 1, must stay inside n_bins
-            if ((int64_t)(((uint32_t)sc - 1u) >> fp.fb) + 1 > nbins[i]) { fp.fast = false; break; }
-        }
         for (int64_t i = p0; i < p1; ++i) {
             freq[i] = 1.0 / g->periods[i];
-            scale[i] = fp.fast ? (uint32_t)std::nearbyint((g->periods[i] / bin) * sc_unit) : 0u;
+            const double sc = round_even((g->periods[i] / bin) * sc_unit);
+            const bool in = sc >= 1.0 && sc < 4294967296.0;
+            scale[i] = in ? (uint32_t)(int64_t)sc : 0u;
+            // the fast fold's largest bin, ((S - 1) >> fb) + 1, must stay inside n_bins
+            fp.fast = fp.fast && in && (int64_t)((scale[i] - 1u) >> fp.fb) + 1 <= nbins[i];
         }
+        if (!fp.fast) std::fill(scale.begin() + p0, scale.begin() + p1, 0u);
         sd.fast_fold = fp.fast ? 1 : 0;
         sd.frac_bits = fp.fast ? fp.fb : 0;
         sd.margin_u = fp.mu;
@@ -1946,9 +2058,8 @@ int bls_download(BlsEngine* e, double* out, void* stream) {
     cudaSetDevice(e->device);
     cudaStream_t st = pick(e, stream);
     const size_t bytes = sizeof(double) * kFields * (size_t)e->spec_total;
-    if (bytes) CUDA_TRY(cudaMemcpyAsync(out, e->d_out.p, bytes, cudaMemcpyDeviceToHost, st),
-                        "download outputs");
-    return check_device_flag(e, st);
+    const int rc = bytes ? copy_out(e, out, e->d_out.p, bytes, st) : BLS_OK;
+    return rc ? rc : check_device_flag(e, st);
 }
 
 int bls_download_curves(BlsEngine* e, const int32_t* curve_ids, int32_t n_ids, double* out,
@@ -1967,10 +2078,10 @@ int bls_download_curves(BlsEngine* e, const int32_t* curve_ids, int32_t n_ids, d
     for (int32_t k = 0; k < n_ids; ++k) {
         const int64_t b = e->spec_off[curve_ids[k]], len = e->spec_off[curve_ids[k] + 1] - b;
         for (int f = 0; f < kFields; ++f) {
-            if (len > 0)
-                CUDA_TRY(cudaMemcpyAsync(out + w, d + (size_t)f * e->spec_total + b,
-                                         sizeof(double) * (size_t)len, cudaMemcpyDeviceToHost, st),
-                         "download a curve's field");
+            const int rc = len > 0 ? copy_out(e, out + w, d + (size_t)f * e->spec_total + b,
+                                              sizeof(double) * (size_t)len, st)
+                                   : BLS_OK;
+            if (rc) return rc;
             w += (size_t)len;
         }
     }
