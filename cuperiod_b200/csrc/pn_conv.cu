@@ -46,7 +46,7 @@ constexpr uint32_t kWeights = kTaps * kWTap;
 constexpr int kWinRows = 136;                       // 128 rows and the taps' shifts, to 8
 constexpr uint32_t kWin = kWinRows * 128;
 constexpr int kMaxStages = 4;
-constexpr int kConvThreads = 192;                   // producer, MMA, four epilogue warps
+constexpr int kConvThreads = 320;                   // producer, MMA, eight epilogue warps
 constexpr uint32_t kSmemMax = 226 * 1024;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) {
@@ -98,7 +98,7 @@ __device__ __forceinline__ void bulk_wait_all() {
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t tmem_alloc(uint32_t slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot),
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(tf + 8 * s, 1);
-            mbar_init(te + 8 * s, 1);
+            mbar_init(te + 8 * s, BWD ? 4 : 8);         // the warps that read it
         }
         mbar_init(wb, 1);
         abort_s = 0;
@@ -261,13 +261,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
     } else if (threadIdx.x == 32) {
         constexpr uint32_t idesc = BWD ? bf16_idesc(128, 32) | kIdescBMn : bf16_idesc(128, 64);
+        const uint64_t dW = BWD ? sw128_mn_desc(sW, 1024) : sw128_desc(sW);
         bool ok = mbar_wait(wb, 0u);
         if (!ok) give_up();
         int n = 0;
         for (int t = blockIdx.x; ok && t < a.n_tiles; t += gridDim.x, ++n) {
             const int st = n % S;
             const uint32_t in = sIn + st * kStage;
-            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / S) & 1u) || *dead) ok = false;
+            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / S) & 1u)) ok = false;
+            const uint64_t dA = sw128_desc(in);
             for (int half = 0; ok && half < (BWD ? 2 : 1); ++half) {
                 // accumulator and how often it was used before
                 const int acc = BWD ? half : n & 1, use = BWD ? n : n / 2;
@@ -284,15 +286,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     // +2 .. -1; the window starts at row -1, and a tap has its own
                     // accumulator
                     const int sh = (k & 1) ? 2 - (k >> 1) : 3 - (k >> 1);
-                    const uint32_t A = BWD ? in + sh * (WINDOW ? 128 : kTile)
-                                       : WINDOW ? in + (k & 1) * kWin + (k >> 1) * 128
-                                                : in + k * kTile;
-                    const uint32_t W = sW + k * kWTap;
+                    const uint32_t A = BWD ? sh * (WINDOW ? 128 : kTile)
+                                       : WINDOW ? (k & 1) * kWin + (k >> 1) * 128
+                                                : k * kTile;
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        umma_bf16(BWD ? D + k * 32 : D, sw128_desc(A + kk * 32),
-                                  BWD ? sw128_mn_desc(W + half * 64 + kk * 2048, 1024)
-                                      : sw128_desc(W + kk * 32),
+                        umma_bf16(BWD ? D + k * 32 : D, desc_at(dA, A + kk * 32),
+                                  desc_at(dW, k * kWTap + (BWD ? half * 64 + kk * 2048 : kk * 32)),
                                   idesc, kk == 0 && (BWD || k == 0) ? 0u : 1u);
                 }
                 umma_commit(tf + 8 * acc);
@@ -304,78 +304,79 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             umma_commit(eb + 8 * st);
         }
     } else if (warp >= 2) {
-        const int quarter = warp & 3, r = quarter * 32 + lane;
+        // warps 2-5 take channels 0-31 (backward: the first accumulator), 6-9 the others
+        const int quarter = warp & 3, part = (warp - 2) >> 2, r = quarter * 32 + lane;
         bool ok = true;
         int n = 0;
         for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++n) {
             const int st = n % S;
             const uint32_t out = sOut + (n & 1) * kOut * kTile;
-            if (threadIdx.x == 64) bulk_wait_read<1>();     // the store of tile n - 2
-            epi_sync();
+            const int acc = BWD ? part : n & 1, use = BWD ? n : n / 2;
+            if (ok) ok = mbar_wait(tf + 8 * acc, (uint32_t)use & 1u) && !*dead;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok && lane == 0) give_up();
+            auto release = [&] {                    // the accumulator is read
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(te + 8 * acc);
+            };
+            if (ok) {
+                tc_fence_after();
+                const uint32_t D = tmem + ((uint32_t)(quarter * 32) << 16) + acc * kAcc;
+                if (BWD) {
+                    const uint32_t mask = sIn + st * kStage + kMask;
 #pragma unroll 1
-            for (int part = 0; part < 2; ++part) {          // halves of 32 channels
-                const int acc = BWD ? part : n & 1, use = BWD ? n : n / 2;
-                if (ok && (BWD || part == 0))
-                    ok = mbar_wait(tf + 8 * acc, (uint32_t)use & 1u) && !*dead;
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok && lane == 0) give_up();
-                if (ok) {
-                    tc_fence_after();
-                    const uint32_t D = tmem + ((uint32_t)(quarter * 32) << 16) + acc * kAcc;
-                    if (BWD) {
-                        const uint32_t mask = sIn + st * kStage + kMask;
+                    for (int e = 0; e < 2; ++e) {
+                        // the taps' products are rounded to bf16 one by one and added
+                        // in tap order
+                        float sum[32];
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) sum[i] = 0.0f;
 #pragma unroll 1
-                        for (int e = 0; e < 2; ++e) {
-                            // the taps' products are rounded to bf16 one by one and added
-                            // in tap order
-                            float sum[32];
+                        for (int k = e ^ 1; k < kTaps; k += 2) {
+                            float v[32];
+                            tmem_ld32(D + k * 32, v);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) sum[i] = 0.0f;
-#pragma unroll 1
-                            for (int k = e ^ 1; k < kTaps; k += 2) {
-                                float v[32];
-                                tmem_ld32(D + k * 32, v);
-#pragma unroll
-                                for (int i = 0; i < 32; i += 2) {
-                                    const uint32_t p = pack2(v[i], v[i + 1]);
-                                    sum[i] += __uint_as_float(p << 16);
-                                    sum[i + 1] += __uint_as_float(p & 0xffff0000u);
-                                }
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const uint4 m = lds128(chunk(mask + e * kTile, r, part * 4 + j));
-                                sts128(chunk(out + e * kTile, r, part * 4 + j),
-                                       make_uint4(pack2_masked(sum[8 * j], sum[8 * j + 1], m.x),
-                                                  pack2_masked(sum[8 * j + 2], sum[8 * j + 3], m.y),
-                                                  pack2_masked(sum[8 * j + 4], sum[8 * j + 5], m.z),
-                                                  pack2_masked(sum[8 * j + 6], sum[8 * j + 7], m.w)));
+                            for (int i = 0; i < 32; i += 2) {
+                                const uint32_t p = pack2(v[i], v[i + 1]);
+                                sum[i] += __uint_as_float(p << 16);
+                                sum[i + 1] += __uint_as_float(p & 0xffff0000u);
                             }
                         }
-                    } else {
-                        float v[32];
-                        tmem_ld32(D + part * 32, v);
+                        if (e == 1) release();
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                v[8 * j + i] =
-                                    fmaxf(v[8 * j + i] + s_bias[part * 32 + 8 * j + i], 0.0f);
-                            sts128(chunk(out, r, part * 4 + j),
-                                   make_uint4(pack2(v[8 * j], v[8 * j + 1]),
-                                              pack2(v[8 * j + 2], v[8 * j + 3]),
-                                              pack2(v[8 * j + 4], v[8 * j + 5]),
-                                              pack2(v[8 * j + 6], v[8 * j + 7])));
+                            const uint4 m = lds128(chunk(mask + e * kTile, r, part * 4 + j));
+                            sts128(chunk(out + e * kTile, r, part * 4 + j),
+                                   make_uint4(pack2_masked(sum[8 * j], sum[8 * j + 1], m.x),
+                                              pack2_masked(sum[8 * j + 2], sum[8 * j + 3], m.y),
+                                              pack2_masked(sum[8 * j + 4], sum[8 * j + 5], m.z),
+                                              pack2_masked(sum[8 * j + 6], sum[8 * j + 7], m.w)));
                         }
                     }
-                }
-                tc_fence_before();
-                if (part == 1) fence_async_smem();
-                if (BWD || part == 1) {
-                    epi_sync();
-                    if (threadIdx.x == 64) mbar_arrive(te + 8 * acc);
+                } else {
+                    float v[32];
+                    tmem_ld32(D + part * 32, v);
+                    release();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            v[8 * j + i] =
+                                fmaxf(v[8 * j + i] + s_bias[part * 32 + 8 * j + i], 0.0f);
+                        sts128(chunk(out, r, part * 4 + j),
+                               make_uint4(pack2(v[8 * j], v[8 * j + 1]),
+                                          pack2(v[8 * j + 2], v[8 * j + 3]),
+                                          pack2(v[8 * j + 4], v[8 * j + 5]),
+                                          pack2(v[8 * j + 6], v[8 * j + 7])));
+                    }
                 }
             }
+            // (the stores that may still read the other buffer are those of tile n - 1, so
+            // past this barrier it is free for tile n + 1)
+            if (threadIdx.x == 64) bulk_wait_read<0>();
+            fence_async_smem();
+            epi_sync();
             if (threadIdx.x == 64) {
                 if (BWD) mbar_arrive(eb + 8 * st);          // the masks are read
                 if (ok && !*dead) {
@@ -406,6 +407,7 @@ constexpr int kWgWinRows = 72;
 constexpr uint32_t kWgWin = kWgWinRows * 128;
 constexpr uint32_t kWgStage = 64 * 128 + 2 * kWgWin;        // dY, odd-plane and even-plane rows
 constexpr int kWgStages = 6;
+constexpr int kWgThreads = 192;                     // producer, MMA, four reading warps
 
 struct WgradArgs {
     int n_blocks;           // blocks of 64 rows
@@ -420,7 +422,7 @@ constexpr int kWgPart = 8 * 64 * 64;
 // (two taps, one row apart in their window, or tap 5 and the block of ones), N = 64 --
 // and writes its sums to the workspace, which wgrad_sum_kernel adds up (adding them to the
 // gradient with atomics took three times the products' time).
-__global__ void __launch_bounds__(kConvThreads, 1)
+__global__ void __launch_bounds__(kWgThreads, 1)
     conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy,
                       const __grid_constant__ CUtensorMap tmX, const WgradArgs a) {
     extern __shared__ uint8_t dsm_raw[];
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (uint32_t i = threadIdx.x; i < 64 * 128 / 16; i += kConvThreads)
+    for (uint32_t i = threadIdx.x; i < 64 * 128 / 16; i += kWgThreads)
         sts128(sOnes + 16 * i, make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u));
     fence_async_smem();
     if (warp == 1) tmem_alloc(saddr(&tmem_slot), 256);
@@ -476,21 +478,21 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         int n = 0;
         for (int t = blockIdx.x; t < a.n_blocks; t += gridDim.x, ++n) {
             const int st = n % kWgStages;
-            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / kWgStages) & 1u) || *dead) {
+            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / kWgStages) & 1u)) {
                 give_up();
                 break;
             }
             tc_fence_after();
             const uint32_t dy = sIn + st * kWgStage, p1 = dy + 8192, p0 = p1 + kWgWin;
+            const uint64_t dB = sw128_mn_desc(dy, 1024);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 // taps 0, 2 | 4, 6 of the odd plane, 1, 3 | 5 of the even one
                 const uint32_t A = (m < 2 ? p1 : p0) + (m & 1) * 256;
-                const uint32_t lbo = m < 3 ? 128u : sOnes - A;
+                const uint64_t dA = sw128_mn_desc(A, m < 3 ? 128u : sOnes - A);
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk)
-                    umma_bf16(tmem + m * 64, sw128_mn_desc(A + kk * 2048, lbo),
-                              sw128_mn_desc(dy + kk * 2048, 1024), idesc,
+                    umma_bf16(tmem + m * 64, desc_at(dA, kk * 2048), desc_at(dB, kk * 2048), idesc,
                               n > 0 || kk > 0 ? 1u : 0u);
             }
             umma_commit(eb + 8 * st);
@@ -670,7 +672,8 @@ struct Wgrad0Args {
     float* part;            // per CTA [16][64 n]: 14 inputs, the bias, nothing
     int* error_flag;
 };
-constexpr int kWg0Stages = 8;
+constexpr int kWg0Stages = 4;
+constexpr int kWg0Ctas = 3;         // an SM: laying out a block's rows is what takes the time
 constexpr uint32_t kWg0Stage = 2 * 64 * 128;
 constexpr int kWg0Part = 16 * 64;
 
@@ -678,7 +681,7 @@ constexpr int kWg0Part = 16 * 64;
 // two warps lay out a block's 64 rows of 14 inputs and a 1 (the bias) as the M-major
 // operand, M = 128 of which 15 are used, N = 64, K = 64 rows a block.
 template <bool PAIRS>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(128, kWg0Ctas)
     conv0_wgrad_kernel(const __grid_constant__ CUtensorMap tmDy, const Wgrad0Args a) {
     extern __shared__ uint8_t dsm_raw[];
     __shared__ __align__(8) uint64_t full_bar[kWg0Stages], empty_bar[kWg0Stages];
@@ -729,16 +732,16 @@ __global__ void __launch_bounds__(128, 1)
         int n = 0;
         for (int t = blockIdx.x; t < a.n_blocks; t += gridDim.x, ++n) {
             const int st = n % kWg0Stages;
-            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / kWg0Stages) & 1u) || *dead) {
+            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / kWg0Stages) & 1u)) {
                 give_up();
                 break;
             }
             tc_fence_after();
-            const uint32_t dy = sIn + st * kWg0Stage, p = dy + 64 * 128;
+            const uint32_t dy = sIn + st * kWg0Stage;
+            const uint64_t dA = sw128_mn_desc(dy + 64 * 128, 0), dB = sw128_mn_desc(dy, 1024);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                umma_bf16(tmem, sw128_mn_desc(p + kk * 2048, 0), sw128_mn_desc(dy + kk * 2048, 1024),
-                          idesc, n > 0 || kk > 0 ? 1u : 0u);
+                umma_bf16(tmem, desc_at(dA, kk * 2048), desc_at(dB, kk * 2048), idesc, n > 0 || kk > 0 ? 1u : 0u);
             umma_commit(eb + 8 * st);
         }
         umma_commit(db);
@@ -795,13 +798,19 @@ __global__ void __launch_bounds__(128, 1)
     if (warp == 0) tmem_free(tmem, 64);
 }
 
-// gw, gb += those partial sums, in order.
-__global__ void __launch_bounds__(64)
+// gw, gb += those partial sums: 16 runs of them, then the runs in order.
+__global__ void __launch_bounds__(1024)
     wgrad0_sum_kernel(const float* part, int n_parts, float* gw, float* gb) {
-    const int k = blockIdx.x, n = threadIdx.x;
+    __shared__ float sum[16][64];
+    const int k = blockIdx.x, n = threadIdx.x & 63, run = threadIdx.x >> 6;
+    const int per = (n_parts + 15) / 16, end = min(n_parts, (run + 1) * per);
     float s = 0.0f;
-#pragma unroll 8
-    for (int z = 0; z < n_parts; ++z) s += part[(int64_t)z * kWg0Part + k * 64 + n];
+#pragma unroll 4
+    for (int z = run * per; z < end; ++z) s += part[(int64_t)z * kWg0Part + k * 64 + n];
+    sum[run][n] = s;
+    __syncthreads();
+    if (run != 0) return;
+    for (int g = 1; g < 16; ++g) s += sum[g][n];
     if (k < 14) gw[n * 16 + k] += s;
     else gb[n] += s;
 }
@@ -831,10 +840,16 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* g, 
 
 // ---- the MLP's products --------------------------------------------------------------------
 
-constexpr int kFcStages = 6;
 constexpr uint32_t kFcA = 128 * 128;
 template <int BN>
 __host__ __device__ constexpr uint32_t fc_stage() { return kFcA + BN * 128; }
+// K blocks of one stage (one wait: the issuing thread spends about 300 cycles on a wait, as
+// long as on five products), and as many stages as fit
+constexpr int kFcBlocks = 3;
+template <int BN>
+__host__ __device__ constexpr int fc_stages() {
+    return (int)((kSmemMax - 1024) / (kFcBlocks * fc_stage<BN>()));
+}
 template <int BN>
 __host__ __device__ constexpr int fc_pitch() { return BN + 4; }     // floats of a partial row
 
@@ -863,7 +878,7 @@ __global__ void __launch_bounds__(128, 1)
     fc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
               const FcArgs g) {
     constexpr uint32_t kFcStage = fc_stage<BN>();
-    constexpr int kFcPitch = fc_pitch<BN>();
+    constexpr int kFcPitch = fc_pitch<BN>(), kFcStages = fc_stages<BN>();
     extern __shared__ uint8_t dsm_raw[];
     __shared__ __align__(8) uint64_t full_bar[kFcStages], empty_bar[kFcStages];
     __shared__ __align__(8) uint64_t done_bar;
@@ -896,41 +911,50 @@ __global__ void __launch_bounds__(128, 1)
         atomicExch(g.error_flag, 1);
     };
     if (tid == 0) {
-        for (int i = 0; i < nk; ++i) {
-            const int st = i % kFcStages;
-            if (i >= kFcStages && !mbar_wait(eb + 8 * st, (uint32_t)(i / kFcStages - 1) & 1u)) {
+        for (int i = 0, n = 0; i < nk; i += kFcBlocks, ++n) {
+            const int st = n % kFcStages, blocks = min(kFcBlocks, nk - i);
+            if (n >= kFcStages && !mbar_wait(eb + 8 * st, (uint32_t)(n / kFcStages - 1) & 1u)) {
                 give_up();
                 break;
             }
             if (*dead) break;
-            const uint32_t in = sIn + st * kFcStage, bar = fb + 8 * st;
-            const int k0 = (kb0 + i) * 64;
-            mbar_expect_tx(bar, kFcStage);
-            if (A_MN) {
-                tma_load_2d(in, &tmA, m0, k0, bar);
-                tma_load_2d(in + kFcA / 2, &tmA, m0 + 64, k0, bar);
-            } else {
-                tma_load_2d(in, &tmA, k0, m0, bar);
+            const uint32_t bar = fb + 8 * st;
+            mbar_expect_tx(bar, blocks * kFcStage);
+            for (int q = 0; q < blocks; ++q) {
+                const uint32_t in = sIn + (st * kFcBlocks + q) * kFcStage;
+                const int k0 = (kb0 + i + q) * 64;
+                if (A_MN) {
+                    tma_load_2d(in, &tmA, m0, k0, bar);
+                    tma_load_2d(in + kFcA / 2, &tmA, m0 + 64, k0, bar);
+                } else {
+                    tma_load_2d(in, &tmA, k0, m0, bar);
+                }
+                if (B_MN) tma_load_2d(in + kFcA, &tmB, n0, k0, bar);
+                else tma_load_2d(in + kFcA, &tmB, k0, n0, bar);
             }
-            if (B_MN) tma_load_2d(in + kFcA, &tmB, n0, k0, bar);
-            else tma_load_2d(in + kFcA, &tmB, k0, n0, bar);
         }
     } else if (tid == 32) {
         constexpr uint32_t idesc =
             bf16_idesc(128, BN) | (A_MN ? kIdescAMn : 0u) | (B_MN ? kIdescBMn : 0u);
-        for (int i = 0; i < nk; ++i) {
-            const int st = i % kFcStages;
-            if (!mbar_wait(fb + 8 * st, (uint32_t)(i / kFcStages) & 1u) || *dead) {
+        for (int i = 0, n = 0; i < nk; i += kFcBlocks, ++n) {
+            const int st = n % kFcStages, blocks = min(kFcBlocks, nk - i);
+            if (!mbar_wait(fb + 8 * st, (uint32_t)(n / kFcStages) & 1u)) {
                 give_up();
                 break;
             }
             tc_fence_after();
-            const uint32_t A = sIn + st * kFcStage, B = A + kFcA;
+            const uint32_t A = sIn + st * kFcBlocks * kFcStage, B = A + kFcA;
+            const uint64_t dA = A_MN ? sw128_mn_desc(A, kFcA / 2) : sw128_desc(A);
+            const uint64_t dB = B_MN ? sw128_mn_desc(B, 1024) : sw128_desc(B);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                umma_bf16(tmem, A_MN ? sw128_mn_desc(A + kk * 2048, kFcA / 2) : sw128_desc(A + kk * 32),
-                          B_MN ? sw128_mn_desc(B + kk * 2048, 1024) : sw128_desc(B + kk * 32), idesc,
-                          i > 0 || kk > 0 ? 1u : 0u);
+            for (int q = 0; q < kFcBlocks; ++q) {
+                if (q >= blocks) break;
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    umma_bf16(tmem, desc_at(dA, q * kFcStage + kk * (A_MN ? 2048 : 32)),
+                              desc_at(dB, q * kFcStage + kk * (B_MN ? 2048 : 32)), idesc,
+                              i > 0 || q > 0 || kk > 0 ? 1u : 0u);
+            }
             umma_commit(eb + 8 * st);
         }
         umma_commit(db);
@@ -1127,7 +1151,7 @@ int conv_weight_grad(const void* dY, const void* X, float* gw, float* gb, float*
     WgradArgs a{(int)((long long)B * L / kWgRows), L, part, err};
     // at least four blocks a CTA, so that adding the sums stays small beside forming them
     const int ctas = a.n_blocks / 4 < n_sm ? (a.n_blocks + 3) / 4 : n_sm;
-    conv_wgrad_kernel<<<ctas, kConvThreads, smem, st>>>(dy, x, a);
+    conv_wgrad_kernel<<<ctas, kWgThreads, smem, st>>>(dy, x, a);
     wgrad_sum_kernel<<<8 * 16, 1024, 0, st>>>(part, ctas, gw, gb);
     return launched();
 }
@@ -1153,12 +1177,13 @@ int conv0_weight_grad(const void* dY, const void* x, float* gw, float* gb, float
     if (rc) return rc;
     constexpr size_t smem = 1024 + kWg0Stages * kWg0Stage;
     Wgrad0Args a{reinterpret_cast<const __nv_bfloat16*>(x), (int)((long long)B * L / 64), L, part, err};
-    const int ctas = a.n_blocks < n_sm ? a.n_blocks : n_sm;
+    const int ctas = a.n_blocks < n_sm * kWg0Ctas ? a.n_blocks : n_sm * kWg0Ctas;
+    static_assert(kWg0Ctas * kWg0Part <= kWgPart, "the workspace holds kWgPart floats an SM");
     const bool pairs = (reinterpret_cast<uintptr_t>(x) & 3u) == 0;
     const auto k = pairs ? conv0_wgrad_kernel<true> : conv0_wgrad_kernel<false>;
     if (raise_smem_limit((const void*)k, smem) != cudaSuccess) return PN_E_CUDA;
     k<<<ctas, 128, smem, st>>>(dy, a);
-    wgrad0_sum_kernel<<<15, 64, 0, st>>>(part, ctas, gw, gb);
+    wgrad0_sum_kernel<<<15, 1024, 0, st>>>(part, ctas, gw, gb);
     return launched();
 }
 
@@ -1175,7 +1200,7 @@ int fc(const void* A, bool a_mn, const void* B, bool b_mn, FcArgs g, int n_sm, c
     int splits = 1;             // enough CTAs for the SMs, at least two K blocks each
     while (g.add && splits < 8 && tiles * splits * 2 <= n_sm && nk >= splits * 4) splits *= 2;
     g.kb_per = (nk + splits - 1) / splits;
-    constexpr size_t smem = 1024 + kFcStages * fc_stage<BN>();
+    constexpr size_t smem = 1024 + fc_stages<BN>() * kFcBlocks * fc_stage<BN>();
     using Kernel = void (*)(CUtensorMap, CUtensorMap, FcArgs);
     Kernel k;
     if constexpr (BN == 64)

@@ -70,6 +70,11 @@ __device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t addr, uint32_t lbo) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
+// The descriptor of the same layout `bytes` further on (the address field does not carry:
+// shared memory ends below 2^18).
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) {
+    return (desc & 0xffffffff00000000ull) | (uint32_t)((uint32_t)desc + (bytes >> 4));
+}
 // A K-major tile without swizzle: 8 x 16-byte core matrices, `lbo` bytes apart along K
 // and `sbo` bytes apart along M.
 __device__ __forceinline__ uint64_t plain_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
