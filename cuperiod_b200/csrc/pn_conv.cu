@@ -156,17 +156,22 @@ __device__ __forceinline__ uint32_t chunk(uint32_t tile, int r, int j) {
 
 // ---- the convolution and its input gradient ---------------------------------------
 
+// Backward: the masks' stages (2 tiles each) are their own, since they are read last: held
+// with the input's they kept the next loads from starting until the epilogue was over.
+template <bool BWD, bool WINDOW>
+__host__ __device__ constexpr int conv_mask_stages() { return !BWD ? 0 : WINDOW ? 2 : 1; }
+
 struct ConvArgs {
     int n_tiles;            // tiles of 128 rows (row pairs)
     int L;                  // rows (pairs) of one curve: 64 or a multiple of 128
-    int stages;
+    int stages;             // of the input
     const float* bias;      // forward
     int* error_flag;
 };
 
 template <bool BWD, bool WINDOW>
 __host__ __device__ constexpr uint32_t conv_stage_bytes() {
-    return BWD ? (WINDOW ? kWin : 4 * kTile) + 2 * kTile : (WINDOW ? 2 * kWin : kTaps * kTile);
+    return BWD ? (WINDOW ? kWin : 4 * kTile) : (WINDOW ? 2 * kWin : kTaps * kTile);
 }
 
 // BWD: tmIn is dY as {64, L, B}, tmOut dX and tmMask the convolution's input, both as
@@ -182,15 +187,17 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 const __grid_constant__ CUtensorMap tmOut,
                 const __grid_constant__ CUtensorMap tmMask, const ConvArgs a) {
     constexpr uint32_t kStage = conv_stage_bytes<BWD, WINDOW>();
-    constexpr uint32_t kMask = WINDOW ? kWin : 4 * kTile;      // BWD: masks' offset in a stage
-    // accumulator columns: forward 64 a tile, two tiles; backward 32 a tap (half of the
-    // channels), two halves
-    constexpr int kAcc = BWD ? kTaps * 32 : 64;
+    constexpr int kMasks = BWD ? conv_mask_stages<BWD, WINDOW>() : 1;
+    // accumulator columns: forward 64 a tile, two tiles; backward 64 a tap, three taps of
+    // the even positions and four of the odd ones (N = 32 and halves of the channels
+    // instead took 52 cycles a product, N = 64 about 60: both read all of A)
+    constexpr int kAcc = BWD ? 3 * 64 : 64;
     constexpr int kCols = BWD ? 512 : 128;
     constexpr int kOut = BWD ? 2 : 1;                          // output tiles of a tile
     extern __shared__ uint8_t dsm_raw[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages];
     __shared__ __align__(8) uint64_t tfull_bar[2], tempty_bar[2], w_bar;
+    __shared__ __align__(8) uint64_t mfull_bar[2], mempty_bar[2];
     __shared__ float s_bias[kCh];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_s;
@@ -199,15 +206,19 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     const uint32_t sOut = sW + kWeights;                       // 2 x kOut tiles
     const uint32_t sIn = sOut + 2 * kOut * kTile;
     const uint32_t fb = saddr(full_bar), eb = saddr(empty_bar), tf = saddr(tfull_bar),
-                   te = saddr(tempty_bar), wb = saddr(&w_bar);
+                   te = saddr(tempty_bar), wb = saddr(&w_bar), mf = saddr(mfull_bar),
+                   me = saddr(mempty_bar);
+    const uint32_t sMask = sIn + a.stages * kStage;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(fb + 8 * s, 1);
-            mbar_init(eb + 8 * s, BWD ? 2 : 1);
+            mbar_init(eb + 8 * s, 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(tf + 8 * s, 1);
             mbar_init(te + 8 * s, BWD ? 4 : 8);         // the warps that read it
+            mbar_init(mf + 8 * s, 1);
+            mbar_init(me + 8 * s, 1);
         }
         mbar_init(wb, 1);
         abort_s = 0;
@@ -255,12 +266,19 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 else
                     for (int k = 0; k < 4; ++k)
                         tma_load_3d(in + k * kTile, &tmIn, 0, o0 - 1 + k, b, bar);
-                tma_load_4d(in + kMask, &tmMask, 0, 0, o0, b, bar);
-                tma_load_4d(in + kMask + kTile, &tmMask, 0, 1, o0, b, bar);
+                const int ms = n % kMasks;
+                if (n >= kMasks && !mbar_wait(me + 8 * ms, (uint32_t)(n / kMasks - 1) & 1u)) {
+                    give_up();
+                    break;
+                }
+                const uint32_t mask = sMask + ms * 2 * kTile;
+                mbar_expect_tx(mf + 8 * ms, 2 * kTile);
+                tma_load_4d(mask, &tmMask, 0, 0, o0, b, mf + 8 * ms);
+                tma_load_4d(mask + kTile, &tmMask, 0, 1, o0, b, mf + 8 * ms);
             }
         }
     } else if (threadIdx.x == 32) {
-        constexpr uint32_t idesc = BWD ? bf16_idesc(128, 32) | kIdescBMn : bf16_idesc(128, 64);
+        constexpr uint32_t idesc = bf16_idesc(128, 64) | (BWD ? kIdescBMn : 0u);
         const uint64_t dW = BWD ? sw128_mn_desc(sW, 1024) : sw128_desc(sW);
         bool ok = mbar_wait(wb, 0u);
         if (!ok) give_up();
@@ -270,9 +288,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             const uint32_t in = sIn + st * kStage;
             if (!mbar_wait(fb + 8 * st, (uint32_t)(n / S) & 1u)) ok = false;
             const uint64_t dA = sw128_desc(in);
-            for (int half = 0; ok && half < (BWD ? 2 : 1); ++half) {
+#pragma unroll
+            for (int e = 0; e < (BWD ? 2 : 1); ++e) {
+                if (!ok) break;
                 // accumulator and how often it was used before
-                const int acc = BWD ? half : n & 1, use = BWD ? n : n / 2;
+                const int acc = BWD ? e : n & 1, use = BWD ? n : n / 2;
                 if (use >= 1 && !mbar_wait(te + 8 * acc, (uint32_t)(use - 1) & 1u)) {
                     ok = false;
                     break;
@@ -280,7 +300,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 tc_fence_after();
                 const uint32_t D = tmem + acc * kAcc;
 #pragma unroll
-                for (int k = 0; k < kTaps; ++k) {
+                for (int k = BWD ? e ^ 1 : 0; k < kTaps; k += BWD ? 2 : 1) {
                     // forward: rows of the tap's parity plane.  Backward: parity 0 takes
                     // taps 1, 3, 5 at rows +1, 0, -1, parity 1 taps 0, 2, 4, 6 at rows
                     // +2 .. -1; the window starts at row -1, and a tap has its own
@@ -291,8 +311,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                                                 : k * kTile;
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        umma_bf16(BWD ? D + k * 32 : D, desc_at(dA, A + kk * 32),
-                                  desc_at(dW, k * kWTap + (BWD ? half * 64 + kk * 2048 : kk * 32)),
+                        umma_bf16(BWD ? D + (k >> 1) * 64 : D, desc_at(dA, A + kk * 32),
+                                  desc_at(dW, k * kWTap + kk * (BWD ? 2048 : 32)),
                                   idesc, kk == 0 && (BWD || k == 0) ? 0u : 1u);
                 }
                 umma_commit(tf + 8 * acc);
@@ -304,15 +324,16 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             umma_commit(eb + 8 * st);
         }
     } else if (warp >= 2) {
-        // warps 2-5 take channels 0-31 (backward: the first accumulator), 6-9 the others
+        // warps 2-5 take channels 0-31 (backward: the even positions), 6-9 the others
         const int quarter = warp & 3, part = (warp - 2) >> 2, r = quarter * 32 + lane;
         bool ok = true;
         int n = 0;
         for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++n) {
-            const int st = n % S;
+            const int ms = n % kMasks;
             const uint32_t out = sOut + (n & 1) * kOut * kTile;
             const int acc = BWD ? part : n & 1, use = BWD ? n : n / 2;
             if (ok) ok = mbar_wait(tf + 8 * acc, (uint32_t)use & 1u) && !*dead;
+            if (BWD && ok) ok = mbar_wait(mf + 8 * ms, (uint32_t)(n / kMasks) & 1u);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok && lane == 0) give_up();
             auto release = [&] {                    // the accumulator is read
@@ -324,18 +345,18 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 tc_fence_after();
                 const uint32_t D = tmem + ((uint32_t)(quarter * 32) << 16) + acc * kAcc;
                 if (BWD) {
-                    const uint32_t mask = sIn + st * kStage + kMask;
+                    const uint32_t mask = sMask + (ms * 2 + part) * kTile;
 #pragma unroll 1
-                    for (int e = 0; e < 2; ++e) {
+                    for (int c = 0; c < 2; ++c) {
                         // the taps' products are rounded to bf16 one by one and added
                         // in tap order
                         float sum[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) sum[i] = 0.0f;
 #pragma unroll 1
-                        for (int k = e ^ 1; k < kTaps; k += 2) {
+                        for (int k = 0; k < 3 + part; ++k) {
                             float v[32];
-                            tmem_ld32(D + k * 32, v);
+                            tmem_ld32(D + k * 64 + c * 32, v);
 #pragma unroll
                             for (int i = 0; i < 32; i += 2) {
                                 const uint32_t p = pack2(v[i], v[i + 1]);
@@ -343,11 +364,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                                 sum[i + 1] += __uint_as_float(p & 0xffff0000u);
                             }
                         }
-                        if (e == 1) release();
+                        if (c == 1) release();
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const uint4 m = lds128(chunk(mask + e * kTile, r, part * 4 + j));
-                            sts128(chunk(out + e * kTile, r, part * 4 + j),
+                            const uint4 m = lds128(chunk(mask, r, c * 4 + j));
+                            sts128(chunk(out + part * kTile, r, c * 4 + j),
                                    make_uint4(pack2_masked(sum[8 * j], sum[8 * j + 1], m.x),
                                               pack2_masked(sum[8 * j + 2], sum[8 * j + 3], m.y),
                                               pack2_masked(sum[8 * j + 4], sum[8 * j + 5], m.z),
@@ -378,7 +399,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             fence_async_smem();
             epi_sync();
             if (threadIdx.x == 64) {
-                if (BWD) mbar_arrive(eb + 8 * st);          // the masks are read
+                if (BWD) mbar_arrive(me + 8 * ms);          // the masks are read
                 if (ok && !*dead) {
                     const int row = t * kRows;
                     if (BWD) {
@@ -1097,7 +1118,8 @@ template <bool BWD, bool WINDOW>
 int launch_conv(const CUtensorMap& in, const CUtensorMap& w, const CUtensorMap& out,
                 const CUtensorMap& mask, ConvArgs a, int n_sm, cudaStream_t st) {
     constexpr uint32_t stage = conv_stage_bytes<BWD, WINDOW>();
-    constexpr uint32_t fixed = 1024 + kWeights + 2 * (BWD ? 2 : 1) * kTile;
+    constexpr uint32_t fixed = 1024 + kWeights + 2 * (BWD ? 2 : 1) * kTile +
+                               conv_mask_stages<BWD, WINDOW>() * 2 * kTile;
     constexpr int fit = (int)((kSmemMax - fixed) / stage);
     constexpr int stages = fit < kMaxStages ? fit : kMaxStages;
     static_assert(stages >= 1, "a stage must fit");
