@@ -224,11 +224,16 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (!BWD && threadIdx.x < kCh) s_bias[threadIdx.x] = a.bias[threadIdx.x];
     if (warp == 1) tmem_alloc(saddr(&tmem_slot), kCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) dependents_may_launch();
+    wait_for_prior();
+    if (!BWD) {
+        if (threadIdx.x < kCh) s_bias[threadIdx.x] = a.bias[threadIdx.x];
+        __syncthreads();
+    }
     const uint32_t tmem = tmem_slot;
     const int S = a.stages;
     volatile int* dead = &abort_s;
@@ -471,6 +476,8 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) dependents_may_launch();
+    wait_for_prior();
     const uint32_t tmem = tmem_slot;
     volatile int* dead = &abort_s;
     auto give_up = [&] {
@@ -559,6 +566,8 @@ __global__ void __launch_bounds__(1024)
     const float* p = part + tap * 64 * 64 + n * 64 + c;
     const int per = (n_parts + 3) / 4, end = min(n_parts, (group + 1) * per);
     float s = 0.0f;
+    dependents_may_launch();
+    wait_for_prior();
 #pragma unroll 8
     for (int z = group * per; z < end; ++z) s += p[(int64_t)z * kWgPart];
     sum[group][i] = s;
@@ -609,16 +618,18 @@ __global__ void __launch_bounds__(128)
         mbar_init(db, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 0) tmem_alloc(saddr(&tmem_slot), 64);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0) dependents_may_launch();
+    wait_for_prior();
     if (tid < kCh) s_bias[tid] = a.bias[tid];
     {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.w) + tid);   // row tid / 2, half tid & 1
         const int r = tid >> 1;
         sts128(W + (uint32_t)((r >> 3) * 256 + (tid & 1) * 128 + (r & 7) * 16), v);
     }
-    if (warp == 0) tmem_alloc(saddr(&tmem_slot), 64);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const int L_in = 2 * a.L;
     auto load_row = [&](int t, uint32_t (&v)[7]) {
@@ -730,6 +741,8 @@ __global__ void __launch_bounds__(128, kWg0Ctas)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) dependents_may_launch();
+    wait_for_prior();
     const uint32_t tmem = tmem_slot;
     volatile int* dead = &abort_s;
     auto give_up = [&] {
@@ -826,6 +839,8 @@ __global__ void __launch_bounds__(1024)
     const int k = blockIdx.x, n = threadIdx.x & 63, run = threadIdx.x >> 6;
     const int per = (n_parts + 15) / 16, end = min(n_parts, (run + 1) * per);
     float s = 0.0f;
+    dependents_may_launch();
+    wait_for_prior();
 #pragma unroll 4
     for (int z = run * per; z < end; ++z) s += part[(int64_t)z * kWg0Part + k * 64 + n];
     sum[run][n] = s;
@@ -842,10 +857,12 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* g, 
     __shared__ float sum[8][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 64;
     float s0 = 0.0f, s1 = 0.0f;
+    dependents_may_launch();
+    wait_for_prior();
 #pragma unroll 8
     for (int m = warp; m < M; m += 8) {
-        const uint32_t v =
-            __ldg(reinterpret_cast<const uint32_t*>(g + (int64_t)m * N + n) + lane);
+        // (not __ldg: the kernel that writes g may still run when this one is launched)
+        const uint32_t v = reinterpret_cast<const uint32_t*>(g + (int64_t)m * N + n)[lane];
         s0 += __uint_as_float(v << 16);
         s1 += __uint_as_float(v & 0xffff0000u);
     }
@@ -925,6 +942,8 @@ __global__ void __launch_bounds__(128, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) dependents_may_launch();
+    wait_for_prior();
     const uint32_t tmem = tmem_slot;
     volatile int* dead = &abort_s;
     auto give_up = [&] {
@@ -1112,7 +1131,23 @@ int sm_count() {
     return n;
 }
 
-int launched() { return cudaGetLastError() == cudaSuccess ? PN_OK : PN_E_CUDA; }
+// A launch that may begin before the kernel ahead of it on the stream has ended (each of these
+// kernels waits for it): a pass is 8 to 34 launches, 1 to 2 us apart without this.
+template <typename... Params, typename... Args>
+int launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
+           const Args&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? PN_OK : PN_E_CUDA;
+}
 
 template <bool BWD, bool WINDOW>
 int launch_conv(const CUtensorMap& in, const CUtensorMap& w, const CUtensorMap& out,
@@ -1127,9 +1162,8 @@ int launch_conv(const CUtensorMap& in, const CUtensorMap& w, const CUtensorMap& 
     if (raise_smem_limit((const void*)conv_kernel<BWD, WINDOW>, smem) != cudaSuccess)
         return PN_E_CUDA;
     a.stages = stages;
-    conv_kernel<BWD, WINDOW><<<a.n_tiles < n_sm ? a.n_tiles : n_sm, kConvThreads, smem, st>>>(
-        in, w, out, mask, a);
-    return launched();
+    return launch(conv_kernel<BWD, WINDOW>, a.n_tiles < n_sm ? a.n_tiles : n_sm, kConvThreads, smem,
+                  st, in, w, out, mask, a);
 }
 
 // Y = relu(conv(X) + bias): X [B][2 L][64], Y [B][L][64], W [64][448] (tap-major columns).
@@ -1173,9 +1207,8 @@ int conv_weight_grad(const void* dY, const void* X, float* gw, float* gb, float*
     WgradArgs a{(int)((long long)B * L / kWgRows), L, part, err};
     // at least four blocks a CTA, so that adding the sums stays small beside forming them
     const int ctas = a.n_blocks / 4 < n_sm ? (a.n_blocks + 3) / 4 : n_sm;
-    conv_wgrad_kernel<<<ctas, kWgThreads, smem, st>>>(dy, x, a);
-    wgrad_sum_kernel<<<8 * 16, 1024, 0, st>>>(part, ctas, gw, gb);
-    return launched();
+    rc = launch(conv_wgrad_kernel, ctas, kWgThreads, smem, st, dy, x, a);
+    return rc ? rc : launch(wgrad_sum_kernel, 8 * 16, 1024, 0, st, (const float*)part, ctas, gw, gb);
 }
 
 int conv0_forward(const void* x, const void* W, const float* bias, void* Y, int B, int L, int n_sm,
@@ -1187,9 +1220,9 @@ int conv0_forward(const void* x, const void* W, const float* bias, void* Y, int 
                 bias, (int)((long long)B * L / kRows), L, err};
     const int ctas = a.n_tiles < n_sm * kConv0Ctas ? a.n_tiles : n_sm * kConv0Ctas;
     constexpr size_t smem = 1024 + kTile;
-    if ((reinterpret_cast<uintptr_t>(x) & 3u) == 0) conv0_kernel<true><<<ctas, 128, smem, st>>>(out, a);
-    else conv0_kernel<false><<<ctas, 128, smem, st>>>(out, a);
-    return launched();
+    return launch((reinterpret_cast<uintptr_t>(x) & 3u) == 0 ? conv0_kernel<true>
+                                                             : conv0_kernel<false>,
+                  ctas, 128, smem, st, out, a);
 }
 
 int conv0_weight_grad(const void* dY, const void* x, float* gw, float* gb, float* part, int B, int L,
@@ -1204,9 +1237,8 @@ int conv0_weight_grad(const void* dY, const void* x, float* gw, float* gb, float
     const bool pairs = (reinterpret_cast<uintptr_t>(x) & 3u) == 0;
     const auto k = pairs ? conv0_wgrad_kernel<true> : conv0_wgrad_kernel<false>;
     if (raise_smem_limit((const void*)k, smem) != cudaSuccess) return PN_E_CUDA;
-    k<<<ctas, 128, smem, st>>>(dy, a);
-    wgrad0_sum_kernel<<<15, 1024, 0, st>>>(part, ctas, gw, gb);
-    return launched();
+    const int rc2 = launch(k, ctas, 128, smem, st, dy, a);
+    return rc2 ? rc2 : launch(wgrad0_sum_kernel, 15, 1024, 0, st, (const float*)part, ctas, gw, gb);
 }
 
 // One product of the MLP; a_mn / b_mn as fc_kernel.
@@ -1235,19 +1267,21 @@ int fc(const void* A, bool a_mn, const void* B, bool b_mn, FcArgs g, int n_sm, c
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 1;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = splits;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k, ta, tb, g) == cudaSuccess ? PN_OK : PN_E_CUDA;
 }
 
 int bias_grad(const void* g, int M, int N, float* db, cudaStream_t st) {
-    bias_grad_kernel<<<N / 64, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(g), M, N, db);
-    return launched();
+    return launch(bias_grad_kernel, N / 64, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(g), M,
+                  N, db);
 }
 
 constexpr int kNetBins = 4096, kNetConv = 6, kNetHidden = 256, kNetClasses = 1024;

@@ -18,6 +18,17 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
+// Programmatic dependent launch: a kernel may be launched while the one before it on the
+// stream still runs.  dependents_may_launch goes after a CTA's tensor-memory allocation
+// (a dependent that held the columns would wait for this grid, and this grid for them);
+// wait_for_prior comes before the first access to global memory.
+__device__ __forceinline__ void dependents_may_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_prior() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
