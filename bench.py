@@ -608,12 +608,13 @@ def run_ours(args) -> None:
         P = info["n_periods"]
         alg_bytes = n_pts * 12 + P * 24 + 7 * 8 * n_curves * P
         achieved = alg_bytes / (kernel_ms / 1000.0) / 1e9
-        # SM-pipe model: 3 native shared atomics per fold at the measured random
-        # rate, 2 FP64 ops per fold, ~10 FP32 ops per box (rates from
+        # SM-pipe model: the native shared atomics of a fold (2 with one weight per
+        # curve, 4 with per-point weights) at the measured random rate, 2 FP64 ops per fold, ~10 FP32 ops per box (rates from
         # csrc/pipe_probe.cu, profiles/pipe_rates.txt)
         f_clk = (clocks.get("sm_mhz") or 1900.0) * 1e6
         n_sm = torch.cuda.get_device_properties(local).multi_processor_count
-        t_atom = info["folds"] * 3 / (16.66 * n_sm * f_clk)
+        words = 2 if args.weights == "uniform" else 4
+        t_atom = info["folds"] * words / (16.66 * n_sm * f_clk)
         t_fp64 = info["folds"] * 2 / (108.0 * n_sm * f_clk)
         t_fp32 = info["boxes"] * 10 / (188.0 * n_sm * f_clk)
         t_pipe = max(t_atom, t_fp64, t_fp32)
@@ -1207,7 +1208,7 @@ def run_catalogue(args) -> None:
         n_sm = torch.cuda.get_device_properties(0).multi_processor_count
         folds = sum(r["folds"] for r in pruned.chunks)
         boxes = sum(r["boxes"] for r in pruned.chunks)
-        t_atom = folds * 3 / (16.66 * n_sm * clocks_mhz * 1e6)
+        t_atom = folds * 2 / (16.66 * n_sm * clocks_mhz * 1e6)
         t_fp32 = boxes * 10 / (188.0 * n_sm * clocks_mhz * 1e6)
         h2d = sum(r["h2d_bytes"] for r in pruned.chunks)
         peaks = {}

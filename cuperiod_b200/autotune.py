@@ -53,7 +53,7 @@ class TileShape:
         return f"smem={smem},tile={tile}"
 
 
-# The engine's defaults first (72 KB and three CTAs per SM for one weight per
+# The engine's defaults first (70 KB and three CTAs per SM for one weight per
 # curve, 108 KB and two for per-point weights), then capped tiles at the default
 # occupancy, then fewer resident CTAs with larger tiles.
 CANDIDATES: tuple[TileShape, ...] = (

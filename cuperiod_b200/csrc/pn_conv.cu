@@ -22,7 +22,7 @@
 //    shared memory in rank order.
 //
 // With the patch matrices, transposes and column sums in memory a pass over 1,024 curves
-// took 2,630 us and a training step of 256 curves 3,370 us; as built 282 and 506 us.
+// took 2,630 us and a training step of 256 curves 3,370 us; as built 240 and 374 us.
 //
 // Every wait on an mbarrier is bounded; one that runs out sets the error flag, after which
 // the CTA's roles finish their loops without further waits or stores.

@@ -1,6 +1,8 @@
 // Kernels of the learned period-proposal network (sm_100a).  No counterpart in
 // the reference: the network ranks log-period windows of the full BLS grid so
 // that the exact search can be restricted to them.
+// The forward and backward passes are in pn_conv.cu; here are single steps that a caller
+// may compose, and those the passes share:
 //
 //   * pn_gemm_kernel<BN>: D[M, N] = A[M, K] . B[N, K]^T, bf16 operands (both
 //     K-major), fp32 accumulation in tensor memory.  One CTA per 128 x BN output
