@@ -482,10 +482,11 @@ void pack_curve(const BlsCurves* cv, int c, int64_t off, const GridBins& gb, dou
         rq_total = rtotal;
         iq_total = total;
         // half the smallest weight in the FP32 screen's units, when the FP32 error of a
-        // box's weight (half an ulp per prefix: 2^-24 of the total) is at most half that
+        // box's weight (5 x 2^-24 of the total: two prefixes of up to twice the total, and
+        // their difference) is less than half that
         const int shift = screen_shift(wide ? MODE_WIDE : MODE_EXACT);
         const double small = std::ldexp(min_i, e_i - shift);
-        if (!d.exact_all && small > std::ldexp(i_total, -shift - 22))
+        if (!d.exact_all && small > std::ldexp(i_total, -shift - 20))
             d.w_small = (float)(0.5 * small);
     } else if (!uniform) {
         // per-point weights: FP64 values scaled by powers of two (exact)

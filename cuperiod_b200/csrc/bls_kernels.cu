@@ -1018,7 +1018,10 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             // (one rounding per prefix, one per difference: 2^-22, 2x slack; one
             // weight: 1.5 * 2^-22 of the largest tm, 1.33x slack), and never 0, so
             // that a box of exactly the mean counts as the dip it is.  Ei: the same of
-            // the weight (half an ulp per prefix, 2^-24 of the total; 2x slack).
+            // the weight inside or outside a box, in units of 2^-24 of the total Wt: a
+            // prefix is up to 2 Wt (the pad counts bins 1..o again) and rounds by 2, two of
+            // them by 4; their difference by 1, Wt by 1 and Wt less the difference by 1,
+            // 7 in all where 8 are taken.
             if (one_weight<MODE>())
                 tmax += 4.0f * fabsf((float)cv.center_frac) * (float)cv.n_points;
             const float Et =
@@ -1026,7 +1029,7 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
             constexpr int kShift = screen_shift<MODE>();
             const float Wt = one_weight<MODE>() ? (float)cv.n_points
                                                 : (float)ldexp(cv.i_total, -kShift);
-            const float Ei = one_weight<MODE>() ? 0.0f : Wt * (1.0f / 8388608.0f);
+            const float Ei = one_weight<MODE>() ? 0.0f : Wt * (1.0f / 2097152.0f);
             const float small = cv.w_small;
 
             // Sweep: starts outer, 32 per warp and step; widths inner in groups of four
