@@ -336,9 +336,11 @@ __device__ __forceinline__ void tls_templates(const TlsArgs& a, double w_total, 
         const float n = (float)num[i], c = (float)cwg[i], d = (float)den[i];
         // cwg^2 / w_total <= den, so de is within 3e-7 den of the exact difference; with de
         // above 1e-4 den (and the template certainly admissible) the quotient bounds sr
-        // from above and is within 2e-2 of it
-        const float cc = c * c * w_inv, de = d - cc;
-        float s = n * n / (de - 1e-6f * d);
+        // from above and is within 2e-2 of it.  (c w_inv is at most about 1, and n over
+        // the difference as large as sr / n: a square of c or n would leave FP32's normal
+        // range for weights below 1e-19)
+        const float cc = c * (c * w_inv), de = d - cc;
+        float s = n * (n / (de - 1e-6f * d));
         if (!(s > 1e-30f && s < 1e37f) || !(d > 1e-30f) || !(de > de_rel * d)) s = CUDART_INF_F;
         est[i] = in && num[i] < 0.0 && den[i] > a.w_eps ? s : -1.0f;
         if (est[i] < CUDART_INF_F) most = fmaxf(most, est[i]);
