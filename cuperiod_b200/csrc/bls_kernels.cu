@@ -505,7 +505,11 @@ __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& 
                     open |= 1u << r;
                     rec[r] = hq + kB * (uint32_t)hl;
                 }
-            int pos = atomicAdd(&sh.open_n, __popc(open));
+            // (a full list is not counted further: the counter stays below kList plus the
+            // CTA's points in flight, however many points are open)
+            int pos = kList;
+            if (*static_cast<volatile int*>(&sh.open_n) < kList)
+                pos = atomicAdd(&sh.open_n, __popc(open));
             const bool fits = pos + __popc(open) <= kList &&
                               point_index<NR, TAIL>(base, NR) < (1 << kOpenBits);
             if (!fits) lost |= 1u << q;
