@@ -200,7 +200,11 @@ __device__ __forceinline__ void tls_fold(const TlsArgs& a, TlsShared& s, const T
                     const int j = tls_point<NR, TAIL>(base, first, r);
                     if (edge >= fold.limit && (!TAIL || j < cv.n_points)) open |= 1u << r;
                 }
-                int pos = atomicAdd(&s.list_n, __popc(open));
+                // (a full list is not counted further: the counter stays below kTList plus
+                // the CTA's points in flight)
+                int pos = kTList;
+                if (*static_cast<volatile int*>(&s.list_n) < kTList)
+                    pos = atomicAdd(&s.list_n, __popc(open));
                 if (pos + __popc(open) > kTList) {
                     lost |= 1u << p;
                     for (; pos < kTList && open != 0u; ++pos, open &= open - 1u)
