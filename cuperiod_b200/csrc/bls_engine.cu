@@ -281,6 +281,26 @@ cudaStream_t pick(BlsEngine* e, void* s) {
     return s ? static_cast<cudaStream_t>(s) : e->stream;
 }
 
+// The staging buffers may be written again once the last prepare's uploads have passed.  A
+// stream capture goes through: this thread waits in relaxed mode (a wait is refused while any
+// thread captures in global mode), and on a capturing stream nothing is recorded (an event of
+// a capture cannot be waited for; its copies read the staging buffers at each replay).
+int wait_uploads(BlsEngine* e) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    const cudaError_t waited = cudaEventSynchronize(e->uploaded);
+    CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    CUDA_TRY(waited, "wait for the last uploads");
+    return BLS_OK;
+}
+int mark_uploads(BlsEngine* e, cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(st, &capture), "capture status");
+    if (capture == cudaStreamCaptureStatusNone)
+        CUDA_TRY(cudaEventRecord(e->uploaded, st), "mark the uploads");
+    return BLS_OK;
+}
+
 // Memory slot of the point with time index j in a curve of n points: every full
 // chunk of kChunk points is stored lane-interleaved (see kChunk in bls_device.h),
 // the tail in time order.
@@ -589,7 +609,8 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     e->prepared = false;
     e->graph_valid = false;
     e->launched = false;
-    CUDA_TRY(cudaEventSynchronize(e->uploaded), "wait for the last uploads");
+    int rc;
+    if ((rc = wait_uploads(e))) return rc;
     const int nc = cv->n_curves;
     const int o = grids[0].oversample;
     std::vector<int> sbase(n_grids + 1, 0);
@@ -624,7 +645,6 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     // pieces of at most kPiece periods over the host threads: 1,024 default grids took 47 ms
     // through vectors of their own (first touches, 16 bytes a period) and a serial copy, 6 ms
     // so; the 92,000 periods of one star's grid 1.6 ms and 0.4.
-    int rc;
     constexpr int64_t kPiece = 8192;
     const size_t grid_bytes = (size_t)P_total * (8 + 8 + 4 + 4) + 64;
     if ((rc = e->h_grid.ensure(grid_bytes))) return rc;
@@ -1129,7 +1149,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
              "upload grid");
     CUDA_TRY(cudaMemcpyAsync(e->d_curves.p, mp, meta_bytes, cudaMemcpyHostToDevice, st),
              "upload descriptors");
-    CUDA_TRY(cudaEventRecord(e->uploaded, st), "mark the uploads");
+    if ((rc = mark_uploads(e, st))) return rc;
     h2d += (int64_t)(grid_bytes + meta_bytes);
     CUDA_TRY(cudaMemsetAsync(e->d_ctl.p, 0, 64, st), "reset control words");
     for (int m = 0; m < kModes; ++m)
