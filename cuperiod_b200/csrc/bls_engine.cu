@@ -243,7 +243,8 @@ struct BlsEngine {
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
     bool launched = false;
-    // the last prepare's uploads: the staging buffers may be written once it has passed
+    // the last prepare's uploads (of any of the three searches; each waits for the one before):
+    // the staging buffers may be written once it has passed
     cudaEvent_t uploaded = nullptr;
 
     // the prepared TLS search
@@ -1554,6 +1555,7 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
     const size_t o_scr = o_ctl + 256;
     const size_t total = o_scr + (in_smem ? 0 : (size_t)ctas * hist_bytes);
     int rc;
+    if ((rc = wait_uploads(e))) return rc;
     if ((rc = e->h_joint.ensure(std::max(staged, (size_t)8 * kJointFields * P_total)))) return rc;
     char* h = e->h_joint.as<char>();
     double t_min = 0.0;
@@ -1572,6 +1574,7 @@ int do_prepare_joint(BlsEngine* e, const BlsGrid* g, const BlsCurves* bv, cudaSt
     if ((rc = e->d_joint.ensure(total))) return rc;
     char* d = e->d_joint.as<char>();
     CUDA_TRY(cudaMemcpyAsync(d, h, staged, cudaMemcpyHostToDevice, st), "upload bands");
+    if ((rc = mark_uploads(e, st))) return rc;
     CUDA_TRY(cudaMemsetAsync(d + o_ctl, 0, 256, st), "reset control words");
 
     JointArgs a{};
@@ -1624,7 +1627,8 @@ int do_download_joint(BlsEngine* e, double* out, cudaStream_t st) {
     if ((rc = e->h_ctl.ensure(64))) return rc;
     int32_t* hflag = e->h_ctl.as<int32_t>();
     const size_t bytes = 8 * (size_t)kJointFields * P;
-    // the staging buffer holds at least this much (do_prepare_joint)
+    // the staging buffer, once it is uploaded, holds at least this much (do_prepare_joint)
+    if ((rc = wait_uploads(e))) return rc;
     char* h = e->h_joint.as<char>();
     CUDA_TRY(cudaMemcpyAsync(h, e->jargs.out, bytes, cudaMemcpyDeviceToHost, st),
              "download joint fields");
@@ -1721,6 +1725,7 @@ int do_prepare_tls(BlsEngine* e, const BlsTlsInputs* in, const double* periods, 
     const size_t o_out = staged;
     const size_t o_ctl = o_out + align256(out_bytes);
     int rc;
+    if ((rc = wait_uploads(e))) return rc;
     if ((rc = e->h_tls.ensure(std::max(staged, out_bytes)))) return rc;
     char* h = e->h_tls.as<char>();
     TlsCurveDesc* cd = reinterpret_cast<TlsCurveDesc*>(h + o_cur);
@@ -1810,6 +1815,7 @@ int do_prepare_tls(BlsEngine* e, const BlsTlsInputs* in, const double* periods, 
     if ((rc = e->d_tls.ensure(o_ctl + 256))) return rc;
     char* d = e->d_tls.as<char>();
     CUDA_TRY(cudaMemcpyAsync(d, h, staged, cudaMemcpyHostToDevice, st), "upload TLS inputs");
+    if ((rc = mark_uploads(e, st))) return rc;
     CUDA_TRY(cudaMemsetAsync(d + o_ctl, 0, 256, st), "reset control words");
 
     TlsArgs a{};
@@ -1864,7 +1870,8 @@ int do_download_tls(BlsEngine* e, double* out, cudaStream_t st) {
     int rc;
     if ((rc = e->h_ctl.ensure(64))) return rc;
     int32_t* hflag = e->h_ctl.as<int32_t>();
-    // the staging buffer holds at least the output (do_prepare_tls)
+    // the staging buffer, once it is uploaded, holds at least the output (do_prepare_tls)
+    if ((rc = wait_uploads(e))) return rc;
     char* h = e->h_tls.as<char>();
     CUDA_TRY(cudaMemcpyAsync(h, e->targs.out, e->tls_out_bytes, cudaMemcpyDeviceToHost, st),
              "download TLS fields");
