@@ -564,10 +564,50 @@ __device__ __forceinline__ void fold_block(const BatchArgs& a, TileShared& sh, c
         fold_lane_exactly<MODE, NR, TAIL>(&a, &s, base, __ffs(lost) - 1, hist_s);
 }
 
+// Fold the curve into the histograms of a tile whose segment has no provable fast fold (more
+// cycles than it covers): the reference's IEEE chain for every point and period.  Bound by
+// its two divisions, of which four points keep as many chains going in a lane.
+template <int MODE>
+__device__ __noinline__ void fold_curve_exactly(const BatchArgs* a, const Tile* tl,
+                                                uint32_t hist_s) {
+    constexpr int NR = 4;
+    const int pt = tl->p_count, n = tl->curve.n_points, width = tl->seg.width;
+    const uint32_t plane = plane_bytes<MODE>(tl->seg.hist_len);
+    const uint32_t pbytes = hist_period_bytes<MODE>(tl->seg.hist_len);
+    const double bin = tl->seg.bin_duration;
+    for (int j0 = (int)threadIdx.x; j0 < n; j0 += kThreads * NR) {
+        PointRegs<MODE, NR> p;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const int j = j0 + r * kThreads;
+            const int64_t i = tl->curve.point_off + min(j, n - 1);
+            p.x[r] = __ldg(a->tau + i);
+            load_words<MODE, NR>(*a, i, j < n, p, r);
+        }
+        uint32_t hq = hist_s;
+        for (int q = 0; q < pt; ++q, hq += pbytes) {
+            const double P = tl->per[q];
+            const int nb = tl->nb[q];
+            int e[NR];
+#pragma unroll
+            for (int r = 0; r < NR; ++r) e[r] = fold_exact(p.x[r], P, bin, width);
+#pragma unroll
+            for (int r = 0; r < NR; ++r)        // (the reference never reads a bin past n_bins)
+                if (j0 + r * kThreads < n && e[r] <= nb)
+                    add_point<MODE, NR>(hq + bin_stride<MODE>() * (uint32_t)e[r], plane, p, r,
+                                        a->error_flag);
+        }
+    }
+}
+
 // Fold the curve into the histograms of the tile.
 template <int MODE>
 __device__ __forceinline__ void fold_curve(const BatchArgs& a, TileShared& s, const Tile& tl,
                                            uint32_t smem_s) {
+    if (!tl.seg.fast_fold) {
+        fold_curve_exactly<MODE>(&a, &tl, smem_s);
+        return;
+    }
     const int pt = tl.p_count, hl = tl.seg.hist_len, n = tl.curve.n_points;
     int base = 0;
     if (MODE != MODE_GENERAL && tl.seg.bin_duration > 1.5f * tl.curve.gap)
