@@ -150,6 +150,7 @@ struct BatchArgs {
     double* debug_prefix;       // test hook: prefix sums of one period (NULL in searches)
     int32_t n_items;
     int32_t obj_flag;           // 0 snr, 1 log-likelihood
+    uint32_t smem_bytes;        // dynamic shared memory of a CTA
 };
 
 // ---- joint-ephemeris multi-band search --------------------------------------

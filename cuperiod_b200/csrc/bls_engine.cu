@@ -1192,6 +1192,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         a.out = e->d_out.as<double>();
         a.out_stride = spec_total;
         a.work_counter = ctl + m;
+        a.smem_bytes = (uint32_t)smem_mode[m];
         a.error_flag = ctl + 8;
         a.debug_prefix = nullptr;
         a.obj_flag = grids[0].objective;

@@ -48,9 +48,9 @@ constexpr int kPts = kChunkPts;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr float kRel = 1.0f / 262144.0f;    // 2^-18: relative slack of FP32 key bounds
 constexpr int kCasLimit = 1 << 16;          // retries of one FP64 shared add
-constexpr int kList = 512;                  // open points, then candidates, of one tile
+constexpr int kList = 512;                  // candidates of one tile
 constexpr int kRegBins = 9;                 // bins a lane holds in registers while scanning
-constexpr int kOpenBits = 28;               // open point: period << kOpenBits | index
+constexpr int kOpenBits = 28;               // open point: period << kOpenBits | point
 constexpr uint32_t kNoPoint = 0xffffffffu;  // (of a 17th period)
 constexpr int kBoxBits = 20;                // box key: duration index << kBoxBits | start
 // Per-point weights: the FP32 screen holds them scaled by 2^-shift, their sum (below
@@ -87,12 +87,13 @@ struct TileShared {
     double red_v[kWarps];
     int red_box[kWarps];
     int red_ne[kWarps];             // GENERAL scan: last non-empty bin per warp
-    // after the sweeps, candidates: period << 25 | box, standing for the four widths of
-    // the box's group at its start; before them, while folding, open points: period <<
-    // kOpenBits | point
+    // candidates: period << 25 | box, standing for the four widths of the box's group at
+    // its start
     uint32_t list[kList];
     int list_n;
-    int open_n;
+    // shared address of the next entry of the fold's list of open points, period << kOpenBits |
+    // point: in the dynamic shared memory past the histograms, which is free until the scans
+    uint32_t open_at;
     uint32_t rescan;                // bit q: period q needs every box in FP64
 };
 
@@ -431,35 +432,55 @@ __device__ __host__ constexpr uint32_t bin_stride() {
     return MODE == MODE_GENERAL ? 16u : 4u;
 }
 
-// Point j of the curve at period q, whose fast fold is not provably the reference's bin:
-// by the reference's IEEE chain.  What the reference never reads, bins past n_bins, is
-// dropped.
+// Where the fold's list of open points begins: past the histograms (at the end of the memory,
+// which is no list, for more points than an entry can name).
 template <int MODE>
-__device__ __noinline__ void fold_exactly(const BatchArgs* a, const Tile* tl, int j, int q,
-                                          uint32_t hist_s) {
-    if (j >= tl->curve.n_points) return;
-    const uint32_t hq = hist_s + (uint32_t)q * hist_period_bytes<MODE>(tl->seg.hist_len);
-    const uint32_t plane = plane_bytes<MODE>(tl->seg.hist_len);
-    const int64_t i = tl->curve.point_off + j;
-    const int e = fold_exact(__ldg(a->tau + i), tl->per[q], tl->seg.bin_duration, tl->seg.width);
-    if (e > tl->nb[q]) return;
-    PointRegs<MODE, 1> p;
-    load_words<MODE, 1>(*a, i, true, p, 0);
-    add_point<MODE, 1>(hq + bin_stride<MODE>() * (uint32_t)e, plane, p, 0, a->error_flag);
+__device__ __forceinline__ uint32_t open_list(const Tile& tl, uint32_t smem_s,
+                                              uint32_t smem_bytes) {
+    return smem_s + (tl.curve.n_points < (1 << kOpenBits) - kChunk
+                         ? (uint32_t)tl.p_count * hist_period_bytes<MODE>(tl.seg.hist_len)
+                         : smem_bytes);
 }
 
-// The open points of one lane's block at period q, when the list is full.
-template <int MODE, int NR, bool TAIL>
-__device__ __noinline__ void fold_lane_exactly(const BatchArgs* a, const Tile* tl, int base, int q,
-                                               uint32_t hist_s) {
+// One point at period q that the fast fold leaves open, by the reference's IEEE chain: moved
+// from the bin the fast fold gave it to the reference's (the sums are integers modulo 2^32, so
+// taking its words out again leaves no trace), or added there (GENERAL, where the fold leaves
+// it out).  What the reference never reads, bins past n_bins, is dropped.
+template <int MODE>
+__device__ __forceinline__ void settle_point(const Tile& tl, int fast_bin, double x,
+                                             const PointRegs<MODE, 1>& p, int q, uint32_t hist_s,
+                                             int32_t* flag) {
+    const uint32_t hq = hist_s + (uint32_t)q * hist_period_bytes<MODE>(tl.seg.hist_len);
+    const uint32_t plane = plane_bytes<MODE>(tl.seg.hist_len);
+    constexpr uint32_t kB = bin_stride<MODE>();
+    const int e = fold_exact(x, tl.per[q], tl.seg.bin_duration, tl.seg.width);
+    if constexpr (MODE != MODE_GENERAL) {
+        if (e == fast_bin) return;
+        constexpr int kW = point_words<MODE>();
+        uint32_t out[kW];
+#pragma unroll
+        for (int k = 0; k < kW; ++k) out[k] = 0u - p.w[0][k];
+        add_words<kW>(hq + kB * (uint32_t)fast_bin, plane, out);
+    }
+    if (e <= tl.nb[q]) add_point<MODE, 1>(hq + kB * (uint32_t)e, plane, p, 0, flag);
+}
+
+// Point j of the curve at those of the periods q_mask at which it is open.
+template <int MODE>
+__device__ __noinline__ void settle_open(const BatchArgs* a, const Tile* tl, int j,
+                                         uint32_t q_mask, uint32_t hist_s) {
+    if (j >= tl->curve.n_points) return;            // (a tail's slot past the last point)
     const SegmentDesc& g = tl->seg;
-    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, g.fast_fold != 0);
-    for (int r = 0; r < NR; ++r) {
-        const int j = point_index<NR, TAIL>(base, r);
-        if (j >= tl->curve.n_points) return;
-        const double x = __ldg(a->tau + tl->curve.point_off + j);
-        if (fc.edge(fc.position(x, tl->freq[q], tl->scale[q])) >= fc.limit)
-            fold_exactly<MODE>(a, tl, j, q, hist_s);
+    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, true);
+    const int64_t i = tl->curve.point_off + j;
+    const double x = __ldg(a->tau + i);
+    PointRegs<MODE, 1> p;
+    load_words<MODE, 1>(*a, i, true, p, 0);
+    for (; q_mask != 0u; q_mask &= q_mask - 1u) {
+        const int q = __ffs(q_mask) - 1;
+        const uint32_t v = fc.position(x, tl->freq[q], tl->scale[q]);
+        if (fc.edge(v) >= fc.limit)
+            settle_point<MODE>(*tl, (int)(v >> fc.fb) + 1, x, p, q, hist_s, a->error_flag);
     }
 }
 
@@ -471,17 +492,21 @@ __device__ __noinline__ void fold_lane_exactly(const BatchArgs* a, const Tile* t
 // cost (one-weight batch of 16 curves, 50,000 periods: 27.7 ms without, 29.8 with).
 //
 // Open points (not decided by the fast fold: 2 in 10^4 of a survey cadence, those on bin
-// edges) go to the bin past the last, which nothing reads, and to a list that the CTA
-// folds exactly at the end.  Folding them here, in whatever form, took a call inside the
-// loop, whose calling convention halves the registers that stay live: words were spilled
-// or formed again at every period (4 four-year curves 53.7 ms so, 48.7 ms with the list;
-// 16 curves of the batched workload 18.3 -> 16.7 ms).
+// edges; many where a cadence meets the edges, as round times and durations do) are added to
+// the fast fold's bin like the others (GENERAL: left out) and put on a list, which the CTA
+// settles at the end, a point a thread; a lane that finds the list full settles its own after
+// the block.  Folding them here, in whatever form, took a call inside the loop, whose calling
+// convention halves the registers that stay live (4 four-year curves 53.7 ms so, 48.7 ms with
+// the list; 16 curves of the batched workload 18.3 -> 16.7 ms).  The list takes what shared
+// memory the histograms leave: with 512 entries and the lanes past them left to themselves,
+// 4 curves of 60,000 points at a tenth of a bin, 4,000 periods, took 1.63 ms, 1.38 ms so;
+// 16 curves of 4,000 points, all on edges, 900 periods, 1.24 ms, 0.65 ms so.
 template <int MODE, int NR, bool TAIL, bool MERGE>
 __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& sh, const Tile& s,
                                                 uint32_t hist_s, const PointRegs<MODE, NR>& p,
                                                 int base, int pt, int hl) {
     const SegmentDesc& g = s.seg;
-    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, g.fast_fold != 0);
+    const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, true);
     const uint32_t plane = plane_bytes<MODE>(hl);
     const uint32_t pbytes = hist_period_bytes<MODE>(hl);
     constexpr uint32_t kB = bin_stride<MODE>();
@@ -490,40 +515,38 @@ __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& 
     for (int q = 0; q < pt; ++q, hq += pbytes) {
         const double f = s.freq[q];
         const uint32_t S = s.scale[q];
-        uint32_t rec[NR], worst = 0u;
+        uint32_t rec[NR], worst = 0u, skip = 0u;
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             const uint32_t v = fc.position(p.x[r], f, S);
             worst = max(worst, fc.edge(v));
             rec[r] = hq + kB + (v >> fc.fb) * kB;
         }
-        if (worst >= fc.limit) {
+        if (__builtin_expect(worst >= fc.limit, 0)) {
             uint32_t open = 0u;
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit) {
-                    open |= 1u << r;
-                    rec[r] = hq + kB * (uint32_t)hl;
-                }
-            // (a full list is not counted further: the counter stays below kList plus the
+            for (int r = NR - 1; r >= 0; --r)
+                open = open + open + (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit ? 1u : 0u);
+            if (MODE == MODE_GENERAL) skip = open;
+            // (a full list is not counted further: open_at stays below the list's end plus the
             // CTA's points in flight, however many points are open)
-            int pos = kList;
-            if (*static_cast<volatile int*>(&sh.open_n) < kList)
-                pos = atomicAdd(&sh.open_n, __popc(open));
-            const bool fits = pos + __popc(open) <= kList &&
-                              point_index<NR, TAIL>(base, NR) < (1 << kOpenBits);
-            if (!fits) lost |= 1u << q;
-            for (; open != 0u && pos < kList; ++pos) {
-                const int r = __ffs(open) - 1;
-                open &= open - 1u;
-                sh.list[pos] = fits ? ((uint32_t)q << kOpenBits) |
-                                          (uint32_t)point_index<NR, TAIL>(base, r)
-                                    : kNoPoint;
+            const uint32_t end = hist_s + a.smem_bytes, bytes = 4u * (uint32_t)__popc(open);
+            uint32_t at = end;
+            if (*static_cast<volatile uint32_t*>(&sh.open_at) < end)
+                at = atomicAdd(&sh.open_at, bytes);
+            if (at + bytes <= end) {
+                for (; open != 0u; at += 4u, open &= open - 1u)
+                    st_u32(at, ((uint32_t)q << kOpenBits) |
+                                   (uint32_t)point_index<NR, TAIL>(base, __ffs(open) - 1));
+            } else {
+                lost |= 1u << q;
+                for (; at < end; at += 4u) st_u32(at, kNoPoint);
             }
         }
         if constexpr (MODE == MODE_GENERAL) {
 #pragma unroll
-            for (int r = 0; r < NR; ++r) add_point<MODE, NR>(rec[r], plane, p, r, a.error_flag);
+            for (int r = 0; r < NR; ++r)
+                if (!(skip >> r & 1u)) add_point<MODE, NR>(rec[r], plane, p, r, a.error_flag);
         } else if constexpr (!MERGE) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) add_words(rec[r], plane, p.w[r]);
@@ -560,8 +583,10 @@ __device__ __forceinline__ void fold_block(const BatchArgs& a, TileShared& sh, c
         load_points<MODE, NR, TAIL>(a, s.curve, base, p);
         lost = fold_points<MODE, NR, TAIL, MERGE>(a, sh, s, hist_s, p, base, pt, hl);
     }
-    for (; lost != 0u; lost &= lost - 1u)
-        fold_lane_exactly<MODE, NR, TAIL>(&a, &s, base, __ffs(lost) - 1, hist_s);
+    // the list was full: this lane's open points of those periods now
+    if (lost != 0u)
+        for (int r = 0; r < NR; ++r)
+            settle_open<MODE>(&a, &s, point_index<NR, TAIL>(base, r), lost, hist_s);
 }
 
 // Fold the curve into the histograms of a tile whose segment has no provable fast fold (more
@@ -625,12 +650,13 @@ __device__ __forceinline__ void fold_curve(const BatchArgs& a, TileShared& s, co
     else if (left > 0)
         fold_block<MODE, 2, true, false>(a, s, tl, smem_s, base, pt, hl);
     __syncthreads();
-    const int open = min(s.open_n, kList);
-    for (int e = threadIdx.x; e < open; e += kThreads) {
-        const uint32_t p = s.list[e];
+    const uint32_t end = min(s.open_at, smem_s + a.smem_bytes);
+    for (uint32_t at = open_list<MODE>(tl, smem_s, a.smem_bytes) + 4u * threadIdx.x; at < end;
+         at += 4u * kThreads) {
+        const uint32_t p = ld_u32(at);
         if (p != kNoPoint)
-            fold_exactly<MODE>(&a, &tl, (int)(p & ((1u << kOpenBits) - 1u)), (int)(p >> kOpenBits),
-                               smem_s);
+            settle_open<MODE>(&a, &tl, (int)(p & ((1u << kOpenBits) - 1u)), 1u << (p >> kOpenBits),
+                              smem_s);
     }
 }
 
@@ -966,7 +992,6 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
         if (tl.item >= a.n_items) break;
         if (tid == 0) {
             s.list_n = 0;
-            s.open_n = 0;
             s.rescan = 0u;
         }
         // (what the fold needs is read here and again below, so that little stays in
@@ -992,6 +1017,7 @@ __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
 
         // ---- 1. fold ---------------------------------------------------------
         const uint32_t smem_s = smem_addr(smem);
+        if (tid == 0) s.open_at = open_list<MODE>(tl, smem_s, a.smem_bytes);
         {
             const int n16 = (int)(tl.p_count * hist_period_bytes<MODE>(tl.seg.hist_len) / 16u);
             uint4* z = reinterpret_cast<uint4*>(smem);
