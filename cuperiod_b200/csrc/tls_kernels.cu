@@ -31,6 +31,8 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "bls_device.h"
 #include "bls_launch.h"
 
@@ -46,6 +48,11 @@ constexpr unsigned kTAll = 0xffffffffu;
 enum : int { TERR_DESC = 1 };
 
 constexpr int kTList = 256;             // open points of one tile
+// Points from which the sweep estimates a template's residue before it divides (tls_templates):
+// with fewer, most templates hold the same point and tie, every lane passes, and the estimate
+// only costs (3 curves, 200,000 periods, with and without it: 20 points 10.2 and 9.2 ms, 50
+// points 9.8 and 9.4, 100 points 9.2 and 9.4 ms).
+constexpr int kTlsEstimate = 80;
 
 struct TlsShared {
     union {
@@ -305,10 +312,12 @@ __device__ __forceinline__ void tls_fold_curve(const TlsArgs& a, TlsShared& s,
 }
 
 // NG templates from di at this lane's start st (`in`: there is one) of the bins v, kept
-// when one is the best so far.  The reference's two divisions per template and start are
-// taken only by the lanes that may hold the warp's best: an FP32 bound on sr decides (one
-// out of FP32's range always passes).
-template <int NG>
+// when one is the best so far.  With EST the reference's two divisions per template and start
+// are taken only by the lanes that may hold the warp's best: an FP32 bound on sr decides (one
+// out of FP32's range always passes).  The first samples are taken ahead of the loop: chosen
+// inside it they cost six selections a template and sample, and the registers that the fold
+// needs (60,000 points in wide bins 12.2 ms so, 8.2 ms; 1,000 points 9.56 and 8.92).
+template <int NG, bool EST>
 __device__ __forceinline__ void tls_templates(const TlsArgs& a, double w_total, float w_inv, float de_rel,
                                               const double2* v, const double* g, int di, int st,
                                               bool in, float& top, double& best, long long& key,
@@ -321,38 +330,46 @@ __device__ __forceinline__ void tls_templates(const TlsArgs& a, double w_total, 
         off[i] = __ldg(a.tmpl_off + di + i);
         wmax = max(wmax, W[i]);
     }
-    for (int k = 0; k < wmax; ++k) {
+    const double2 e0 = v[st];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        const double t = g[off[i]];
+        num[i] = __dmul_rn(t, e0.x);
+        cwg[i] = __dmul_rn(t, e0.y);
+        den[i] = __dmul_rn(__dmul_rn(t, t), e0.y);
+    }
+    for (int k = 1; k < wmax; ++k) {
         const double2 e = v[st + k];
 #pragma unroll
         for (int i = 0; i < NG; ++i)
             if (k < W[i]) {
                 const double t = g[off[i] + k];
-                const double x = __dmul_rn(t, e.x), y = __dmul_rn(t, e.y),
-                             z = __dmul_rn(__dmul_rn(t, t), e.y);
-                num[i] = k == 0 ? x : __dadd_rn(num[i], x);
-                cwg[i] = k == 0 ? y : __dadd_rn(cwg[i], y);
-                den[i] = k == 0 ? z : __dadd_rn(den[i], z);
+                num[i] = __dadd_rn(num[i], __dmul_rn(t, e.x));
+                cwg[i] = __dadd_rn(cwg[i], __dmul_rn(t, e.y));
+                den[i] = __dadd_rn(den[i], __dmul_rn(__dmul_rn(t, t), e.y));
             }
     }
     float est[NG], most = 0.0f;
+    if (EST) {
 #pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        const float n = (float)num[i], c = (float)cwg[i], d = (float)den[i];
-        // cwg^2 / w_total <= den, so de is within 3e-7 den of the exact difference; with de
-        // above 1e-4 den (and the template certainly admissible) the quotient bounds sr
-        // from above and is within 2e-2 of it.  (c w_inv is at most about 1, and n over
-        // the difference as large as sr / n: a square of c or n would leave FP32's normal
-        // range for weights below 1e-19)
-        const float cc = c * (c * w_inv), de = d - cc;
-        float s = n * (n / (de - 1e-6f * d));
-        if (!(s > 1e-30f && s < 1e37f) || !(d > 1e-30f) || !(de > de_rel * d)) s = CUDART_INF_F;
-        est[i] = in && num[i] < 0.0 && den[i] > a.w_eps ? s : -1.0f;
-        if (est[i] < CUDART_INF_F) most = fmaxf(most, est[i]);
+        for (int i = 0; i < NG; ++i) {
+            const float n = (float)num[i], c = (float)cwg[i], d = (float)den[i];
+            // cwg^2 / w_total <= den, so de is within 3e-7 den of the exact difference; with de
+            // above 1e-4 den (and the template certainly admissible) the quotient bounds sr
+            // from above and is within 2e-2 of it.  (c w_inv is at most about 1, and n over
+            // the difference as large as sr / n: a square of c or n would leave FP32's normal
+            // range for weights below 1e-19)
+            const float cc = c * (c * w_inv), de = d - cc;
+            float s = n * (n / (de - 1e-6f * d));
+            if (!(s > 1e-30f && s < 1e37f) || !(d > 1e-30f) || !(de > de_rel * d)) s = CUDART_INF_F;
+            est[i] = in && num[i] < 0.0 && den[i] > a.w_eps ? s : -1.0f;
+            if (est[i] < CUDART_INF_F) most = fmaxf(most, est[i]);
+        }
+        top = fmaxf(top, __uint_as_float(__reduce_max_sync(kTAll, __float_as_uint(most))));
     }
-    top = fmaxf(top, __uint_as_float(__reduce_max_sync(kTAll, __float_as_uint(most))));
 #pragma unroll
     for (int i = 0; i < NG; ++i)
-        if (est[i] >= top * (1.0f - 2e-2f)) {
+        if (EST ? est[i] >= top * (1.0f - 2e-2f) : in && num[i] < 0.0 && den[i] > a.w_eps) {
             const double de = __dsub_rn(den[i], __ddiv_rn(__dmul_rn(cwg[i], cwg[i]), w_total));
             if (de > __dmul_rn(a.den_rel, den[i])) {
                 const double sr = __ddiv_rn(__dmul_rn(num[i], num[i]), de);
@@ -430,13 +447,18 @@ __global__ void __launch_bounds__(kTThreads, 3) tls_kernel(const __grid_constant
             for (int s0 = warp * 32; s0 < nb; s0 += kTThreads) {
                 const bool in = s0 + lane < nb;
                 const int st = in ? s0 + lane : 0;
-                int di = 0;
-                for (; di + 4 <= a.n_dur; di += 4)
-                    tls_templates<4>(a, w_total, w_inv, de_rel, v, g, di, st, in, top, best, best_key,
-                                     best_depth);
-                for (; di < a.n_dur; ++di)
-                    tls_templates<1>(a, w_total, w_inv, de_rel, v, g, di, st, in, top, best, best_key,
-                                     best_depth);
+                auto templates = [&](auto est) {
+                    constexpr bool kEst = decltype(est)::value;
+                    int di = 0;
+                    for (; di + 4 <= a.n_dur; di += 4)
+                        tls_templates<4, kEst>(a, w_total, w_inv, de_rel, v, g, di, st, in, top,
+                                               best, best_key, best_depth);
+                    for (; di < a.n_dur; ++di)
+                        tls_templates<1, kEst>(a, w_total, w_inv, de_rel, v, g, di, st, in, top,
+                                               best, best_key, best_depth);
+                };
+                if (cv.n_points >= kTlsEstimate) templates(std::true_type{});
+                else templates(std::false_type{});
             }
             __syncwarp();
 #pragma unroll
