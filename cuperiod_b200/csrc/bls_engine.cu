@@ -569,6 +569,10 @@ void parallel_for(int64_t n, F&& fn, int64_t most = INT32_MAX) {
 constexpr size_t kDefaultSmem[kModes] = {70 * 1024, 108 * 1024, 108 * 1024, 70 * 1024,
                                          108 * 1024};
 
+// BlsTune.smem_per_cta is taken up to the device's opt-in limit less this, whatever static
+// shared state the kernels come to hold.
+constexpr size_t kTuneStatic = 1552;
+
 // A grid segment of at least this many periods may be cut by bin count (do_prepare).
 constexpr int kSplitPeriods = 512;
 
@@ -972,7 +976,12 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     for (int m = 0; m < kModes; ++m) modes[m] = n_mode[m] > 0;
     size_t smem_mode[kModes];
     for (int m = 0; m < kModes; ++m) {
+        // the opt-in limit covers the kernel's static shared state too
+        const size_t limit = modes[m] ? e->smem_optin + 1024 - search_static_smem(m) : 0;
         size_t sm = e->tune.smem_per_cta > 0 ? (size_t)e->tune.smem_per_cta : kDefaultSmem[m];
+        // (a request for nearly all of it gets what is left)
+        if (modes[m] && sm <= e->smem_optin + 1024 - kTuneStatic)
+            sm = std::min(sm, limit & ~size_t(15));
         for (int s = 0; s < ns && modes[m]; ++s) {
             if (segs[s].empty_periods || grid_mode[seg_grid[s]][m] == 0) continue;
             const size_t need = screen_bytes(segs[s].d.hist_len) + 16 +
@@ -980,8 +989,6 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
             if (need > sm) sm = need;
         }
         sm = (sm + 15) & ~size_t(15);
-        // the opt-in limit covers the kernel's static shared state too
-        const size_t limit = modes[m] ? e->smem_optin + 1024 - search_static_smem(m) : 0;
         if (modes[m] && sm > limit)
             return fail(BLS_E_RESOURCE,
                         "BLS: %zu bytes of shared memory per CTA exceed the device's %zu "
