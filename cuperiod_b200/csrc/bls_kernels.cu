@@ -1867,7 +1867,7 @@ cudaError_t launch_rows(const double* out, int64_t out_stride, int n_curves,
                         int harmonic_max, int32_t* n_peaks, int64_t* index, double* fields,
                         cudaStream_t stream) {
     if (n_curves <= 0) return cudaSuccess;
-    // the list while it fits beside the bitmap: up to 890,000 periods
+    // the list while it fits beside the bitmap: up to 917,504 periods
     const size_t bits = sizeof(uint32_t) * (size_t)((max_periods + 31) / 32);
     const size_t list = kRowList * (2 * sizeof(double) + sizeof(int32_t)) + kRowBins * sizeof(int);
     const int list_cap = bits + list <= 160 * 1024 && max_periods <= INT32_MAX ? kRowList : 0;
