@@ -38,8 +38,9 @@ constexpr int kMaxDur = 32;         // deduplicated box widths per segment
 constexpr int kMaxTile = 16;        // periods per work item
 constexpr int kHalfBits = 13;       // UNIFORM: bits of the low word
 constexpr int kCountShift = 18;     // packed prefix: R * 2^18 + count
-constexpr int kMaxExactPoints = (1 << 17) - 1;  // UNIFORM / WIDE: 32-bit prefix words
-                                                // stay exact; longer curves take GENERAL
+constexpr int kMaxExactPoints = (1 << 17) - 1;  // the integer modes' sums stay exact (bits of
+                                                // a value, count of a packed prefix); longer
+                                                // curves take GENERAL
 constexpr int kMaxPoints = 1 << 30;             // per curve (int32 indices)
 
 // One CTA folds points in chunks of kChunkThreads x kChunkPts.  The host stores

@@ -1229,7 +1229,7 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     in.trials = trials;
     in.h2d_bytes = h2d;
     in.ctas = ctas_total;
-in.smem_per_cta = 0;
+    in.smem_per_cta = 0;
     for (int m : {MODE_PAIR, MODE_UNIFORM, MODE_WIDE, MODE_EXACT, MODE_GENERAL})
         if (in.smem_per_cta == 0 && modes[m]) in.smem_per_cta = (int32_t)smem_mode[m];
     in.uniform_curves = n_uniform;
@@ -1241,7 +1241,7 @@ in.smem_per_cta = 0;
     return BLS_OK;
 }
 
-// Enqueue one search (both accumulation modes) on `st`.
+// Enqueue one search (a launch per accumulation mode in use) on `st`.
 int enqueue_search(BlsEngine* e, cudaStream_t st) {
     // the work counters (words 0..kModes-1) and the error flag (word 8): every
     // search starts clean, so BLS_E_DEVICE reports this search's descriptors only

@@ -35,7 +35,7 @@ cudaError_t launch_best(const double* power, int n_curves, const int64_t* spec_o
 
 // Scratch of the allocation-free search (bls_launch_best_noalloc): one
 // file-scope device array per device.  Bytes [0, 64): the work counters of the
-// two accumulation modes (words 0 and 1) and the error flag (word 8), which
+// accumulation modes (words 0 to kModes - 1) and the error flag (word 8), which
 // must all be zero when a search starts.  From byte 256: per curve the best
 // index (int64), then best power, power mean and power standard deviation
 // (double), kStaticMaxCurves entries each, written in full by best_kernel.
