@@ -1011,13 +1011,16 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         for (int c = 0; c < nc; ++c)
             if (curves[c].d.mode == m) members[gid[c]].push_back(c);
         // few periods in all: tiles that give every resident CTA one (1,000 periods of
-        // one 300-point curve: 23 us in tiles of 3, 42 in tiles of 16, 28 in tiles of 1)
+        // one 300-point curve: 23 us in tiles of 3, 42 in tiles of 16, 28 in tiles of 1),
+        // or four, of at least four periods (4 curves of 60,000 points on a regular cadence,
+        // 36 periods a CTA: 1.36 ms in tiles of 16, 0.99 of 9; at random times 0.99 and 0.97)
         int64_t searched = 0;
         for (int k = 0; k < n_grids; ++k)
             searched += (int64_t)members[k].size() * (pbase[k + 1] - pbase[k]);
         const int64_t slots = (int64_t)e->n_sm * std::max(1, max_resident_ctas(m, smem_mode[m]));
+        const int64_t per_cta = std::max<int64_t>(1, (searched + slots - 1) / slots);
         const int spread = (int)std::min<int64_t>(
-            kMaxTile, std::max<int64_t>(1, (searched + slots - 1) / slots));
+            kMaxTile, per_cta <= 4 ? per_cta : std::max<int64_t>(4, (per_cta + 3) / 4));
         struct Cand {
             int grid;
             int64_t tiles;
