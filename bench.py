@@ -56,7 +56,7 @@ LB_WORKLOAD = ("long-baseline precision stress BLS: {n} curves of 60,000 points 
 # over the first 256 curves of this workload, from one ncu capture
 # (profiles/bls_search_kernel_launches_256curves.txt); a launch's traffic grows in
 # proportion to its curves (points in, 7 fields x periods out)
-TRAFFIC_256 = 58348800 + 678396928
+TRAFFIC_256 = 56890112 + 678989056
 CLOCK_FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
                 "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
                 "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -609,8 +609,8 @@ def run_ours(args) -> None:
         alg_bytes = n_pts * 12 + P * 24 + 7 * 8 * n_curves * P
         achieved = alg_bytes / (kernel_ms / 1000.0) / 1e9
         # SM-pipe model: the native shared atomics of a fold (2 with one weight per
-        # curve, 4 with per-point weights) at the measured random rate, 2 FP64 ops per fold, ~10 FP32 ops per box (rates from
-        # csrc/pipe_probe.cu, profiles/pipe_rates.txt)
+        # curve, 4 with per-point weights) at the measured random rate, 2 FP64 ops per
+        # fold, ~10 FP32 ops per box (rates from profiles/pipe_rates.txt)
         f_clk = (clocks.get("sm_mhz") or 1900.0) * 1e6
         n_sm = torch.cuda.get_device_properties(local).multi_processor_count
         words = 2 if args.weights == "uniform" else 4

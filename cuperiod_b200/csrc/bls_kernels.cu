@@ -926,8 +926,8 @@ __device__ __forceinline__ void copy_words(T* to, const T* from, int lane) {
 // registers), per-point weights two.  Bound by latency between its barriers with 24 (16)
 // resident warps: neither issue nor the shared-memory pipe is above two thirds busy.
 // 96 curves of the batched workload (mean 9,900 points, 50,000 periods): 152.8 ms with
-// three words a point, five barriers a period and a screened sweep; 99.4 ms as built.
-// 16 curves with per-point errors 52.7 -> 31.1 ms (38-bit weights), 8 with outlying
+// three words a point, five barriers a period and a screened sweep; 100 ms as built.
+// 16 curves with per-point errors 52.7 -> 30.0 ms (38-bit weights), 8 with outlying
 // errors 56.2 -> 21.3 ms (FP64 sums by compare-and-swap before).
 template <int MODE, int OBJ>
 __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
