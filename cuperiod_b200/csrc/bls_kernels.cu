@@ -521,15 +521,16 @@ __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& 
             const uint32_t v = fc.position(p.x[r], f, S);
             worst = max(worst, fc.edge(v));
             rec[r] = hq + kB + (v >> fc.fb) * kB;
-            // (formed here once: left to the compiler they are formed behind the branch, from
-            // positions that take the registers meanwhile; 4 four-year curves 47.7 -> 47.1 ms)
-            asm("" : "+r"(rec[r]));
+            // (formed here once where runs are merged: left to the compiler they are formed
+            // behind the branch, from positions that take the registers meanwhile; 4 four-year
+            // curves 47.7 -> 46.9 ms.  Without runs, or with six words, it costs up to 1%)
+            if (MERGE && MODE != MODE_EXACT) asm("" : "+r"(rec[r]));
         }
         if (__builtin_expect(worst >= fc.limit, 0)) {
             uint32_t open = 0u;
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
-                if (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit) open |= 1u << r;
+            for (int r = NR - 1; r >= 0; --r)
+                open = open + open + (fc.edge(fc.position(p.x[r], f, S)) >= fc.limit ? 1u : 0u);
             if (MODE == MODE_GENERAL) skip = open;
             // (a full list is not counted further: open_at stays below the list's end plus the
             // CTA's points in flight, however many points are open)
