@@ -996,6 +996,8 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
                         "the period range (max_period_days)",
                         sm, limit);
         smem_mode[m] = sm;
+        // (before anything asks how many CTAs are resident with that much)
+        if (modes[m]) CUDA_TRY(configure_search(m, sm), "shared-memory opt-in");
     }
     // per mode: one group per grid with curves of that mode -- the grid's tile
     // prefix and its curves largest first -- groups in decreasing cost per curve
@@ -1163,8 +1165,6 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
     if ((rc = mark_uploads(e, st))) return rc;
     h2d += (int64_t)(grid_bytes + meta_bytes);
     CUDA_TRY(cudaMemsetAsync(e->d_ctl.p, 0, 64, st), "reset control words");
-    for (int m = 0; m < kModes; ++m)
-        if (modes[m]) CUDA_TRY(configure_search(m, smem_mode[m]), "shared-memory opt-in");
 
     const char* dgp = e->d_period.as<char>();
     const double* dper = reinterpret_cast<const double*>(dgp);
