@@ -1013,16 +1013,22 @@ int do_prepare(BlsEngine* e, const BlsGrid* grids, int n_grids, const int32_t* g
         for (int c = 0; c < nc; ++c)
             if (curves[c].d.mode == m) members[gid[c]].push_back(c);
         // few periods in all: tiles that give every resident CTA one (1,000 periods of
-        // one 300-point curve: 23 us in tiles of 3, 42 in tiles of 16, 28 in tiles of 1),
-        // or four, of at least four periods (4 curves of 60,000 points on a regular cadence,
-        // 36 periods a CTA: 1.36 ms in tiles of 16, 0.99 of 9; at random times 0.99 and 0.97)
-        int64_t searched = 0;
-        for (int k = 0; k < n_grids; ++k)
+        // one 300-point curve: 23 us in tiles of 3, 42 in tiles of 16, 28 in tiles of 1); from
+        // 4,000 points a curve, where a tile takes long, four of at least four periods (4
+        // curves of 60,000 points on a regular cadence, 36 periods a CTA: 1.36 ms in tiles of
+        // 16, 0.99 of 9; 16 of 4,000 0.39 and 0.37; one of 2,000, 9 a CTA, 67 and 76 us)
+        int64_t searched = 0, curves_in = 0, points_in = 0;
+        for (int k = 0; k < n_grids; ++k) {
             searched += (int64_t)members[k].size() * (pbase[k + 1] - pbase[k]);
+            curves_in += (int64_t)members[k].size();
+            for (int32_t c : members[k]) points_in += curves[c].d.n_points;
+        }
         const int64_t slots = (int64_t)e->n_sm * std::max(1, max_resident_ctas(m, smem_mode[m]));
         const int64_t per_cta = std::max<int64_t>(1, (searched + slots - 1) / slots);
+        const bool long_tiles = points_in >= 4000 * curves_in;
         const int spread = (int)std::min<int64_t>(
-            kMaxTile, per_cta <= 4 ? per_cta : std::max<int64_t>(4, (per_cta + 3) / 4));
+            kMaxTile, per_cta <= 4 || !long_tiles ? per_cta
+                                                  : std::max<int64_t>(4, (per_cta + 3) / 4));
         struct Cand {
             int grid;
             int64_t tiles;
