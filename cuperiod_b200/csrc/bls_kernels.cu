@@ -465,22 +465,25 @@ __device__ __forceinline__ void settle_point(const Tile& tl, int fast_bin, doubl
     if (e <= tl.nb[q]) add_point<MODE, 1>(hq + kB * (uint32_t)e, plane, p, 0, flag);
 }
 
-// Point j of the curve at those of the periods q_mask at which it is open.
+// The points j, j + step, ... of the curve, `count` of them, at those of the periods q_mask at
+// which they are open.
 template <int MODE>
-__device__ __noinline__ void settle_open(const BatchArgs* a, const Tile* tl, int j,
-                                         uint32_t q_mask, uint32_t hist_s) {
-    if (j >= tl->curve.n_points) return;            // (a tail's slot past the last point)
+__device__ __noinline__ void settle_open(const BatchArgs* a, const Tile* tl, int j, int count,
+                                         int step, uint32_t q_mask, uint32_t hist_s) {
     const SegmentDesc& g = tl->seg;
     const FoldConst fc(g.frac_bits, g.margin_u, g.margin_phi, true);
-    const int64_t i = tl->curve.point_off + j;
-    const double x = __ldg(a->tau + i);
-    PointRegs<MODE, 1> p;
-    load_words<MODE, 1>(*a, i, true, p, 0);
-    for (; q_mask != 0u; q_mask &= q_mask - 1u) {
-        const int q = __ffs(q_mask) - 1;
-        const uint32_t v = fc.position(x, tl->freq[q], tl->scale[q]);
-        if (fc.edge(v) >= fc.limit)
-            settle_point<MODE>(*tl, (int)(v >> fc.fb) + 1, x, p, q, hist_s, a->error_flag);
+    for (; count > 0; --count, j += step) {
+        if (j >= tl->curve.n_points) return;        // (a tail's slots past the last point)
+        const int64_t i = tl->curve.point_off + j;
+        const double x = __ldg(a->tau + i);
+        PointRegs<MODE, 1> p;
+        load_words<MODE, 1>(*a, i, true, p, 0);
+        for (uint32_t m = q_mask; m != 0u; m &= m - 1u) {
+            const int q = __ffs(m) - 1;
+            const uint32_t v = fc.position(x, tl->freq[q], tl->scale[q]);
+            if (fc.edge(v) >= fc.limit)
+                settle_point<MODE>(*tl, (int)(v >> fc.fb) + 1, x, p, q, hist_s, a->error_flag);
+        }
     }
 }
 
@@ -523,7 +526,7 @@ __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& 
             rec[r] = hq + kB + (v >> fc.fb) * kB;
             // (formed here once where runs are merged: left to the compiler they are formed
             // behind the branch, from positions that take the registers meanwhile; 4 four-year
-            // curves 47.7 -> 46.9 ms.  Without runs, or with six words, it costs up to 1%)
+            // curves 47.7 -> 46.8 ms.  Without runs, or with six words, it costs up to 1%)
             if (MERGE && MODE != MODE_EXACT) asm("" : "+r"(rec[r]));
         }
         if (__builtin_expect(worst >= fc.limit, 0)) {
@@ -589,8 +592,8 @@ __device__ __forceinline__ void fold_block(const BatchArgs& a, TileShared& sh, c
     }
     // the list was full: this lane's open points of those periods now
     if (lost != 0u)
-        for (int r = 0; r < NR; ++r)
-            settle_open<MODE>(&a, &s, point_index<NR, TAIL>(base, r), lost, hist_s);
+        settle_open<MODE>(&a, &s, point_index<NR, TAIL>(base, 0), NR, TAIL ? 1 : kThreads, lost,
+                          hist_s);
 }
 
 // Fold the curve into the histograms of a tile whose segment has no provable fast fold (more
@@ -659,8 +662,8 @@ __device__ __forceinline__ void fold_curve(const BatchArgs& a, TileShared& s, co
          at += 4u * kThreads) {
         const uint32_t p = ld_u32(at);
         if (p != kNoPoint)
-            settle_open<MODE>(&a, &tl, (int)(p & ((1u << kOpenBits) - 1u)), 1u << (p >> kOpenBits),
-                              smem_s);
+            settle_open<MODE>(&a, &tl, (int)(p & ((1u << kOpenBits) - 1u)), 1, 1,
+                              1u << (p >> kOpenBits), smem_s);
     }
 }
 
