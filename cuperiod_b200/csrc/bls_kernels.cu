@@ -503,7 +503,7 @@ __device__ __noinline__ void settle_open(const BatchArgs* a, const Tile* tl, int
 // the list; 16 curves of the batched workload 18.3 -> 16.7 ms).  The list takes what shared
 // memory the histograms leave: with 512 entries and the lanes past them left to themselves,
 // 4 curves of 60,000 points at a tenth of a bin, 4,000 periods, took 1.63 ms, 1.38 ms so;
-// 16 curves of 4,000 points, all on edges, 900 periods, 1.24 ms, 0.65 ms so.
+// 16 curves of 4,000 points, all on edges, 900 periods, 1.24 ms, 0.64 ms so.
 template <int MODE, int NR, bool TAIL, bool MERGE>
 __device__ __forceinline__ uint32_t fold_points(const BatchArgs& a, TileShared& sh, const Tile& s,
                                                 uint32_t hist_s, const PointRegs<MODE, NR>& p,
@@ -930,8 +930,8 @@ __device__ __forceinline__ void copy_words(T* to, const T* from, int lane) {
 // registers), per-point weights two.  Bound by latency between its barriers with 24 (16)
 // resident warps: neither issue nor the shared-memory pipe is above two thirds busy.
 // 96 curves of the batched workload (mean 9,900 points, 50,000 periods): 152.8 ms with
-// three words a point, five barriers a period and a screened sweep; 100 ms as built.
-// 16 curves with per-point errors 52.7 -> 30.0 ms (38-bit weights), 8 with outlying
+// three words a point, five barriers a period and a screened sweep; 99.4 ms as built.
+// 16 curves with per-point errors 52.7 -> 30.3 ms (38-bit weights), 8 with outlying
 // errors 56.2 -> 21.3 ms (FP64 sums by compare-and-swap before).
 template <int MODE, int OBJ>
 __global__ void __launch_bounds__(kThreads, one_weight<MODE>() ? 3 : 2)
